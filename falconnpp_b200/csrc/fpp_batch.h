@@ -35,12 +35,31 @@ struct BatchRequest {
   // launch waiting only for its own chunk, so the copy overlaps the hashing
   const float* Q_host = nullptr;
   cudaStream_t copy_stream = nullptr;
+  int32_t* out_host = nullptr;      // host (nullable): nq x out_stride, copied back before the call returns
+  bool want_totals = false;         // sum the candidate and tie counts of the batch (BatchTotals)
   bool stage_timing = false;        // CUDA events around the hash and the fused kernel (synchronises)
   bool tc_rotation = false;        // opt-in, BF16/FP8, fhtDim 256: rotate on the tensor cores (FP16 operands,
                                    // not the reference's FP32 hash: probes can differ)
 };
 
+// Sums over the queries of a batch, accumulated by the kernels.
+struct BatchTotals {
+  unsigned long long cand = 0;         // candidates incl. duplicates
+  unsigned long long unique = 0;       // unique candidates
+  unsigned long long empty = 0;        // probed empty buckets
+  unsigned long long select_ties = 0;  // probe cuts replayed
+  unsigned long long topk_ties = 0;    // top-k lists replayed
+};
+
+// Device words of a batch: the first four 32-bit words (work counter, status,
+// re-hashed tables, unused), then the totals.
+struct BatchCounters {
+  unsigned work, status, tc_exact, pad;
+  BatchTotals totals;
+};
+
 struct BatchResult {
+  BatchTotals totals;  // with want_totals
   int launches = 0;
   int grid = 0;
   bool graph_replayed = false;
@@ -88,7 +107,8 @@ struct BatchWorkspace {
   int mmax = 0;
   int fht = 0;
   int grid = 0;
-  unsigned* counters = nullptr;
+  BatchCounters* counters = nullptr;
+  BatchCounters* h_counters = nullptr;  // pinned copy
   // query order: key per query, histogram of the keys, the permutation
   uint32_t* okey = nullptr;
   uint32_t* ohist = nullptr;
@@ -141,6 +161,12 @@ struct BfWorkspace {
 };
 
 int ensure_lowp_rows(const Params& P, DeviceIndex& di, int mode, cudaStream_t s, Error& err);
+
+// Whether a plain FP32 query (uniform k <= 1024 and qProbes) runs through
+// batch_query: inside its limits, and with its scratch for nq queries within
+// a fixed budget (the three-kernel path sizes its scratch from the candidates
+// it finds, so it reaches further).
+bool plain_through_batch(const Params& P, const DeviceIndex& di, int nq);
 
 int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const BatchRequest& rq, cudaStream_t s,
                 BatchResult& res, Error& err);

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kPcThreads) k_probe_cut(ProbeCutArgs a) {
     run += tot;
   }
   if (__syncthreads_or(tie) && tid == 0) {
+    if (a.totals) atomicAdd(&a.totals->select_ties, 1ull);
     // a tie at the cut: the reference's max-heap of each table's next list
     // entry, popped qProbes times
     int* track = hi + L;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kPcThreads) k_probe_cut(ProbeCutArgs a) {
   __syncthreads();
   const size_t ob = (size_t)q * a.stride;
   run = 0;
+  unsigned empty = 0;
   for (int base = 0; base < Qp; base += kPcThreads) {
     const int p = base + tid;
     uint32_t g = 0, o = 0, sz = 0;
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(kPcThreads) k_probe_cut(ProbeCutArgs a) {
       g = probe[p];
       o = a.bucket_off[g];
       sz = a.bucket_off[g + 1] - o;
+      empty += sz == 0u;
     }
     long long tot;
     const long long ex = block_exclusive_scan((long long)sz, tmp, &tot) + run;
@@ -107,6 +110,7 @@ __global__ void __launch_bounds__(kPcThreads) k_probe_cut(ProbeCutArgs a) {
     }
     run += tot;
   }
+  if (a.totals && empty) atomicAdd(&a.totals->empty, (unsigned long long)empty);
   if (tid == 0) a.pc_n[q] = Qp;
 }
 
@@ -127,6 +131,11 @@ KernelSel pick_kernel_ext(int mode, int d, bool big) {
     if (v32 == 1) return ext_pair<kRowsF32, 1, 1>(big);
     if (v32 == 2) return ext_pair<kRowsF32, 2, 2>(big);
     return ext_pair<kRowsF32, 4, 4>(big);
+  }
+  if (mode == kRowsI8) {
+    if (v32 == 1) return ext_pair<kRowsI8, 1, 1>(big);
+    if (v32 == 2) return ext_pair<kRowsI8, 1, 2>(big);
+    return ext_pair<kRowsI8, 1, 4>(big);
   }
   if (mode == kRowsBF16) {
     if (v32 == 1) return ext_pair<kRowsBF16, 1, 1>(big);

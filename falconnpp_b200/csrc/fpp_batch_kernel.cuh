@@ -39,6 +39,7 @@ struct BatchArgs {
   size_t row_bytes;
   int nchunk;
   const float* Xscale;
+  const float* row_norm_max;  // kRowsI8: the largest row norm
   const uint32_t* flips;
   const uint32_t* bucket_off;
   const int32_t* ids;
@@ -64,6 +65,7 @@ struct BatchArgs {
   int* gheap_i;
   int mmax;
   unsigned int* work;
+  BatchTotals* totals;   // nullable: candidate and tie counts summed over the batch
   unsigned int* status;  // bit 0: candidate capacity overflow; bit 1: per-query k/qProbes out of range
   const uint32_t* order;  // processing order of the queries (nullable: 0, 1, ...)
   const uint32_t* tflips;  // non-null: rotate on the tensor cores when a query keeps one probe per table
@@ -112,6 +114,7 @@ struct ProbeCutArgs {
   uint32_t* pc_pe;
   int* pc_n;
   int stride;  // qprobes_max
+  BatchTotals* totals;  // nullable
 };
 cudaError_t probe_cut_lists(const ProbeCutArgs& a, int nq, cudaStream_t s);
 
@@ -310,6 +313,58 @@ struct FinishShared {
   long long* tmp;
 };
 
+// The top k of the nsel candidates sid / ssc (ids, FP32 score bits) by (score
+// desc, id asc) into orow / ovrow.  Equal scores in the kept list, or at the
+// k-th place, leave the order to the reference's heap: then nothing is
+// written and the result is false.  Every thread of the block calls it.
+template <int GROUPS>
+__device__ __forceinline__ bool write_top_k(const uint32_t* sid, const uint32_t* ssc, unsigned nsel, int k,
+                                            unsigned long long* s_top, int32_t* orow, float* ovrow, int tid) {
+  const unsigned kk = (unsigned)k;
+  const unsigned kept = min(nsel, kk);
+  unsigned dup = 0;
+  // s_top[0..kept): the best candidates by (score desc, id asc).  Equal
+  // FP32 scores in the kept list, or at the k-th place, leave the order to
+  // the reference's heap (dup).
+  if (nsel <= 2u * kBThreads) {
+    // rank by counting: no sort, two barriers
+    for (unsigned i = tid; i < nsel; i += kBThreads) {
+      const uint32_t ki = ord_key_bits(ssc[i]);
+      const uint32_t ii = sid[i];
+      unsigned gt = 0, eq = 0, before = 0;
+      for (unsigned j = 0; j < nsel; ++j) {
+        const uint32_t kj = ord_key_bits(ssc[j]);
+        gt += kj > ki;
+        eq += kj == ki;
+        before += (kj == ki) & (sid[j] < ii);
+      }
+      const unsigned r = gt + before;
+      if (r < kept) s_top[r] = ((unsigned long long)(~ki) << 32) | ii;
+      dup |= (eq > 1u) & (gt < kk);
+    }
+  } else {
+    for (unsigned i = tid; i < nsel; i += kBThreads)
+      s_top[i] = ((unsigned long long)(~ord_key_bits(ssc[i])) << 32) | sid[i];
+    __syncthreads();
+    block_sort_u64(s_top, (int)nsel);
+    for (unsigned i = tid; i + 1 < nsel && i < kk; i += kBThreads)
+      dup |= (s_top[i] >> 32) == (s_top[i + 1] >> 32);
+  }
+  const bool exact = !__syncthreads_or(dup);
+  if (exact) {
+    for (int j = tid; j < k; j += kBThreads) {
+      if ((unsigned)j < kept) {
+        orow[j] = (int32_t)(uint32_t)s_top[j];
+        if (ovrow) ovrow[j] = __uint_as_float(ord_key_inv_dev(~(uint32_t)(s_top[j] >> 32)));
+      } else {
+        orow[j] = 0;
+        if (ovrow) ovrow[j] = 0.0f;
+      }
+    }
+  }
+  return exact;
+}
+
 template <int MODE, int VI32, int GROUPS>
 __device__ __forceinline__ bool finish_query(const BatchArgs& a, const BatchSmem<GROUPS>& sm,
                                              unsigned long long* s_top, uint32_t* uq, uint32_t* sc, unsigned U, int k,
@@ -383,50 +438,11 @@ __device__ __forceinline__ bool finish_query(const BatchArgs& a, const BatchSmem
                                   (size_t)a.ld * 4, a.ld / 4, nullptr, warp, kBWarps, lane, nullptr);
       __syncthreads();
     }
-    const unsigned kept = min(nsel, kk);
-    unsigned dup = 0;
-    // s_top[0..kept): the best candidates by (score desc, id asc).  Equal
-    // FP32 scores in the kept list, or at the k-th place, leave the order to
-    // the reference's heap (dup).
-    if (nsel <= 2u * kBThreads) {
-      // rank by counting: no sort, two barriers
-      for (unsigned i = tid; i < nsel; i += kBThreads) {
-        const uint32_t ki = ord_key_bits(ssc[i]);
-        const uint32_t ii = sid[i];
-        unsigned gt = 0, eq = 0, before = 0;
-        for (unsigned j = 0; j < nsel; ++j) {
-          const uint32_t kj = ord_key_bits(ssc[j]);
-          gt += kj > ki;
-          eq += kj == ki;
-          before += (kj == ki) & (sid[j] < ii);
-        }
-        const unsigned r = gt + before;
-        if (r < kept) s_top[r] = ((unsigned long long)(~ki) << 32) | ii;
-        dup |= (eq > 1u) & (gt < kk);
-      }
-    } else {
-      for (unsigned i = tid; i < nsel; i += kBThreads)
-        s_top[i] = ((unsigned long long)(~ord_key_bits(ssc[i])) << 32) | sid[i];
-      __syncthreads();
-      block_sort_u64(s_top, (int)nsel);
-      for (unsigned i = tid; i + 1 < nsel && i < kk; i += kBThreads)
-        dup |= (s_top[i] >> 32) == (s_top[i + 1] >> 32);
-    }
-    exact = !__syncthreads_or(dup);
-    if (exact) {
-      for (int j = tid; j < k; j += kBThreads) {
-        if ((unsigned)j < kept) {
-          orow[j] = (int32_t)(uint32_t)s_top[j];
-          if (ovrow) ovrow[j] = __uint_as_float(ord_key_inv_dev(~(uint32_t)(s_top[j] >> 32)));
-        } else {
-          orow[j] = 0;
-          if (ovrow) ovrow[j] = 0.0f;
-        }
-      }
-    }
+    exact = write_top_k<GROUPS>(sid, ssc, nsel, k, s_top, orow, ovrow, tid);
   }
   bool bits_dirty = use_bitset;
   if (!exact) {
+    if (a.totals && tid == 0) atomicAdd(&a.totals->topk_ties, 1ull);
     // the reference's min-heap over the candidates in ascending id order
     // (FalconnPP.cpp:633-673): all of them in FP32 mode, the shortlist otherwise
     const bool whole = (MODE == kRowsF32);
@@ -465,6 +481,41 @@ __device__ __forceinline__ bool finish_query(const BatchArgs& a, const BatchSmem
   return bits_dirty;
 }
 
+// The top k of one query from the int8 screen: sc[0..U) holds upper bounds of
+// the exact FP32 scores, the histogram counts the lower bounds by
+// (key >> 16) - base.  The bin of the k-th largest lower bound gives a cut
+// that k exact scores reach, so every candidate of the top k, and every one
+// that ties with its last place, has an upper bound at or above it; those are
+// re-scored in exact FP32 and ranked.  False (and nothing written) when more
+// than kBMaxTop candidates pass or equal scores leave the order to the
+// reference's heap: the caller then scores every candidate in FP32.
+template <int VI32, int GROUPS>
+__device__ __forceinline__ bool finish_screened(const BatchArgs& a, const BatchSmem<GROUPS>& sm,
+                                                unsigned long long* s_top, const uint32_t* uq, const uint32_t* sc,
+                                                unsigned U, int k, int base, int32_t* orow, float* ovrow,
+                                                const FinishShared& fs, int tid, int warp, int lane) {
+  hist_find(sm.hist(), (unsigned)k, fs.tmp, fs.s_bstar, fs.s_above, fs.s_inbin);
+  const uint32_t bstar = *fs.s_bstar;
+  const uint32_t t = bstar == 0u ? 0u : (uint32_t)((int)bstar + base) << 16;
+  if (tid == 0) *fs.s_sel = 0;
+  __syncthreads();
+  uint32_t* sid = sm.sid();
+  uint32_t* ssc = sm.ssc();
+  for (unsigned i = tid; i < U; i += kBThreads) {
+    if (ord_key_bits(sc[i]) >= t) {
+      const unsigned pos = atomicAdd(fs.s_sel, 1u);
+      if (pos < (unsigned)kBMaxTop) sid[pos] = uq[i];
+    }
+  }
+  __syncthreads();
+  const unsigned nsel = *fs.s_sel;
+  if (nsel > (unsigned)kBMaxTop) return false;
+  rerank_rows<kRowsF32, VI32>(sid, nsel, ssc, sm.q, reinterpret_cast<const unsigned char*>(a.Xc), (size_t)a.ld * 4,
+                              a.ld / 4, nullptr, warp, kBWarps, lane, nullptr);
+  __syncthreads();
+  return write_top_k<GROUPS>(sid, ssc, nsel, k, s_top, orow, ovrow, tid);
+}
+
 // HASH: kHashAuto rotates on the tensor cores where a query keeps one probe
 // per table (and a.tflips is set), exactly otherwise; kHashTC only on the
 // tensor cores (the host uses it when every query of the batch keeps one
@@ -495,6 +546,7 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
   __shared__ uint32_t hist[256];
   __shared__ uint32_t s_pre, s_rem;
   __shared__ unsigned s_cnt, s_u, s_sel, s_q, s_ovf, s_bstar, s_above, s_inbin, s_qmax;
+  __shared__ float s_q2, s_r2;  // kRowsI8: |q|^2 and |q - q^|^2
   __shared__ long long tmp[32];
 
   const int tid = threadIdx.x;
@@ -523,6 +575,8 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
     if (tid == 0) {
       s_q = atomicAdd(a.work, 1u);
       s_qmax = 0u;
+      s_q2 = 0.0f;
+      s_r2 = 0.0f;
     }
     __syncthreads();
     const unsigned qu = s_q;
@@ -676,6 +730,7 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
           run += tot;
         }
       } else if (tid == 0) {
+        if (a.totals) atomicAdd(&a.totals->select_ties, 1ull);
         float* hv = sm.phv();
         int* hi = sm.phi();
         int* track = hi + L;
@@ -766,6 +821,7 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
       }
     } else {
       long long run = 0;
+      unsigned empty = 0;
       for (int base = 0; base < Qp; base += kBThreads) {
         const int p = base + tid;
         uint32_t o = 0, sz = 0;
@@ -773,6 +829,7 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
           const uint32_t g = s_probe[p];
           o = a.bucket_off[g];
           sz = a.bucket_off[g + 1] - o;
+          empty += sz == 0u;
           // the bucket's ids (the 16-byte aligned part, at most 16 KB) into L2
           const uint32_t w0 = o & ~3u, w1 = min(o + sz, w0 + 4096u) & ~3u;
           if (w1 > w0) prefetch_l2(a.ids + w0, (w1 - w0) * 4u);
@@ -785,6 +842,7 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
         }
         run += tot;
       }
+      if (a.totals && empty) atomicAdd(&a.totals->empty, (unsigned long long)empty);
     }
     if (tid == 0) {
       s_u = 0;
@@ -916,6 +974,10 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
       __syncthreads();
     }
     const unsigned U = s_u;
+    if (a.totals && tid == 0) {
+      atomicAdd(&a.totals->cand, (unsigned long long)C);
+      atomicAdd(&a.totals->unique, (unsigned long long)U);
+    }
     if (a.dump_counts && tid == 0) {
       a.dump_counts[2 * (size_t)q] = C;
       a.dump_counts[2 * (size_t)q + 1] = U;
@@ -941,35 +1003,86 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
       const float qm = __uint_as_float(s_qmax);
       qscale = qm > 0.0f ? qm / 448.0f : 1.0f;  // 448: largest finite E4M3
     }
-    if (MODE != kRowsF32) fill_query_parts<MODE>(sm.q, qscale, sm.qx);
-    for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
-    __syncthreads();
-    if (MODE == kRowsF32) {
-      rerank_rows<MODE, VI, 2>(uq, U, sc, sm.q, a.Xrows, a.row_bytes, a.nchunk, nullptr, warp, kBWarps, lane,
-                               s_hist);
-    } else if (a.nchunk <= 16 && 9 * 16 * a.row_bytes <= (size_t)(4 * kHT) &&
-               7 * 16 * a.row_bytes <= BatchSmem<GROUPS>::kQ - BatchSmem<GROUPS>::kProbe) {
-      // two tiles in flight per warp, both staged in shared memory that the
-      // rerank leaves idle: the hash-set region (reset at the end of the
-      // query) holds every warp's first stage and warp 7's second, the
-      // probe list, top-k and rotation regions (unused until the shortlist)
-      // the second stages of warps 0..6
-      const size_t sb = 16 * a.row_bytes;
-      unsigned char* st0 = smem_raw + (size_t)warp * sb;
-      unsigned char* st1 = warp < kBWarps - 1 ? smem_raw + BatchSmem<GROUPS>::kProbe + (size_t)warp * sb
-                                              : smem_raw + (size_t)kBWarps * sb;
-      rerank_rows_mma_2stage<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, warp,
-                                   kBWarps, lane, s_hist, st0, st1);
-    } else {
-      rerank_rows_mma<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, warp, kBWarps,
-                            lane, s_hist);
-    }
-    __syncthreads();
-
-    // ---- 5. shortlist by the first scores, exact FP32 re-score, top-k
     const FinishShared fs{hist, &s_pre, &s_rem, &s_cnt, &s_sel, &s_bstar, &s_above, &s_inbin, tmp};
-    const bool bits_dirty =
-        finish_query<MODE, VI32, GROUPS>(a, sm, s_top, uq, sc, U, k, orow, ovrow, use_bitset, bits, fs, tid, warp, lane);
+    // two tiles in flight per warp, both staged in shared memory that the
+    // rerank leaves idle: the hash-set region (reset at the end of the
+    // query) holds every warp's first stage and warp 7's second, the
+    // probe list, top-k and rotation regions (unused until the shortlist)
+    // the second stages of warps 0..6
+    const bool staged = a.nchunk <= 16 && 9 * 16 * a.row_bytes <= (size_t)(4 * kHT) &&
+                        7 * 16 * a.row_bytes <= BatchSmem<GROUPS>::kQ - BatchSmem<GROUPS>::kProbe;
+    unsigned char* st0 = smem_raw + (size_t)warp * 16 * a.row_bytes;
+    unsigned char* st1 = warp < kBWarps - 1 ? smem_raw + BatchSmem<GROUPS>::kProbe + (size_t)warp * 16 * a.row_bytes
+                                            : smem_raw + (size_t)kBWarps * 16 * a.row_bytes;
+    bool bits_dirty = use_bitset;
+    if constexpr (MODE == kRowsI8) {
+      // exact FP32 scores of the candidates that can reach the top k: the
+      // int8 rows (a quarter of the FP32 bytes) bound every score, and only
+      // the rows whose upper bound reaches the k-th lower bound are read in
+      // FP32.  The gathered-row bytes bound this phase: 3,000 queries at
+      // qProbes 80 on 1M x 200 took 3.86 ms with every row read in FP32 and
+      // take 3.06 ms.  Few candidates (at most 4 k) go straight to FP32: most of them
+      // would be read twice.
+      bool done = false;
+      if (U > 4u * (unsigned)k) {
+        for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
+        const float qmax = __uint_as_float(s_qmax);
+        float2 sums = fill_query_parts_i8(sm.q, qmax, sm.qx);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          sums.x += __shfl_xor_sync(kFullMask, sums.x, o);
+          sums.y += __shfl_xor_sync(kFullMask, sums.y, o);
+        }
+        if (lane == 0) {
+          atomicAdd(&s_q2, sums.x);
+          atomicAdd(&s_r2, sums.y);
+        }
+        __syncthreads();
+        ScreenArgs scr;
+        scr.qs = __fdiv_rn(__fdiv_rn(qmax, 127.0f), 254.0f);
+        scr.qn = sqrtf(s_q2) * (1.0f + 0x1p-10f);
+        const float smax = scr.qn * __ldg(a.row_norm_max) * 1.01f;  // no score is larger
+        // block-uniform: both values come from shared memory and the index
+        if (s_r2 <= s_q2 * (0.95f * kScreenQRel * kScreenQRel) && scr.qn > 1e-18f && smax < 1e30f) {
+          scr.base = (int)(ord_key(smax) >> 16) - (kHistBins - 1);
+          if (staged)
+            rerank_rows_mma_2stage<kRowsI8>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, nullptr, 1.0f, warp,
+                                            kBWarps, lane, s_hist, st0, st1, scr);
+          else
+            rerank_rows_mma<kRowsI8>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, nullptr, 1.0f, warp, kBWarps,
+                                     lane, s_hist, scr);
+          __syncthreads();
+          done = finish_screened<VI32, GROUPS>(a, sm, s_top, uq, sc, U, k, scr.base, orow, ovrow, fs, tid, warp, lane);
+        }
+      }
+      if (!done) {
+        for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
+        __syncthreads();
+        rerank_rows<kRowsF32, VI32, 1>(uq, U, sc, sm.q, reinterpret_cast<const unsigned char*>(a.Xc), (size_t)a.ld * 4,
+                                       a.ld / 4, nullptr, warp, kBWarps, lane, s_hist);
+        __syncthreads();
+        bits_dirty = finish_query<kRowsF32, VI32, GROUPS>(a, sm, s_top, uq, sc, U, k, orow, ovrow, use_bitset, bits, fs,
+                                                          tid, warp, lane);
+      }
+    } else {
+      if (MODE != kRowsF32) fill_query_parts<MODE>(sm.q, qscale, sm.qx);
+      for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
+      __syncthreads();
+      if (MODE == kRowsF32) {
+        rerank_rows<MODE, VI, 2>(uq, U, sc, sm.q, a.Xrows, a.row_bytes, a.nchunk, nullptr, warp, kBWarps, lane,
+                                 s_hist);
+      } else if (staged) {
+        rerank_rows_mma_2stage<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, warp,
+                                     kBWarps, lane, s_hist, st0, st1);
+      } else {
+        rerank_rows_mma<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, warp, kBWarps,
+                              lane, s_hist);
+      }
+      __syncthreads();
+      // ---- 5. shortlist by the first scores, exact FP32 re-score, top-k
+      bits_dirty = finish_query<MODE, VI32, GROUPS>(a, sm, s_top, uq, sc, U, k, orow, ovrow, use_bitset, bits, fs, tid,
+                                                    warp, lane);
+    }
     // ---- 6. leave the hash set empty and the bitset clear
     {
       const uint4 e4 = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);

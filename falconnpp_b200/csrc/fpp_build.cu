@@ -72,21 +72,124 @@ __global__ void k_center_final(const float* __restrict__ part, long long nchunks
   mean[j] = __fdiv_rn(s, (float)n);
 }
 
-__global__ void k_center_apply(const float* __restrict__ X, long long n, int d, int ld,
-                               const float* __restrict__ mean, float* __restrict__ Xc, int* __restrict__ bad) {
-  const long long total = n * (long long)ld;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long i = t / ld;
-    const int j = (int)(t - i * ld);
-    float v = 0.0f;
-    if (j < d) {
-      const float x = X[i * d + j];
-      if (!isfinite(x)) atomicOr(bad, 1);
-      v = __fsub_rn(x, mean[j]);
+// One warp per row, four consecutive elements per lane and step.  APPLY: Xc =
+// X - mean (row stride ld, zero padded), flag non-finite values; otherwise Xc
+// is read.  With `i8`, the row's int8 copy for the screen of the FP32 form
+// (fpp_rows.cuh: head, then rint(x / scale)) and the largest row norm.  Bound
+// by HBM: one read of the row and one write of each copy (550 us at 1M x 200
+// with the int8 copy; an element per thread without it took 721 us).
+template <bool APPLY>
+__global__ void __launch_bounds__(256) k_center_rows(const float* __restrict__ X, long long n, int d, int ld,
+                                                     const float* __restrict__ mean, float* __restrict__ Xc,
+                                                     unsigned char* __restrict__ i8, int i8_bytes,
+                                                     float* __restrict__ norm_max, int* __restrict__ bad) {
+  constexpr int NC = 4;  // float4 chunks per lane held in registers (d <= 512)
+  const int lane = threadIdx.x & 31;
+  const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int nchunk = ld >> 2;
+  const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  float nmax = 0.0f;
+  bool nonfinite = false;
+  auto centred = [&](long long i, int c) {  // chunk c of row i of X - mean, zero past d
+    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float* p = X + i * d + 4 * c;
+    const float* m = mean + 4 * c;
+    if (vec) {
+      x = __ldg(reinterpret_cast<const float4*>(p));
+    } else {
+      x.x = p[0];  // ld - d < 4: the first element of a chunk is inside
+      if (4 * c + 1 < d) x.y = p[1];
+      if (4 * c + 2 < d) x.z = p[2];
+      if (4 * c + 3 < d) x.w = p[3];
     }
-    Xc[t] = v;
+    nonfinite |= !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z) && isfinite(x.w));
+    x.x = __fsub_rn(x.x, m[0]);
+    if (4 * c + 1 < d) x.y = __fsub_rn(x.y, m[1]);
+    if (4 * c + 2 < d) x.z = __fsub_rn(x.z, m[2]);
+    if (4 * c + 3 < d) x.w = __fsub_rn(x.w, m[3]);
+    return x;
+  };
+  for (long long i = w; i < n; i += nw) {
+    float4 v[NC];
+    float mx = 0.0f, ss = 0.0f;
+    float4* orow = reinterpret_cast<float4*>(Xc + i * ld);
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      const int c = lane + 32 * e;
+      v[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (c < nchunk) {
+        if (APPLY) {
+          v[e] = centred(i, c);
+          orow[c] = v[e];
+        } else {
+          v[e] = orow[c];
+        }
+      }
+      mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[e].x), fabsf(v[e].y))), fmaxf(fabsf(v[e].z), fabsf(v[e].w)));
+      ss = fmaf(v[e].x, v[e].x, fmaf(v[e].y, v[e].y, fmaf(v[e].z, v[e].z, fmaf(v[e].w, v[e].w, ss))));
+    }
+    if (APPLY)
+      for (int c = lane + 32 * NC; c < nchunk; c += 32) orow[c] = centred(i, c);  // d > 512: no int8 copy
+    if (!i8) continue;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      mx = fmaxf(mx, __shfl_xor_sync(kFullMask, mx, o));
+      ss += __shfl_xor_sync(kFullMask, ss, o);
+    }
+    // whatever the rounding of inv, the residual below is that of the int8
+    // values stored
+    const float s = mx / 127.0f;
+    const float inv = s > 0.0f ? 1.0f / s : 0.0f;
+    float rr = 0.0f;
+    unsigned char* row = i8 + (size_t)i * i8_bytes;
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      const int c = lane + 32 * e;
+      const float x[4] = {v[e].x, v[e].y, v[e].z, v[e].w};
+      uint32_t pack = 0;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int qv = max(-127, min(127, __float2int_rn(x[t] * inv)));
+        const float r = fmaf(-(float)qv, s, x[t]);
+        rr = fmaf(r, r, rr);
+        pack |= (uint32_t)(qv & 255) << (8 * t);
+      }
+      if (8 + 4 * c < i8_bytes) *reinterpret_cast<uint32_t*>(row + 8 + 4 * c) = pack;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) rr += __shfl_xor_sync(kFullMask, rr, o);
+    const float nrm = sqrtf(ss) * (1.0f + 0x1p-10f);
+    // the bound of the row's part of a score's error (kScreenRel in
+    // fpp_rows.cuh); a row whose sums overflow gets +inf and is never screened
+    // out.  The squares of a tiny row underflow: 1e-18 bounds what is lost.
+    float err = (sqrtf(rr) + 1e-18f) * (1.0f + 0x1p-9f) + (nrm + 1e-18f) * (1.0f / 2048.0f);
+    if (!(err < 1e30f)) err = __int_as_float(0x7f800000);
+    if (lane == 0) *reinterpret_cast<float2*>(row) = make_float2(s, err);
+    nmax = fmaxf(nmax, nrm < 1e30f ? nrm : __int_as_float(0x7f800000));  // NaN: +inf
   }
+  if (bad && __any_sync(kFullMask, nonfinite) && lane == 0) atomicOr(bad, 1);
+  if (i8 && lane == 0) atomicMax(reinterpret_cast<unsigned*>(norm_max), __float_as_uint(nmax));  // >= 0: bits order
+}
+
+static bool alloc_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
+  if (P.n_features > 512) return false;
+  const size_t bytes = (size_t)P.n_points * i8_row_bytes(P.n_features);
+  if (dev_malloc(&di.i8_norm_max, sizeof(float)) == cudaSuccess && dev_malloc(&di.Xi8, bytes) == cudaSuccess &&
+      cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s) == cudaSuccess)
+    return true;
+  cudaGetLastError();  // the FP32 form works without the copy
+  cudaFree(di.Xi8);
+  cudaFree(di.i8_norm_max);
+  di.Xi8 = nullptr;
+  di.i8_norm_max = nullptr;
+  return false;
+}
+
+void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
+  if (!alloc_screen_rows(P, di, s)) return;
+  k_center_rows<false><<<1184, 256, 0, s>>>(nullptr, P.n_points, P.n_features, di.ld, nullptr, di.Xc, di.Xi8,
+                                            i8_row_bytes(P.n_features), di.i8_norm_max, nullptr);
 }
 
 // ---------------------------------------------------------------- hashing
@@ -546,6 +649,8 @@ void free_index(DeviceIndex& di) {
   cudaFree(di.ids);
   cudaFree(di.Xlp);
   cudaFree(di.Xlp_scale);
+  cudaFree(di.Xi8);
+  cudaFree(di.i8_norm_max);
   di = DeviceIndex();
 }
 
@@ -654,7 +759,9 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     dim3 g1((unsigned)nchunks_c, (unsigned)((d + 255) / 256));
     k_center_partial<<<g1, 256, 0, s>>>(Xd, n, d, part);
     k_center_final<<<(d + 255) / 256, 256, 0, s>>>(part, nchunks_c, n, d, di.center);
-    k_center_apply<<<(unsigned)std::max(1, nsm * 8), 256, 0, s>>>(Xd, n, d, ld, di.center, di.Xc, d_bad);
+    alloc_screen_rows(P, di, s);
+    k_center_rows<true><<<(unsigned)std::max(1, nsm * 8), 256, 0, s>>>(Xd, n, d, ld, di.center, di.Xc, di.Xi8,
+                                                                       i8_row_bytes(d), di.i8_norm_max, d_bad);
     FPP_CUDA(cudaGetLastError());
     FPP_CUDA(cudaMemcpyAsync(&h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));

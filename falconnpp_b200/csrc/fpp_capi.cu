@@ -156,33 +156,39 @@ void set_batch_stats(fpp_index* h, const fpp::BatchResult& res) {
   h->qst.tc_exact = res.tc_exact;
 }
 
-// Runs the batched form for device queries/outputs (uniform k, the handle's
-// qProbes).  With check_status false the call does not wait for the kernel;
-// the caller reads the status words (h->bw.counters + 1) after its own copies
-// and reports an overflow with batched_overflow_error().
-int run_batched(fpp_index* h, const float* dQ, int nq, int k, int32_t* dout, cudaStream_t s,
-                bool check_status = true, const float* Q_host = nullptr, cudaStream_t copy_stream = nullptr) {
+// Runs the batched kernels for device queries/outputs (uniform k, the
+// handle's qProbes).  With Q_host / out_host the queries are copied in (in
+// chunks that overlap the hashing) and the results copied out; either way the
+// call returns once the results are written.  plain: the FP32 form with the
+// three-kernel path's statistics, whatever the handle's batched options.
+int run_batched(fpp_index* h, const float* dQ, int nq, int k, int32_t* dout, cudaStream_t s, bool plain,
+                const float* Q_host = nullptr, int32_t* out_host = nullptr, cudaStream_t copy_stream = nullptr) {
   fpp::BatchRequest rq;
   rq.Q = dQ;
   rq.Q_host = Q_host;
+  rq.out_host = out_host;
   rq.copy_stream = copy_stream;
   rq.nq = nq;
   rq.k_uniform = k;
   rq.qprobes_uniform = h->P.qProbes;
   rq.k_max = k;
   rq.qprobes_max = h->P.qProbes;
-  rq.mode = h->precision;
-  rq.shortlist_mult = h->shortlist_mult;
   rq.out = dout;
   rq.out_stride = k;
-  rq.use_graph = h->use_graph;
-  rq.blocks_per_sm = h->blocks_per_sm;
-  rq.reorder = h->reorder;
-  rq.tc_rotation = h->tc_rotation;
-  rq.split_hash = h->split_hash;
   rq.tc_hash = h->tc_hash;
   rq.stage_timing = h->ws.stage_timing;
-  rq.check_status = check_status;
+  if (plain) {
+    rq.mode = fpp::kRerankFP32;
+    rq.want_totals = true;
+  } else {
+    rq.mode = h->precision;
+    rq.shortlist_mult = h->shortlist_mult;
+    rq.use_graph = h->use_graph;
+    rq.blocks_per_sm = h->blocks_per_sm;
+    rq.reorder = h->reorder;
+    rq.tc_rotation = h->tc_rotation;
+    rq.split_hash = h->split_hash;
+  }
   fpp::BatchResult res;
   fpp::Error err{0, ""};
   const int rc = fpp::batch_query(h->P, h->di, h->bw, rq, s, res, err);
@@ -190,6 +196,13 @@ int run_batched(fpp_index* h, const float* dQ, int nq, int k, int32_t* dout, cud
   if (res.overflow) return fail(FPP_ERR_UNSUPPORTED, "batched query: candidate capacity exceeded");
   set_batch_stats(h, res);
   h->qst.total_probes = (long long)nq * h->P.qProbes;
+  if (plain) {
+    h->qst.total_cand = (long long)res.totals.cand;
+    h->qst.total_unique = (long long)res.totals.unique;
+    h->qst.total_empty = (long long)res.totals.empty;
+    h->qst.n_select_ties = (int)res.totals.select_ties;
+    h->qst.n_topk_ties = (int)res.totals.topk_ties;
+  }
   return FPP_OK;
 }
 
@@ -381,8 +394,9 @@ int fpp_query(fpp_index* h, const float* queries, int n_queries, int n_neighbors
   }
   const auto t0 = std::chrono::high_resolution_clock::now();
   fpp::Error err{0, ""};
-  if (h->form == 1 && n_queries > 0) {
-    // batched form: stage the queries and results through the workspace
+  const bool plain = h->form == 0;
+  if (n_queries > 0 && (!plain || fpp::plain_through_batch(P, h->di, n_queries))) {
+    // stage the queries and results through the workspace
     size_t capq = h->ws.cap_Qd, capo = h->ws.cap_out;
     cudaError_t e = cudaSuccess;
     if ((size_t)n_queries * P.n_features > capq) {
@@ -402,18 +416,8 @@ int fpp_query(fpp_index* h, const float* queries, int n_queries, int n_neighbors
     if (e != cudaSuccess) return fail(FPP_ERR_OUT_OF_MEMORY, std::string("query: ") + cudaGetErrorString(e));
     if (!h->cstream && cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking) != cudaSuccess)
       h->cstream = nullptr;
-    // the queries are copied by the batched form itself (in chunks that
-    // overlap the hashing); one synchronisation: results and the kernel's
-    // status words come back together
-    rc = run_batched(h, h->ws.Qd, n_queries, n_neighbors, h->ws.out, h->stream, false, queries, h->cstream);
+    rc = run_batched(h, h->ws.Qd, n_queries, n_neighbors, h->ws.out, h->stream, plain, queries, out, h->cstream);
     if (rc) return rc;
-    unsigned status = 0;
-    e = cudaMemcpyAsync(out, h->ws.out, sizeof(int32_t) * n_queries * n_neighbors, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&status, h->bw.counters + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) return fail(FPP_ERR_CUDA, std::string("query: ") + cudaGetErrorString(e));
-    if (status & 1u) return fail(FPP_ERR_UNSUPPORTED, "batched query: candidate capacity exceeded");
   } else {
     rc = fpp::query_index(P, h->di, queries, false, n_queries, n_neighbors, out, false, h->ws, h->qst, h->stream,
                           err, nullptr);
@@ -450,8 +454,8 @@ int fpp_query_device(fpp_index* h, const float* d_queries, int n_queries, int n_
   if (use_device(h)) return FPP_ERR_CUDA;
   cudaStream_t s = stream ? (cudaStream_t)stream : h->stream;
   fpp::Error err{0, ""};
-  if (h->form == 1) {
-    rc = run_batched(h, d_queries, n_queries, n_neighbors, d_out, s);
+  if (h->form == 1 || fpp::plain_through_batch(h->P, h->di, n_queries)) {
+    rc = run_batched(h, d_queries, n_queries, n_neighbors, d_out, s, h->form == 0);
     if (rc) return rc;
     return ok();
   }

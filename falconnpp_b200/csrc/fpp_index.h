@@ -73,7 +73,14 @@ struct DeviceIndex {
   float* Xlp_scale = nullptr;        // per-row FP32 scale (fp8)
   int lp_mode = kRerankFP32;
   int ld_lp = 0;
+  // int8 rows that screen the FP32 form's candidates (null: not available,
+  // the form then scores every candidate in FP32), and the largest row norm
+  unsigned char* Xi8 = nullptr;      // [n][i8_row_bytes(d)]
+  float* i8_norm_max = nullptr;
 };
+
+// Bytes of an int8 screening row: an 8-byte head and d elements, padded to 16.
+inline int i8_row_bytes(int d) { return (d + 8 + 15) & ~15; }
 
 struct BuildStats {
   double ms_center = 0, ms_hash = 0, ms_sort = 0, ms_csr = 0, ms_total = 0;
@@ -97,6 +104,11 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
                 int32_t* dump_codes, float* dump_scores);
 
 void free_index(DeviceIndex& di);
+
+// The int8 screening rows of the centred data di.Xc (asynchronous on s).
+// Only for d <= 512, the batched form's range.  A failed allocation leaves
+// the index without them.
+void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s);
 
 // The sign flip words (and, for fhtDim 256, their per-view copy for the
 // tensor-core rotation) from the sign bits, into di.flips / di.tflips;

@@ -227,6 +227,11 @@ int fpp_load(fpp_index* h, const char* path) {
     return fail(FPP_ERR_INVALID_ARGUMENT, std::string("load: ") + path + ": " + why);
   }
   di.max_kept = max_kept;
+  fpp::make_screen_rows(P, di, h->stream);
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
+    fpp::free_index(di);
+    return fail(FPP_ERR_CUDA, "load: the device failed");
+  }
   h->P = P;
   h->params_set = true;
   h->bits = std::move(bits);

@@ -20,7 +20,9 @@
 
 namespace fpp {
 
-enum RowMode : int { kRowsF32 = 0, kRowsBF16 = 1, kRowsFP8 = 2 };
+// kRowsI8: the FP32 form screened by int8 rows (exact FP32 results; an
+// internal kernel mode, not a precision a caller selects).
+enum RowMode : int { kRowsF32 = 0, kRowsBF16 = 1, kRowsFP8 = 2, kRowsI8 = 3 };
 constexpr uint32_t kNoRow = 0xffffffffu;
 
 template <int MODE>
@@ -208,10 +210,18 @@ __device__ __forceinline__ void mma_e4m3_m16n8k32(float (&d)[4], uint32_t a0, ui
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void mma_s8_m16n8k32(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 template <int MODE>
 struct QueryParts {
-  static constexpr int NP = MODE == kRowsBF16 ? 2 : 3;   // B columns in use
-  static constexpr int PC = MODE == kRowsBF16 ? 64 : 32; // 16-byte chunks per part (d <= 512)
+  static constexpr int NP = MODE == kRowsFP8 ? 3 : 2;   // B columns in use
+  // 16-byte chunks per part (d <= 512; an int8 row starts with 8 bytes that are not elements)
+  static constexpr int PC = MODE == kRowsBF16 ? 64 : MODE == kRowsFP8 ? 32 : 36;
   static constexpr int EPC = RowFmt<MODE>::EPC;
   static constexpr int kBytes = NP * PC * 16;
 };
@@ -244,11 +254,78 @@ __device__ __forceinline__ void fill_query_parts(const float* qs, float qscale, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Int8 screen of the FP32 form.  A stored row is [scale f32][err f32][d int8,
+// zero padded to 16 bytes]: x^ = scale * int8 with scale = max|x| / 127, and
+// err bounds the row's part of the score error per unit of query norm,
+//   err = |x - x^| (1 + 2^-10) + |x| 2^-11          (kScreenRel)
+// The query is q^ = (qmax / 127) (q1 + q2 / 254) in two int8 parts; products
+// and sums are exact integers, so a score's distance from the exact FP32 dot
+// of the parity order is at most |q| |x - x^| + |q - q^| |x^| + rounding:
+// |q| err as long as |q - q^| <= |q| kScreenQRel (checked per query), since
+// the FP32 dot (at most 21 roundings on the longest path for d <= 512) and the
+// few roundings here stay below 2^-17 |q| |x|.
+constexpr float kScreenRel = 1.0f / 2048.0f;
+constexpr float kScreenQRel = 1.0f / 2048.0f - 1.0f / 65536.0f;
+
+struct ScreenArgs {
+  float qs;    // (qmax / 127) / 254
+  float qn;    // |q|, rounded up
+  int base;    // key >> 16 of the score that bin 0 holds
+};
+
+// The first int8 element of a row or a query part.
+constexpr int kI8Head = 8;
+
+// Upper bound of a row's score to score[r]; its lower bound into the
+// 2048-bin histogram of key >> 16 (7 mantissa bits: bins of 0.8 %), bin 0
+// holding everything from 16 octaves below the largest possible score down.
+// A row whose bound is not usable (non-finite data, a product near overflow)
+// gets +inf, so it is always re-scored.
+__device__ __forceinline__ void screen_put(uint32_t* score, unsigned r, int hi, int lo, float sx, float ex,
+                                           const ScreenArgs& sa, uint32_t* hist) {
+  const float s = __fmul_rn((float)(hi * 254 + lo), __fmul_rn(sx, sa.qs));
+  const float raw = __fmul_rn(sa.qn, ex);
+  const bool ok = raw < 1e30f;
+  const float dl = fmaxf(raw, 1e-30f);
+  const float up = ok ? __fadd_rn(s, dl) : __int_as_float(0x7f800000);
+  const float lw = ok ? __fsub_rn(s, dl) : __int_as_float((int)0xff800000u);
+  score[r] = __float_as_uint(up);
+  const int b = (int)(ord_key_bits(__float_as_uint(lw)) >> 16) - sa.base;
+  atomicAdd(hist + min(max(b, 0), 2047), 1u);
+}
+
+// The query's int8 parts into qx (zero head and padding included); returns
+// this thread's share of |q|^2 and |q - q^|^2.
+__device__ __forceinline__ float2 fill_query_parts_i8(const float* qs, float qmax, unsigned char* qx) {
+  using P = QueryParts<kRowsI8>;
+  constexpr int per_part = P::PC * 16;
+  const float s1 = qmax / 127.0f;
+  const float s2 = s1 / 254.0f;
+  float2 sums = make_float2(0.0f, 0.0f);
+  for (int e = threadIdx.x; e < per_part; e += blockDim.x) {
+    int v1 = 0, v2 = 0;
+    if (e >= kI8Head) {
+      const float x = qs[e - kI8Head];
+      if (s1 > 0.0f) {
+        v1 = max(-127, min(127, __float2int_rn(__fdiv_rn(x, s1))));
+        v2 = s2 > 0.0f ? max(-127, min(127, __float2int_rn(__fdiv_rn(fmaf(-(float)v1, s1, x), s2)))) : 0;
+      }
+      const float res = fmaf(-(float)v2, s2, fmaf(-(float)v1, s1, x));
+      sums.x = fmaf(x, x, sums.x);
+      sums.y = fmaf(res, res, sums.y);
+    }
+    qx[e] = (unsigned char)(signed char)v1;
+    qx[per_part + e] = (unsigned char)(signed char)v2;
+  }
+  return sums;
+}
+
 template <int MODE>
 __device__ __forceinline__ void rerank_rows_mma(const uint32_t* ids, unsigned U, uint32_t* score,
                                                 const unsigned char* qx, const unsigned char* rows, size_t row_bytes,
                                                 int nchunk, const float* scale, float qscale, int warp, int nwarps,
-                                                int lane, uint32_t* hist11) {
+                                                int lane, uint32_t* hist11, const ScreenArgs& scr = ScreenArgs()) {
   using P = QueryParts<MODE>;
   const int g = lane >> 2;
   const int c = lane & 3;
@@ -303,6 +380,8 @@ __device__ __forceinline__ void rerank_rows_mma(const uint32_t* ids, unsigned U,
     const uint4* p0 = reinterpret_cast<const uint4*>(rows + (size_t)id0 * row_bytes) + c;
     const uint4* p1 = reinterpret_cast<const uint4*>(rows + (size_t)id1 * row_bytes) + c;
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int iacc[4] = {0, 0, 0, 0};
+    float e0 = 0.0f, e1 = 0.0f;
     for (int j0 = 0; j0 < JN; j0 += 4) {
       uint4 x0[4], x1[4];
 #pragma unroll
@@ -311,11 +390,20 @@ __device__ __forceinline__ void rerank_rows_mma(const uint32_t* ids, unsigned U,
         x0[jj] = (ok && l0) ? __ldg(p0 + 4 * (j0 + jj)) : zero;
         x1[jj] = (ok && l1) ? __ldg(p1 + 4 * (j0 + jj)) : zero;
       }
+      if (MODE == kRowsI8 && j0 == 0) {  // lane c = 0 holds chunk 0, the row's head
+        f0 = __uint_as_float(x0[0].x);
+        e0 = __uint_as_float(x0[0].y);
+        f1 = __uint_as_float(x1[0].x);
+        e1 = __uint_as_float(x1[0].y);
+      }
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
         if (j0 + jj < JN) {
-          const uint4 b = g < P::NP ? qpart[4 * (j0 + jj)] : zero;
-          if (MODE == kRowsBF16) {
+          const uint4 b = g < P::NP && 4 * (j0 + jj) + c < P::PC ? qpart[4 * (j0 + jj)] : zero;
+          if (MODE == kRowsI8) {
+            mma_s8_m16n8k32(iacc, x0[jj].x, x1[jj].x, x0[jj].y, x1[jj].y, b.x, b.y);
+            mma_s8_m16n8k32(iacc, x0[jj].z, x1[jj].z, x0[jj].w, x1[jj].w, b.z, b.w);
+          } else if (MODE == kRowsBF16) {
             mma_bf16_m16n8k16(acc, x0[jj].x, x1[jj].x, x0[jj].y, x1[jj].y, b.x, b.y);
             mma_bf16_m16n8k16(acc, x0[jj].z, x1[jj].z, x0[jj].w, x1[jj].w, b.z, b.w);
           } else {
@@ -324,6 +412,13 @@ __device__ __forceinline__ void rerank_rows_mma(const uint32_t* ids, unsigned U,
           }
         }
       }
+    }
+    if (MODE == kRowsI8) {  // parts 0 and 1 of the query are columns 0 and 1: lane c = 0
+      if (c == 0) {
+        if (l0) screen_put(score, r0, iacc[0], iacc[1], f0, e0, scr, hist11);
+        if (l1) screen_put(score, r1, iacc[2], iacc[3], f1, e1, scr, hist11);
+      }
+      continue;
     }
     // row g: columns 2c, 2c+1 in acc[0..1]; row g + 8 in acc[2..3]
     float s0 = acc[0] + acc[1];
@@ -380,7 +475,8 @@ __device__ __forceinline__ void rerank_rows_mma_2stage(const uint32_t* ids, unsi
                                                        const unsigned char* qx, const unsigned char* rows,
                                                        size_t row_bytes, int nchunk, const float* scale, float qscale,
                                                        int warp, int nwarps, int lane, uint32_t* hist11,
-                                                       unsigned char* stage0, unsigned char* stage1) {
+                                                       unsigned char* stage0, unsigned char* stage1,
+                                                       const ScreenArgs& scr = ScreenArgs()) {
   using P = QueryParts<MODE>;
   const int g = lane >> 2;
   const int c = lane & 3;
@@ -426,6 +522,8 @@ __device__ __forceinline__ void rerank_rows_mma_2stage(const uint32_t* ids, unsi
   // (row g: columns 2c, 2c+1 in acc[0..1]; row g + 8 in acc[2..3])
   auto compute = [&](unsigned t, uint32_t sa, uint32_t i0, uint32_t i1, float f0, float f1) {
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    int iacc[4] = {0, 0, 0, 0};
+    float e0 = 0.0f, e1 = 0.0f;
 #pragma unroll
     for (int jj = 0; jj < 4; ++jj) {
       if (jj < JN) {
@@ -433,7 +531,16 @@ __device__ __forceinline__ void rerank_rows_mma_2stage(const uint32_t* ids, unsi
         const uint4 a0 = (ok && i0 != kNoRow) ? ld_shared_u4(sa + 64u * jj) : zero;
         const uint4 a1 = (ok && i1 != kNoRow) ? ld_shared_u4(sa + rb8 + 64u * jj) : zero;
         const uint4 b = g < P::NP ? qpart[4 * jj] : zero;
-        if (MODE == kRowsBF16) {
+        if (MODE == kRowsI8) {
+          if (jj == 0) {  // lane c = 0 holds chunk 0, the row's head
+            f0 = __uint_as_float(a0.x);
+            e0 = __uint_as_float(a0.y);
+            f1 = __uint_as_float(a1.x);
+            e1 = __uint_as_float(a1.y);
+          }
+          mma_s8_m16n8k32(iacc, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
+          mma_s8_m16n8k32(iacc, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
+        } else if (MODE == kRowsBF16) {
           mma_bf16_m16n8k16(acc, a0.x, a1.x, a0.y, a1.y, b.x, b.y);
           mma_bf16_m16n8k16(acc, a0.z, a1.z, a0.w, a1.w, b.z, b.w);
         } else {
@@ -444,6 +551,13 @@ __device__ __forceinline__ void rerank_rows_mma_2stage(const uint32_t* ids, unsi
     }
     const unsigned r0 = t * 16u + g;
     const unsigned r1 = r0 + 8u;
+    if (MODE == kRowsI8) {  // parts 0 and 1 of the query are columns 0 and 1: lane c = 0
+      if (c == 0) {
+        if (r0 < U) screen_put(score, r0, iacc[0], iacc[1], f0, e0, scr, hist11);
+        if (r1 < U) screen_put(score, r1, iacc[2], iacc[3], f1, e1, scr, hist11);
+      }
+      return;
+    }
     float s0 = acc[0] + acc[1];
     float s1 = acc[2] + acc[3];
     s0 += __shfl_xor_sync(0xffffffffu, s0, 1);

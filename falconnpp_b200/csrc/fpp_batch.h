@@ -148,8 +148,9 @@ struct BatchWorkspace {
   void release();
 };
 
-// Scratch of the brute-force low-precision block kernel (fpp_bf_lowp.cu):
-// query rows, per-query scales, the per-(query, split) shortlist heaps.
+// Scratch of the brute-force low-precision block kernels (fpp_bf_lowp.cu):
+// query rows, per-query scales, the candidate lists (per query, or per query
+// and segment).
 struct BfWorkspace {
   unsigned char* qrows = nullptr;
   float* qscale = nullptr;
@@ -157,6 +158,15 @@ struct BfWorkspace {
   int* heap_n = nullptr;
   unsigned* status = nullptr;
   size_t cap_q = 0, cap_qs = 0, cap_hv = 0, cap_n = 0;
+  // threshold scan: sampled tile maxima, thresholds, the queries it reports
+  // (count, then indexes), and those queries with their results
+  float* tmax = nullptr;
+  float* thr = nullptr;
+  unsigned* fail = nullptr;
+  float* fq = nullptr;
+  int32_t* fo = nullptr;
+  float* fv = nullptr;
+  size_t cap_t = 0, cap_thr = 0, cap_f = 0, cap_fq = 0, cap_fo = 0, cap_fv = 0;
   void release();
 };
 

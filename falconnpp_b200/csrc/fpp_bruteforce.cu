@@ -8,7 +8,9 @@
 //                 best k of its slice in shared memory: candidates above the
 //                 running k-th score are appended to a buffer that is sorted
 //                 and cut back to k when it fills;
-//   k_bf_merge:   one block per query merges the slices' best-k lists.
+//   k_bf_merge:   one block per query merges the slices' best-k lists;
+//   k_bf_rescore: the FP64 scores of a query's candidates only, where the
+//                 tensor-core scan of fpp_bf_scan.h has found them.
 // FP64 is used only here.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -17,6 +19,7 @@
 #include <string>
 
 #include "../../include/falconnpp_b200.h"
+#include "fpp_bf_scan.h"
 #include "fpp_handle.h"
 
 namespace fpp {
@@ -181,23 +184,84 @@ __global__ void __launch_bounds__(kBfThreads) k_bf_merge(const unsigned long lon
   }
 }
 
-}  // namespace
-}  // namespace fpp
+// k_bf_rescore — one block per query: the FP64 inner products of the query's
+// candidates (the same order as k_bf_partial: the same bits), ranked by (score
+// desc, id asc).  A query whose list overflowed, or without k scores at its
+// threshold, goes to `fail` (count, then indexes).
+constexpr int kRescoreMax = 2048;
 
-extern "C" int fpp_bruteforce_topk_f64(const float* d_X, long long n_points, int n_features, const float* d_Q,
-                                       int n_queries, int k, int32_t* d_out, double* d_out_val, void* stream) {
-  using namespace fpp;
-  if (!d_X || !d_Q || !d_out || n_points < 1 || n_features < 1 || n_queries < 0)
-    return set_last_error(FPP_ERR_INVALID_ARGUMENT, "bruteforce: NULL buffer or bad sizes");
-  if (k < 1 || k > kBfMaxK || k > n_points)
-    return set_last_error(FPP_ERR_INVALID_ARGUMENT, "bruteforce: need 1 <= k <= min(256, n_points)");
-  if (n_features > 1024) return set_last_error(FPP_ERR_UNSUPPORTED, "bruteforce: n_features must be <= 1024");
-  if (n_points >= (1LL << 32) - 1) return set_last_error(FPP_ERR_UNSUPPORTED, "bruteforce: too many points");
-  if (n_queries == 0) return clear_last_error();
-  cudaStream_t s = (cudaStream_t)stream;
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+__global__ void __launch_bounds__(kBfThreads) k_bf_rescore(const float* __restrict__ X, int d, const float* __restrict__ Q,
+                                                           const unsigned long long* __restrict__ list,
+                                                           const int* __restrict__ count, const float* __restrict__ thr,
+                                                           int cap, int k, int q_base, unsigned* __restrict__ fail,
+                                                           int32_t* __restrict__ out, double* __restrict__ out_val) {
+  __shared__ double qs[256];
+  __shared__ unsigned long long key[kRescoreMax];
+  __shared__ uint32_t id[kRescoreMax];
+  __shared__ unsigned reach;
+  const int q = blockIdx.x, tid = threadIdx.x;
+  const int c = count[q];
+  if (c < k || c > cap) {
+    if (tid == 0) fail[1 + atomicAdd(fail, 1u)] = (unsigned)(q_base + q);
+    return;
+  }
+  if (tid < d) qs[tid] = (double)Q[(size_t)q * d + tid];  // d <= 256
+  if (tid == 0) reach = 0;
+  __syncthreads();
+  const unsigned long long kt = dkey((double)thr[q] + (double)kTruthSlack);
+  unsigned mine = 0;
+  for (int i = tid; i < c; i += kBfThreads) {
+    const uint32_t p = ~(uint32_t)list[(size_t)q * cap + i];
+    const float* x = X + (size_t)p * d;
+    double s = 0.0;
+    if ((d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+      for (int j = 0; j < d; j += 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(x + j));
+        s = fma(qs[j], (double)v.x, s);
+        s = fma(qs[j + 1], (double)v.y, s);
+        s = fma(qs[j + 2], (double)v.z, s);
+        s = fma(qs[j + 3], (double)v.w, s);
+      }
+    } else {
+      for (int j = 0; j < d; ++j) s = fma(qs[j], (double)__ldg(x + j), s);
+    }
+    key[i] = dkey(s);
+    id[i] = p;
+    mine += key[i] >= kt;
+  }
+  atomicAdd(&reach, mine);
+  __syncthreads();
+  if (reach < (unsigned)k) {
+    if (tid == 0) fail[1 + atomicAdd(fail, 1u)] = (unsigned)(q_base + q);
+    return;
+  }
+  for (int i = tid; i < c; i += kBfThreads) {
+    const unsigned long long ki = key[i];
+    if (ki < kt) continue;  // k others are at least kt
+    int rank = 0;
+    for (int j = 0; j < c && rank < k; ++j) rank += before(key[j], id[j], ki, id[i]);
+    if (rank < k) {
+      out[(size_t)q * k + rank] = (int32_t)id[i];
+      if (out_val) {
+        const unsigned long long u = (ki & 0x8000000000000000ull) ? (ki ^ 0x8000000000000000ull) : ~ki;
+        out_val[(size_t)q * k + rank] = __longlong_as_double((long long)u);
+      }
+    }
+  }
+}
+
+__global__ void k_bf_rows32(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
+                            const unsigned* __restrict__ idx, int w, int scatter) {
+  const size_t r = blockIdx.x, t = idx[blockIdx.x];
+  const uint32_t* src = in + (scatter ? r : t) * (size_t)w;
+  uint32_t* dst = out + (scatter ? t : r) * (size_t)w;
+  for (int j = threadIdx.x; j < w; j += blockDim.x) dst[j] = src[j];
+}
+
+// The FP64 scores of every point (k_bf_partial, k_bf_merge); returns after the
+// results are written.
+cudaError_t topk_direct(const float* d_X, long long n_points, int n_features, const float* d_Q, int n_queries, int k,
+                        int32_t* d_out, double* d_out_val, int nsm, cudaStream_t s) {
   const int qblocks = (n_queries + kQB - 1) / kQB;
   // slices: enough blocks to fill the GPU, each at least a few thousand points
   long long slices = std::max(1LL, std::min<long long>((long long)nsm * 4 / qblocks + 1, n_points / 4096 + 1));
@@ -210,7 +274,7 @@ extern "C" int fpp_bruteforce_topk_f64(const float* d_X, long long n_points, int
   if (e == cudaSuccess) e = fpp::dev_malloc(&pid, sizeof(uint32_t) * np);
   if (e != cudaSuccess) {
     cudaFree(pkey);
-    return set_last_error(FPP_ERR_OUT_OF_MEMORY, "bruteforce: cannot allocate the partial lists");
+    return e;
   }
   BfArgs a;
   a.X = d_X;
@@ -233,6 +297,92 @@ extern "C" int fpp_bruteforce_topk_f64(const float* d_X, long long n_points, int
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   cudaFree(pkey);
   cudaFree(pid);
+  return e;
+}
+
+// Through candidates (fpp_bf_scan.h): BF16 scores with a bound of their error
+// pick, for each query, the rows that can be in its top k, and only those get
+// FP64 scores.  The ids and scores are those of topk_direct; queries that
+// cannot be settled this way (equal scores by the thousand, zero or non-finite
+// data) go through it.  1M x 200, 500 queries, k = 20: 60 ms
+// direct, 2.3 ms this way (0.7 ms of kernels; the rest is the one allocation).
+cudaError_t topk_candidates(TruthScan& ts, const float* d_X, long long n, int d, const float* d_Q, int nq, int k,
+                            int32_t* d_out, double* d_out_val, int nsm, cudaStream_t s) {
+  unsigned* fail = nullptr;
+  float* fq = nullptr;
+  int32_t* fo = nullptr;
+  double* fv = nullptr;
+  unsigned st = 0, nf = 0;
+  cudaError_t e = dev_malloc(&fail, sizeof(unsigned) * ((size_t)nq + 1));
+  if (e == cudaSuccess) e = cudaMemsetAsync(fail, 0, sizeof(unsigned), s);
+  if (e == cudaSuccess) e = ts.prepare(d_X, n, d, s);
+  for (int q0 = 0; q0 < nq && e == cudaSuccess; q0 += ts.step) {
+    const int m = std::min(ts.step, nq - q0);
+    const float* Q = d_Q + (size_t)q0 * d;
+    if ((e = ts.scan(n, d, Q, m, nsm, s)) != cudaSuccess) break;
+    k_bf_rescore<<<m, kBfThreads, 0, s>>>(d_X, d, Q, ts.list(), ts.count(), ts.thr(), ts.cap, k, q0, fail,
+                                          d_out + (size_t)q0 * k, d_out_val ? d_out_val + (size_t)q0 * k : nullptr);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&st, ts.status(), sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&nf, fail, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+  const cudaError_t e2 = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = e2;
+  if (e == cudaSuccess && st) {
+    e = topk_direct(d_X, n, d, d_Q, nq, k, d_out, d_out_val, nsm, s);
+  } else if (e == cudaSuccess && nf) {
+    if ((e = dev_malloc(&fq, sizeof(float) * (size_t)nf * d)) == cudaSuccess &&
+        (e = dev_malloc(&fo, sizeof(int32_t) * (size_t)nf * k)) == cudaSuccess &&
+        (e = dev_malloc(&fv, sizeof(double) * (size_t)nf * k)) == cudaSuccess) {
+      k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(d_Q), reinterpret_cast<uint32_t*>(fq), fail + 1,
+                                     d, 0);
+      e = topk_direct(d_X, n, d, fq, (int)nf, k, fo, fv, nsm, s);
+      k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(fo), reinterpret_cast<uint32_t*>(d_out),
+                                     fail + 1, k, 1);
+      if (d_out_val)
+        k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(fv), reinterpret_cast<uint32_t*>(d_out_val),
+                                       fail + 1, 2 * k, 1);
+      const cudaError_t e3 = cudaStreamSynchronize(s);
+      if (e == cudaSuccess) e = e3;
+    }
+  }
+  cudaFree(fail);
+  cudaFree(fq);
+  cudaFree(fo);
+  cudaFree(fv);
+  return e;
+}
+
+}  // namespace
+}  // namespace fpp
+
+extern "C" int fpp_bruteforce_topk_f64(const float* d_X, long long n_points, int n_features, const float* d_Q,
+                                       int n_queries, int k, int32_t* d_out, double* d_out_val, void* stream) {
+  using namespace fpp;
+  if (!d_X || !d_Q || !d_out || n_points < 1 || n_features < 1 || n_queries < 0)
+    return set_last_error(FPP_ERR_INVALID_ARGUMENT, "bruteforce: NULL buffer or bad sizes");
+  if (k < 1 || k > kBfMaxK || k > n_points)
+    return set_last_error(FPP_ERR_INVALID_ARGUMENT, "bruteforce: need 1 <= k <= min(256, n_points)");
+  if (n_features > 1024) return set_last_error(FPP_ERR_UNSUPPORTED, "bruteforce: n_features must be <= 1024");
+  if (n_points >= (1LL << 32) - 1) return set_last_error(FPP_ERR_UNSUPPORTED, "bruteforce: too many points");
+  if (n_queries == 0) return clear_last_error();
+  cudaStream_t s = (cudaStream_t)stream;
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // one allocation for the scan; where it does not fit, or the data are too
+  // few to sample (or d > 256), every point gets its FP64 score
+  TruthScan ts;
+  cudaError_t e;
+  if (ts.plan(n_points, n_features, n_queries, k) && dev_malloc(&ts.slab, ts.bytes) == cudaSuccess) {
+    e = topk_candidates(ts, d_X, n_points, n_features, d_Q, n_queries, k, d_out, d_out_val, nsm, s);
+    cudaFree(ts.slab);
+  } else {
+    cudaGetLastError();
+    e = topk_direct(d_X, n_points, n_features, d_Q, n_queries, k, d_out, d_out_val, nsm, s);
+  }
+  if (e == cudaErrorMemoryAllocation)
+    return set_last_error(FPP_ERR_OUT_OF_MEMORY, "bruteforce: cannot allocate the partial lists");
   if (e != cudaSuccess) return set_last_error(FPP_ERR_CUDA, std::string("bruteforce: ") + cudaGetErrorString(e));
   return clear_last_error();
 }

@@ -174,38 +174,12 @@ fail:
 void BatchWorkspace::release() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (graph) cudaGraphDestroy(graph);
-  cudaFree(bitset);
-  cudaFree(uniq);
-  cudaFree(score);
-  cudaFree(gdump);
-  cudaFree(gheap_v);
-  cudaFree(gheap_i);
-  cudaFree(counters);
-  cudaFreeHost(h_counters);
+  cudaFree(slab);
+  cudaFree(bslab);
   for (auto& ev : tev)
     if (ev) cudaEventDestroy(ev);
   for (auto& ev : cev)
     if (ev) cudaEventDestroy(ev);
-  cudaFree(okey);
-  cudaFree(ohist);
-  cudaFree(order);
-  cudaFree(glv);
-  cudaFree(glb);
-  cudaFree(gprobe);
-  cudaFree(gpo);
-  cudaFree(gpe);
-  cudaFree(ggv);
-  cudaFree(ggc);
-  cudaFree(grhv);
-  cudaFree(grhi);
-  cudaFree(ext_lv);
-  cudaFree(ext_lb);
-  cudaFree(hheap_v);
-  cudaFree(hheap_i);
-  cudaFree(pc_g);
-  cudaFree(pc_o);
-  cudaFree(pc_pe);
-  cudaFree(pc_n);
   *this = BatchWorkspace();
 }
 
@@ -305,36 +279,43 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   const int groups = grid * (kBThreads / (F < 32 ? 1 : F / 32));
   const long long list_cap = big ? (long long)L * mmax : 0;
   const long long probe_cap = big ? rq.qprobes_max : 0;
-  // (re)allocate per-block scratch when the shape grows
+  const long long heap_cap = split ? (long long)nsm * 64 * std::max(mmax, 1) : 0;  // pair heaps of the hash kernel
+  // (re)allocate per-block scratch when the shape grows, in one piece
   if (!bw.bitset || bw.grid < grid || bw.nwords != nwords || bw.cap < cap || bw.fht < F || bw.mmax < mmax ||
-      bw.list_cap < list_cap || bw.probe_cap < probe_cap) {
+      bw.list_cap < list_cap || bw.probe_cap < probe_cap || bw.hheap_cap < heap_cap) {
     bw.release();
-    if ((e = fpp::dev_malloc(&bw.bitset, sizeof(uint32_t) * (size_t)grid * nwords)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = cudaMemsetAsync(bw.bitset, 0, sizeof(uint32_t) * (size_t)grid * nwords, s)) != cudaSuccess)
-      return fail(e, "memset");
-    if ((e = fpp::dev_malloc(&bw.uniq, sizeof(uint32_t) * (size_t)grid * cap)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.score, sizeof(uint32_t) * (size_t)grid * cap)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.gdump, sizeof(float) * (size_t)groups * F)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.gheap_v, sizeof(float) * (size_t)groups * std::max(mmax, 1))) != cudaSuccess)
-      return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.gheap_i, sizeof(int) * (size_t)groups * std::max(mmax, 1))) != cudaSuccess)
-      return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.counters, sizeof(BatchCounters))) != cudaSuccess) return fail(e, "alloc");
-    if ((e = cudaMallocHost(&bw.h_counters, sizeof(BatchCounters))) != cudaSuccess) return fail(e, "alloc");
+    Slab slab;
+    slab.reserve(&bw.bitset, (size_t)grid * nwords);
+    slab.reserve(&bw.uniq, (size_t)grid * cap);
+    slab.reserve(&bw.score, (size_t)grid * cap);
+    slab.reserve(&bw.gdump, (size_t)groups * F);
+    slab.reserve(&bw.gheap_v, (size_t)groups * std::max(mmax, 1));
+    slab.reserve(&bw.gheap_i, (size_t)groups * std::max(mmax, 1));
+    slab.reserve(&bw.counters, 1);
+    if (heap_cap) {
+      slab.reserve(&bw.hheap_v, heap_cap);
+      slab.reserve(&bw.hheap_i, heap_cap);
+    }
     if (big) {
       const size_t gl = (size_t)grid * list_cap, gp = (size_t)grid * probe_cap;
       const size_t gg = (size_t)groups * 2 * (kBigM1 + 1), gr = (size_t)groups * kBigM1;
-      if ((e = fpp::dev_malloc(&bw.glv, sizeof(float) * gl)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.glb, sizeof(uint32_t) * gl)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.gprobe, sizeof(uint32_t) * gp)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.gpo, sizeof(uint32_t) * gp)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.gpe, sizeof(uint32_t) * gp)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.ggv, sizeof(float) * gg)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.ggc, sizeof(int) * gg)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.grhv, sizeof(float) * gr)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.grhi, sizeof(int) * gr)) != cudaSuccess)
-        return fail(e, "alloc");
+      slab.reserve(&bw.glv, gl);
+      slab.reserve(&bw.glb, gl);
+      slab.reserve(&bw.gprobe, gp);
+      slab.reserve(&bw.gpo, gp);
+      slab.reserve(&bw.gpe, gp);
+      slab.reserve(&bw.ggv, gg);
+      slab.reserve(&bw.ggc, gg);
+      slab.reserve(&bw.grhv, gr);
+      slab.reserve(&bw.grhi, gr);
     }
+    if ((e = slab.alloc(&bw.slab)) != cudaSuccess) {
+      bw = BatchWorkspace();
+      return fail(e, "alloc");
+    }
+    if ((e = cudaMemsetAsync(bw.bitset, 0, sizeof(uint32_t) * (size_t)grid * nwords, s)) != cudaSuccess)
+      return fail(e, "memset");
+    bw.hheap_cap = heap_cap;
     bw.list_cap = list_cap;
     bw.probe_cap = probe_cap;
     bw.grid = grid;
@@ -345,33 +326,33 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   }
   grid = std::min(grid, bw.grid);
   const long long ext_stride = (long long)L * std::max(mmax, 1);
+  // per-batch buffers: lists of the hash, processing order, probe cuts
+  const bool pcut = split && !big;
+  const long long ext_need = split ? (long long)rq.nq * ext_stride : 0;
+  const long long pc_need = pcut ? (long long)rq.nq * rq.qprobes_max : 0;
+  if (!bw.bslab || bw.batch_cap < rq.nq || bw.ext_cap < ext_need || bw.pc_cap < pc_need) {
+    cudaFree(bw.bslab);
+    bw.batch_cap = bw.ext_cap = bw.pc_cap = 0;
+    Slab slab;
+    slab.reserve(&bw.okey, (size_t)rq.nq);
+    slab.reserve(&bw.order, (size_t)rq.nq);
+    slab.reserve(&bw.ohist, (size_t)kOrderMaxBins);
+    slab.reserve(&bw.ext_lv, (size_t)ext_need);
+    slab.reserve(&bw.ext_lb, (size_t)ext_need);
+    slab.reserve(&bw.pc_g, (size_t)pc_need);
+    slab.reserve(&bw.pc_o, (size_t)pc_need);
+    slab.reserve(&bw.pc_pe, (size_t)pc_need);
+    slab.reserve(&bw.pc_n, (size_t)rq.nq);
+    if ((e = slab.alloc(&bw.bslab)) != cudaSuccess) return fail(e, "alloc");
+    if ((e = cudaMemsetAsync(bw.ohist, 0, sizeof(uint32_t) * kOrderMaxBins, s)) != cudaSuccess)
+      return fail(e, "memset");
+    bw.batch_cap = rq.nq;
+    bw.ext_cap = ext_need;
+    bw.pc_cap = pc_need;
+  }
   const bool vhash = split && rq.tc_hash && F == 256 && di.tflips && L <= 128 && 2 * rq.qprobes_max <= L;
   if (split) {
     const long long max_groups = (long long)nsm * 64;
-    if (!bw.ext_lv || bw.ext_cap < (long long)rq.nq * ext_stride) {
-      cudaFree(bw.ext_lv);
-      cudaFree(bw.ext_lb);
-      bw.ext_lv = nullptr;
-      bw.ext_lb = nullptr;
-      bw.ext_cap = 0;
-      const size_t ne = (size_t)rq.nq * ext_stride;
-      if ((e = fpp::dev_malloc(&bw.ext_lv, sizeof(float) * ne)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.ext_lb, sizeof(uint32_t) * ne)) != cudaSuccess)
-        return fail(e, "alloc");
-      bw.ext_cap = (long long)ne;
-    }
-    if (!bw.hheap_v || bw.hheap_cap < max_groups * std::max(mmax, 1)) {
-      cudaFree(bw.hheap_v);
-      cudaFree(bw.hheap_i);
-      bw.hheap_v = nullptr;
-      bw.hheap_i = nullptr;
-      bw.hheap_cap = 0;
-      const size_t nh = (size_t)max_groups * std::max(mmax, 1);
-      if ((e = fpp::dev_malloc(&bw.hheap_v, sizeof(float) * nh)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.hheap_i, sizeof(int) * nh)) != cudaSuccess)
-        return fail(e, "alloc");
-      bw.hheap_cap = (long long)nh;
-    }
     if (rq.stage_timing) {
       for (auto& ev : bw.tev)
         if (!ev && (e = cudaEventCreate(&ev)) != cudaSuccess) return fail(e, "event create");
@@ -442,19 +423,6 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   while ((1 << log2D) < D) ++log2D;
   const void* okern = order_key_kernel(F);
   const bool reorder = rq.reorder && okern && rq.nq >= 2 * grid && 2 * D <= kOrderMaxBins;
-  if (reorder && bw.order_cap < rq.nq) {
-    cudaFree(bw.okey);
-    cudaFree(bw.ohist);
-    cudaFree(bw.order);
-    bw.okey = bw.ohist = bw.order = nullptr;
-    bw.order_cap = 0;
-    if ((e = fpp::dev_malloc(&bw.okey, sizeof(uint32_t) * (size_t)rq.nq)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.order, sizeof(uint32_t) * (size_t)rq.nq)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = fpp::dev_malloc(&bw.ohist, sizeof(uint32_t) * kOrderMaxBins)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = cudaMemsetAsync(bw.ohist, 0, sizeof(uint32_t) * kOrderMaxBins, s)) != cudaSuccess)
-      return fail(e, "memset");
-    bw.order_cap = rq.nq;
-  }
   if (reorder && split) {
     k_order_key_ext<<<(rq.nq + 255) / 256, 256, 0, s>>>(bw.ext_lb, rq.nq, ext_stride, 2 * D, bw.okey, bw.ohist);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "order key launch");
@@ -473,25 +441,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "order scatter launch");
   }
   // split hash, small lists: the probe cut of every query in its own kernel
-  const bool pcut = split && !big;
   if (pcut) {
-    const long long npc = (long long)rq.nq * rq.qprobes_max;
-    if (!bw.pc_g || bw.pc_cap < npc || bw.pc_ncap < rq.nq) {
-      cudaFree(bw.pc_g);
-      cudaFree(bw.pc_o);
-      cudaFree(bw.pc_pe);
-      cudaFree(bw.pc_n);
-      bw.pc_g = bw.pc_o = bw.pc_pe = nullptr;
-      bw.pc_n = nullptr;
-      bw.pc_cap = bw.pc_ncap = 0;
-      if ((e = fpp::dev_malloc(&bw.pc_g, sizeof(uint32_t) * (size_t)npc)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.pc_o, sizeof(uint32_t) * (size_t)npc)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.pc_pe, sizeof(uint32_t) * (size_t)npc)) != cudaSuccess ||
-          (e = fpp::dev_malloc(&bw.pc_n, sizeof(int) * (size_t)rq.nq)) != cudaSuccess)
-        return fail(e, "alloc");
-      bw.pc_cap = npc;
-      bw.pc_ncap = rq.nq;
-    }
     ProbeCutArgs pa;
     pa.ext_lv = bw.ext_lv;
     pa.ext_lb = bw.ext_lb;
@@ -678,13 +628,13 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     if (rq.out_host && (e = cudaMemcpyAsync(rq.out_host, rq.out, sizeof(int32_t) * (size_t)rq.nq * rq.out_stride,
                                             cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return fail(e, "result copy");
-    if ((e = cudaMemcpyAsync(bw.h_counters, bw.counters, sizeof(BatchCounters), cudaMemcpyDeviceToHost, s)) !=
-        cudaSuccess)
+    BatchCounters hc;
+    if ((e = cudaMemcpyAsync(&hc, bw.counters, sizeof(hc), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return fail(e, "status");
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(e, "batch kernel");
-    res.overflow = (bw.h_counters->status & 1u) != 0;
-    res.bad_params = (bw.h_counters->status & 2u) != 0;
-    if (totals) res.totals = bw.h_counters->totals;
+    res.overflow = (hc.status & 1u) != 0;
+    res.bad_params = (hc.status & 2u) != 0;
+    if (totals) res.totals = hc.totals;
   }
   return kOk;
 }

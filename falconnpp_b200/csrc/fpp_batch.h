@@ -96,6 +96,8 @@ struct BatchKey {
 
 // Per-block scratch of the batched kernel (kept between calls) and the cached graph.
 struct BatchWorkspace {
+  unsigned char* slab = nullptr;   // the per-block scratch and the counters
+  unsigned char* bslab = nullptr;  // the per-batch buffers (order, ext_, pc_)
   uint32_t* bitset = nullptr;
   long long nwords = 0;
   uint32_t* uniq = nullptr;
@@ -108,12 +110,10 @@ struct BatchWorkspace {
   int fht = 0;
   int grid = 0;
   BatchCounters* counters = nullptr;
-  BatchCounters* h_counters = nullptr;  // pinned copy
   // query order: key per query, histogram of the keys, the permutation
   uint32_t* okey = nullptr;
   uint32_t* ohist = nullptr;
   uint32_t* order = nullptr;
-  long long order_cap = 0;
   // big-list form scratch (see BatchArgs)
   float* glv = nullptr;
   uint32_t* glb = nullptr;
@@ -129,7 +129,7 @@ struct BatchWorkspace {
   // split hash: per-query lists and the hash kernel's pair-heap scratch
   float* ext_lv = nullptr;
   uint32_t* ext_lb = nullptr;
-  long long ext_cap = 0;
+  long long batch_cap = 0, ext_cap = 0, pc_cap = 0;  // queries, list and probe entries that bslab holds
   float* hheap_v = nullptr;
   int* hheap_i = nullptr;
   long long hheap_cap = 0;
@@ -138,7 +138,6 @@ struct BatchWorkspace {
   uint32_t* pc_o = nullptr;
   uint32_t* pc_pe = nullptr;
   int* pc_n = nullptr;
-  long long pc_cap = 0, pc_ncap = 0;
   cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};  // stage timing: start, fused start, end, hash end
   cudaEvent_t cev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // chunked query copy: chunks, start
   cudaGraphExec_t graph_exec = nullptr;

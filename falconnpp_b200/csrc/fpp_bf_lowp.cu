@@ -1530,6 +1530,7 @@ bool TruthScan::plan(long long n, int d, int nq, int k) {
   o_list = take((size_t)step * cap * 8);
   o_count = take((size_t)step * 4);
   o_words = take(16);
+  o_fail = take(((size_t)nq + 1) * 4);
   bytes = o;
   return true;
 }

@@ -26,12 +26,14 @@ struct TruthScan {
   unsigned long long* list() const { return reinterpret_cast<unsigned long long*>(slab + o_list); }
   int* count() const { return reinterpret_cast<int*>(slab + o_count); }
   float* thr() const { return reinterpret_cast<float*>(slab + o_thr); }
+  unsigned* fail() const { return reinterpret_cast<unsigned*>(slab + o_fail); }  // room for a count and nq indexes
   unsigned* status() const { return reinterpret_cast<unsigned*>(slab + o_words) + 1; }  // bit 0: a CTA gave up
 
  private:
   int xstride = 0, j = 0, ldo = 0;
   long long sample_tiles = 0;
-  size_t o_rows = 0, o_err = 0, o_qrows = 0, o_qnorm = 0, o_tmax = 0, o_thr = 0, o_list = 0, o_count = 0, o_words = 0;
+  size_t o_rows = 0, o_err = 0, o_qrows = 0, o_qnorm = 0, o_tmax = 0, o_thr = 0, o_list = 0, o_count = 0, o_words = 0,
+         o_fail = 0;
 };
 
 }  // namespace fpp

@@ -308,13 +308,12 @@ cudaError_t topk_direct(const float* d_X, long long n_points, int n_features, co
 // direct, 2.3 ms this way (0.7 ms of kernels; the rest is the one allocation).
 cudaError_t topk_candidates(TruthScan& ts, const float* d_X, long long n, int d, const float* d_Q, int nq, int k,
                             int32_t* d_out, double* d_out_val, int nsm, cudaStream_t s) {
-  unsigned* fail = nullptr;
+  unsigned* fail = ts.fail();
   float* fq = nullptr;
   int32_t* fo = nullptr;
   double* fv = nullptr;
   unsigned st = 0, nf = 0;
-  cudaError_t e = dev_malloc(&fail, sizeof(unsigned) * ((size_t)nq + 1));
-  if (e == cudaSuccess) e = cudaMemsetAsync(fail, 0, sizeof(unsigned), s);
+  cudaError_t e = cudaMemsetAsync(fail, 0, sizeof(unsigned), s);
   if (e == cudaSuccess) e = ts.prepare(d_X, n, d, s);
   for (int q0 = 0; q0 < nq && e == cudaSuccess; q0 += ts.step) {
     const int m = std::min(ts.step, nq - q0);
@@ -346,7 +345,6 @@ cudaError_t topk_candidates(TruthScan& ts, const float* d_X, long long n, int d,
       if (e == cudaSuccess) e = e3;
     }
   }
-  cudaFree(fail);
   cudaFree(fq);
   cudaFree(fo);
   cudaFree(fv);

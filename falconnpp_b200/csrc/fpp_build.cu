@@ -8,12 +8,13 @@
 //      (sign flip + shuffle FWHT), picks the top-iProbes cross-polytope codes
 //      per layer and combines the two layers (FalconnPP.cpp:75-201).  Each
 //      (table, point) emits iProbes (bucket, score, id) entries;
-//   3. a stable LSD radix sort of the entries by (global bucket, score desc)
-//      replaces the per-bucket max-heaps: entries arrive in ascending id
-//      order, so equal scores stay in ascending id order;
-//   4. per-bucket limits iLimit = ceil(alpha * B / iProbes) (FP32), raised to
-//      min(bucket_minSize, B) (FalconnPP.cpp:233-242), give CSR offsets; the
-//      first iLimit ids of every bucket are compacted into the 1D table;
+//   3. per-bucket limits iLimit = ceil(alpha * B / iProbes) (FP32), raised to
+//      min(bucket_minSize, B) (FalconnPP.cpp:233-242), give CSR offsets, and
+//      the bucket sizes the places of a chunk's entries, bucket by bucket;
+//   4. every entry goes to its bucket's place, then each bucket is sorted by
+//      (score desc, id asc) on its own (a warp for up to 32 entries, a block's
+//      shared memory above), replacing the per-bucket max-heaps; its first
+//      iLimit ids are the 1D table's;
 //   5. where equal scores make the reference's heap order differ from
 //      (score desc, id asc) — ties at the iLimit cut, and (by default) ties
 //      inside the kept prefix — k_repair replays the reference's max-heap on
@@ -172,22 +173,37 @@ __global__ void __launch_bounds__(256) k_center_rows(const float* __restrict__ X
   if (i8 && lane == 0) atomicMax(reinterpret_cast<unsigned*>(norm_max), __float_as_uint(nmax));  // >= 0: bits order
 }
 
-static bool alloc_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
-  if (P.n_features > 512) return false;
-  const size_t bytes = (size_t)P.n_points * i8_row_bytes(P.n_features);
-  if (dev_malloc(&di.i8_norm_max, sizeof(float)) == cudaSuccess && dev_malloc(&di.Xi8, bytes) == cudaSuccess &&
-      cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s) == cudaSuccess)
-    return true;
-  cudaGetLastError();  // the FP32 form works without the copy
-  cudaFree(di.Xi8);
-  cudaFree(di.i8_norm_max);
-  di.Xi8 = nullptr;
-  di.i8_norm_max = nullptr;
-  return false;
+cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
+  const size_t n = (size_t)P.n_points, d = (size_t)P.n_features;
+  const size_t words = (size_t)2 * P.n_tables * 3 * (P.fhtDim < 32 ? 1 : P.fhtDim / 32);
+  const size_t nb = (size_t)P.n_tables * 4 * P.n_proj * P.n_proj;
+  di.ld = (P.n_features + 3) & ~3;
+  cudaError_t e = cudaSuccess;
+  for (bool i8 = d <= 512;; i8 = false) {
+    Slab slab;
+    slab.reserve(&di.Xc, n * di.ld);
+    slab.reserve(&di.center, d);
+    slab.reserve(&di.flips, words);
+    if (P.fhtDim == 256) slab.reserve(&di.tflips, words);
+    slab.reserve(&di.bucket_off, nb + 1);
+    di.Xi8 = nullptr;
+    di.i8_norm_max = nullptr;
+    if (i8) {
+      slab.reserve(&di.Xi8, n * i8_row_bytes(P.n_features));
+      slab.reserve(&di.i8_norm_max, 1);
+    }
+    e = slab.alloc(&di.slab);
+    if (e == cudaSuccess || !i8) break;
+    cudaGetLastError();
+    size_t have = 0, all = 0;
+    if (cudaMemGetInfo(&have, &all) != cudaSuccess || have >= slab.bytes()) break;  // not for want of room
+  }
+  return e;
 }
 
 void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
-  if (!alloc_screen_rows(P, di, s)) return;
+  if (!di.Xi8) return;
+  cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s);
   k_center_rows<false><<<1184, 256, 0, s>>>(nullptr, P.n_points, P.n_features, di.ld, nullptr, di.Xc, di.Xi8,
                                             i8_row_bytes(P.n_features), di.i8_norm_max, nullptr);
 }
@@ -200,94 +216,186 @@ struct HashArgs {
   int L, l0, l1;
   int D, log2D, P;
   uint32_t NB;
-  uint64_t* keys;
-  uint32_t* vals;
-  uint32_t* counts;  // [L * NB]
+  uint64_t* keys;    // (bucket of the chunk << 32) | ~ord(score)
+  uint32_t* ranks;   // place among the bucket's entries, in order of arrival
+  uint32_t* counts;  // [chunk tables * NB]
   int32_t* dump_codes;
   float* dump_scores;
 };
 
-template <int FHT>
+template <int FHT, int KEEP>
 struct HashSmem {
   static constexpr int G = Geo<FHT>::G;
   static constexpr int GROUPS = 128 / G;
-  // per group: dump of one rotated vector, two top lists, one heap
-  static constexpr size_t per_group = FHT * 4 + 2 * (kMaxIProbes + 1) * 8 + kMaxIProbes * 8;
-  static constexpr size_t bytes = GROUPS * per_group;
+  // per group: the point and a rotated vector, two top lists, one heap (the
+  // lists with an entry more than is kept)
+  static constexpr int kCap = KEEP ? KEEP : kMaxIProbes;
+  static constexpr size_t kVec = FHT < 32 ? FHT : LaneVector<FHT>::kFloats;
+  static constexpr size_t kLists = 2 * (kCap + 1) * 8 + kCap * 8;
+  static constexpr size_t bytes = GROUPS * (2 * kVec * 4 + kLists);
 };
 
-// Block = 128 threads; a group of G lanes per point; grid-stride over points.
-template <int FHT>
-__global__ void __launch_bounds__(128, 4) k_build_hash(HashArgs a) {
+// Block = 128 threads; a group of FHT / 32 lanes per point; grid-stride over
+// points.  KEEP: iProbes where it is 1..3 and the vector has 32 or more points
+// (the key selection and the pairs in registers), 0 for the general form.
+// Bound by issue slots (1,580 instructions per four points and layer, 65 % of
+// the slots) beside 290 shuffles (one a clock per SM).  1M x 200, 100 tables,
+// iProbes 3: 103 ms; 228 ms with the sorted insertion, a pair heap in lane 0
+// and the rounds and layers unrolled (the code then missed the instruction
+// caches, a third of the stalls).  64 elements per lane: 105 ms; signs as
+// float pairs multiplied in, from memory: 119 ms.
+template <int FHT, int KEEP>
+__global__ void __launch_bounds__(128, KEEP == 3 ? 5 : 4) k_build_hash(HashArgs a) {
   constexpr int E = Geo<FHT>::E;
-  constexpr int G = Geo<FHT>::G;
   constexpr int WORDS = Geo<FHT>::WORDS;
-  constexpr int GROUPS = HashSmem<FHT>::GROUPS;
+  using SM = HashSmem<FHT, KEEP>;
+  constexpr int G = SM::G;
+  constexpr int GROUPS = SM::GROUPS;
+  constexpr int CAP = SM::kCap;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);
   const int grp = threadIdx.x / G;
   const unsigned gmask = (G == 32) ? kFullMask : (((1u << G) - 1u) << (lane & ~(G - 1)));
-  unsigned char* gs = smem_raw + grp * HashSmem<FHT>::per_group;
-  float* ydump = reinterpret_cast<float*>(gs);
-  float* lv1 = reinterpret_cast<float*>(gs + FHT * 4);
-  int* lc1 = reinterpret_cast<int*>(lv1 + (kMaxIProbes + 1));
-  float* lv2 = reinterpret_cast<float*>(lc1 + (kMaxIProbes + 1));
-  int* lc2 = reinterpret_cast<int*>(lv2 + (kMaxIProbes + 1));
-  float* hv = reinterpret_cast<float*>(lc2 + (kMaxIProbes + 1));
-  int* hi = reinterpret_cast<int*>(hv + kMaxIProbes);
+  float* yv = reinterpret_cast<float*>(smem_raw) + grp * SM::kVec;  // 16-byte aligned
+  float* xs = reinterpret_cast<float*>(smem_raw) + (GROUPS + grp) * SM::kVec;
+  unsigned char* gs = smem_raw + 2 * GROUPS * SM::kVec * 4 + grp * SM::kLists;
+  float* lv1 = reinterpret_cast<float*>(gs);
+  int* lc1 = reinterpret_cast<int*>(lv1 + (CAP + 1));
+  float* lv2 = reinterpret_cast<float*>(lc1 + (CAP + 1));
+  int* lc2 = reinterpret_cast<int*>(lv2 + (CAP + 1));
+  float* hv = reinterpret_cast<float*>(lc2 + (CAP + 1));
+  int* hi = reinterpret_cast<int*>(hv + CAP);
 
-  const int P = a.P;
+  const int P = KEEP ? KEEP : a.P;
   const int cnt = min(P + 1, a.D);
+  const int twoD = 2 * a.D;
   const long long groups_total = (long long)gridDim.x * GROUPS;
   const long long n_iter = (a.n + groups_total - 1) / groups_total;
   for (long long it = 0; it < n_iter; ++it) {
     const long long pt_ll = it * groups_total + (long long)blockIdx.x * GROUPS + grp;
     const bool active = pt_ll < a.n;  // inactive groups still join every shuffle
     const int pt = active ? (int)pt_ll : 0;
-    float xr[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int idx = gl * E + e;
-      xr[e] = (active && idx < a.d) ? __ldg(a.Xc + (size_t)pt * a.ld + idx) : 0.0f;
+    // the point in shared memory (in registers it would cost a fifth of the warps)
+    __syncwarp();
+    for (int i = gl; i < FHT; i += G) {
+      const float x = active && i < a.d ? __ldg(a.Xc + (size_t)pt * a.ld + i) : 0.0f;
+      if constexpr (FHT < 32)
+        xs[i] = x;
+      else
+        LaneVector<FHT>::at(xs, i) = x;
     }
+    __syncwarp();
     for (int l = a.l0; l < a.l1; ++l) {
 #pragma unroll 1
       for (int layer = 0; layer < 2; ++layer) {
-        float y[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) y[e] = xr[e];
-        hd3_rotate<FHT>(y, a.flips + ((size_t)(layer * a.L + l) * 3) * WORDS, gl);
         float* lv = layer == 0 ? lv1 : lv2;
         int* lc = layer == 0 ? lc1 : lc2;
-        const bool ok = group_top_cp_checked<FHT>(y, gl, a.D, a.log2D, P, cnt, lv, lc);
-        if (!ok) {  // group-uniform: replay the reference's heap scan
+        const uint32_t* flips = a.flips + ((size_t)(layer * a.L + l) * 3) * WORDS;
+        if constexpr (KEEP > 0) {
+          f2 y[E / 2];
+          LaneVector<FHT>::load(xs, y, gl);
+          hd3_rotate_pairs<FHT>(y, flips, gl);
+          if constexpr (KEEP == 1) {
+            // one code per layer: the two-pass strict top-1 gives value and code
+            // at once (6.7 ms against 7.5 ms for keys, 100K x 200, 50 tables)
+            float ye[32];
 #pragma unroll
-          for (int e = 0; e < E; ++e) ydump[gl * E + e] = y[e];
-          __syncwarp(gmask);
-          if (gl == 0) replay_layer_topp(ydump, a.D, a.log2D, P, hv, hi, lv, lc);
-          __syncwarp(gmask);
+            for (int j = 0; j < 16; ++j) {
+              ye[2 * j] = f2_lo(y[j]);
+              ye[2 * j + 1] = f2_hi(y[j]);
+            }
+            const bool ok = group_top1_strict<FHT>(ye, gl, a.D, a.log2D, lv, lc);
+            if (__all_sync(kFullMask, ok)) {
+              __syncwarp();
+              continue;
+            }
+          }
+          constexpr int C = KEEP == 1 ? 2 : 4;
+          uint32_t k[C];
+          auto bits = [&](int e) { return (uint32_t)(y[e / 2] >> (32 * (e & 1))); };
+          const bool fast = __all_sync(kFullMask, group_top_keys<FHT, C>(bits, gl, a.D, cnt, k));
+          LaneVector<FHT>::store(yv, y, gl);
+          __syncwarp();
+          if (fast) {
+            if (gl == 0) {
+#pragma unroll
+              for (int t = 0; t < KEEP; ++t) {
+                const int pos = (int)(k[t] & (FHT - 1));
+                const float x = LaneVector<FHT>::at(yv, pos);
+                lv[t] = cp_value(x);
+                lc[t] = cp_code(x, pos, a.log2D);
+              }
+            }
+          } else if (!group_top_stored<FHT>(yv, gl, a.D, a.log2D, cnt, lv, lc) && gl == 0) {
+            // the reference's scan, FalconnPP.cpp:103-156
+            int n = 0;
+            for (int r = 0; r < a.D; ++r) {
+              const float x = LaneVector<FHT>::at(yv, r);
+              topp_offer<int>(hv, hi, n, P, cp_value(x), cp_code(x, r, a.log2D));
+            }
+            for (int j = P - 1; j >= 0; --j) {
+              lv[j] = hv[0];
+              lc[j] = hi[0];
+              heap_pop<true, int>(hv, hi, n);
+            }
+          }
+          __syncwarp();
+        } else {
+          float y[E];
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            const int i = gl * E + e;
+            y[e] = FHT < 32 ? xs[i] : LaneVector<FHT>::at(xs, i);
+          }
+          hd3_rotate<FHT>(y, flips, gl);
+          const bool ok = group_top_cp_checked<FHT>(y, gl, a.D, a.log2D, P, cnt, lv, lc);
+          if (!ok) {  // group-uniform: replay the reference's heap scan
+#pragma unroll
+            for (int e = 0; e < E; ++e) yv[gl * E + e] = y[e];
+            __syncwarp(gmask);
+            if (gl == 0) replay_layer_topp(yv, a.D, a.log2D, P, hv, hi, lv, lc);
+            __syncwarp(gmask);
+          }
         }
       }
       if (gl == 0 && active) {
-        // two-layer combination, FalconnPP.cpp:162-189 (always replayed: P^2 offers)
-        int hn = 0;
-        const int twoD = 2 * a.D;
-        for (int i = 0; i < P; ++i)
-          for (int j = 0; j < P; ++j)
-            topp_offer<int>(hv, hi, hn, P, __fadd_rn(lv2[j], lv1[i]), lc1[i] * twoD + lc2[j]);
         const size_t ebase = ((size_t)(l - a.l0) * a.n + pt) * P;
         const size_t dbase = ((size_t)l * a.n + pt) * P;
-        for (int j = 0; j < P; ++j) {  // drain order of the min-heap (FalconnPP.cpp:196-201)
-          const float s = hv[0];
-          const int b = hi[0];
-          heap_pop<true, int>(hv, hi, hn);
-          a.keys[ebase + j] = ((uint64_t)((uint32_t)(l - a.l0) * a.NB + (uint32_t)b) << 32) | (uint64_t)(~ord_key(s));
-          a.vals[ebase + j] = (uint32_t)pt;
-          atomicAdd(a.counts + (size_t)l * a.NB + b, 1u);
+        auto put = [&](int j, float s, int b) {  // entry j of the drain order (FalconnPP.cpp:196-201)
+          const uint32_t rel = (uint32_t)(l - a.l0) * a.NB + (uint32_t)b;
+          a.keys[ebase + j] = ((uint64_t)rel << 32) | (uint64_t)(~ord_key(s));
+          a.ranks[ebase + j] = atomicAdd(a.counts + rel, 1u);
           if (a.dump_codes) {
             a.dump_codes[dbase + j] = b;
             a.dump_scores[dbase + j] = s;
+          }
+        };
+        bool done = false;
+        if constexpr (KEEP > 0) {
+          // the lists are strict except where a replay filled them from ties
+          float s[4];
+          int ij[4];
+          bool strict = true;
+#pragma unroll
+          for (int t = 1; t < KEEP; ++t) strict = strict && lv1[t - 1] > lv1[t] && lv2[t - 1] > lv2[t];
+          done = strict && top_pairs(lv1, lv2, KEEP, KEEP, s, ij);
+          if (done) {
+#pragma unroll
+            for (int r = 0; r < KEEP; ++r) put(KEEP - 1 - r, s[r], lc1[ij[r] >> 2] * twoD + lc2[ij[r] & 3]);
+          }
+        }
+        if (!done) {
+          // two-layer combination, FalconnPP.cpp:162-189, replayed: P^2 offers
+          int hn = 0;
+          for (int i = 0; i < P; ++i)
+            for (int j = 0; j < P; ++j)
+              topp_offer<int>(hv, hi, hn, P, __fadd_rn(lv2[j], lv1[i]), lc1[i] * twoD + lc2[j]);
+          for (int j = 0; j < P; ++j) {
+            const float s = hv[0];
+            const int b = hi[0];
+            heap_pop<true, int>(hv, hi, hn);
+            put(j, s, b);
           }
         }
       }
@@ -419,205 +527,492 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(ScanArgs a) {
   }
 }
 
-// ---------------------------------------------------------------- radix sort
-constexpr int kRsThreads = 256;
-constexpr int kRsItems = 16;
-constexpr int kRsTile = kRsThreads * kRsItems;
-
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* __restrict__ keys, long long N, int shift,
-                                                         uint32_t* __restrict__ hist, int ntiles) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  const long long base = (long long)blockIdx.x * kRsTile;
-#pragma unroll 4
-  for (int i = 0; i < kRsItems; ++i) {
-    const long long idx = base + (long long)i * kRsThreads + threadIdx.x;
-    if (idx < N) atomicAdd(&h[(uint32_t)(keys[idx] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
-}
-
-// one block per digit: exclusive scan over the tiles of that digit
-__global__ void __launch_bounds__(1024) k_rs_scan(uint32_t* __restrict__ hist, int ntiles,
-                                                  uint32_t* __restrict__ digit_total) {
-  __shared__ long long tmp[32];
-  uint32_t* h = hist + (size_t)blockIdx.x * ntiles;
-  const int per = (ntiles + 1023) / 1024;
-  const int t0 = threadIdx.x * per;
-  long long s = 0;
-  for (int i = 0; i < per; ++i)
-    if (t0 + i < ntiles) s += h[t0 + i];
-  long long total;
-  long long run = block_exclusive_scan(s, tmp, &total);
-  for (int i = 0; i < per; ++i)
-    if (t0 + i < ntiles) {
-      const uint32_t v = h[t0 + i];
-      h[t0 + i] = (uint32_t)run;
-      run += v;
-    }
-  if (threadIdx.x == 0) digit_total[blockIdx.x] = (uint32_t)total;
-}
-
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t* __restrict__ kin,
-                                                            const uint32_t* __restrict__ vin,
-                                                            uint64_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                            long long N, int shift, const uint32_t* __restrict__ hist,
-                                                            int ntiles, const uint32_t* __restrict__ digit_total) {
-  __shared__ long long tmp[32];
-  __shared__ uint32_t base[256];
-  __shared__ uint32_t wcnt[kRsThreads / 32][257];
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  long long tot;
-  const long long dbase = block_exclusive_scan((long long)digit_total[tid], tmp, &tot);
-  base[tid] = (uint32_t)dbase + hist[(size_t)tid * ntiles + blockIdx.x];
-  for (int w = 0; w < kRsThreads / 32; ++w) wcnt[w][tid] = 0;
-  if (tid == 0)
-    for (int w = 0; w < kRsThreads / 32; ++w) wcnt[w][256] = 0;
-  __syncthreads();
-  const long long tbase = (long long)blockIdx.x * kRsTile;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int it = 0; it < kRsItems; ++it) {
-    const long long idx = tbase + (long long)it * kRsThreads + tid;
-    const bool valid = idx < N;
-    const uint64_t k = valid ? kin[idx] : 0ull;
-    const uint32_t v = valid ? vin[idx] : 0u;
-    const uint32_t dg = valid ? ((uint32_t)(k >> shift) & 255u) : 256u;
-    const unsigned peers = __match_any_sync(kFullMask, dg);
-    const int rank = __popc(peers & lt);
-    if (valid && lane == __ffs(peers) - 1) wcnt[warp][dg] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      uint32_t o = base[dg];
-      for (int w = 0; w < warp; ++w) o += wcnt[w][dg];
-      kout[o + rank] = k;
-      vout[o + rank] = v;
-    }
-    __syncthreads();
-    uint32_t s = 0;
-    for (int w = 0; w < kRsThreads / 32; ++w) {
-      s += wcnt[w][tid];
-      wcnt[w][tid] = 0;
-    }
-    base[tid] += s;
-    __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------- compaction
-struct CompactArgs {
-  const uint64_t* keys;  // sorted
-  const uint32_t* vals;
-  long long N;
-  const uint32_t* counts;  // global [L*NB]
+// ---------------------------------------------------------------- buckets
+// An entry in its bucket's place: (~ord(score) << 32) | id, so ascending order
+// is (score desc, id asc).
+struct BucketArgs {
+  const uint64_t* keys;
+  const uint32_t* ranks;
+  unsigned N;                // entries of the chunk
+  unsigned n;                // points
+  int P;
+  const uint32_t* counts;    // chunk-local
   const uint32_t* segstart;  // chunk-local
-  const uint32_t* off;       // global
-  unsigned long long gbase;  // first global bucket of the chunk
+  const uint32_t* off;       // chunk's slice of the global offsets
+  unsigned nb;               // buckets of the chunk
   float alpha;
-  int P, minSize;
+  int minSize;
   int exact_order;
+  uint64_t* seg;
   int32_t* ids;
-  uint32_t* flags;       // chunk-local, one per bucket
-  uint32_t* repair;      // chunk-local bucket list
-  unsigned int* n_repair;
+  // work lists of the chunk: buckets of 33 to kMediumCap entries, larger ones,
+  // and the buckets to repair now, by size class; counters: [0] medium, [1]
+  // large, [2] next large, [3 + c] repairs of class c
+  uint32_t* medium;
+  uint32_t* large;
+  uint32_t* repair[3];
+  unsigned* counters;
+  unsigned long long* n_repaired;  // over all chunks
+  // repairs put off to the end of the build, by class: copies of the buckets'
+  // entries and the items that name them; deferred: entries used, items by class
+  uint64_t* arena;
+  struct RepairItem* items[3];
+  unsigned* deferred;
+  unsigned arena_entries;
 };
 
-__global__ void k_compact(CompactArgs a) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// A bucket whose ties the reference's heap decides: B entries (in any order),
+// the first kp of the heap's order to ids[out..).
+struct RepairItem {
+  uint32_t pos, B, kp, out;
+};
+
+constexpr unsigned kMediumCap = 512;
+constexpr unsigned kArenaEntries = 1u << 23;
+constexpr unsigned kRepairItems = 1u << 16;  // per class
+
+// Random 8-byte writes into the chunk's buckets: a chunk is small enough that
+// most of them meet in L2.  (Seven passes of a stable radix sort over 12-byte
+// entries took 62 ms for 300M entries; this and the bucket sorts take the
+// place of those, of a compaction pass and of the ids' array.)
+__global__ void __launch_bounds__(256) k_bucket_scatter(BucketArgs a) {
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
   if (i >= a.N) return;
   const uint64_t key = a.keys[i];
-  const uint32_t grel = (uint32_t)(key >> 32);
-  const unsigned long long g = a.gbase + grel;
-  const uint32_t B = a.counts[g];
-  bool limited;
-  const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
-  const uint32_t rank = (uint32_t)(i - (long long)a.segstart[grel]);
-  if (rank < kp) {
-    a.ids[a.off[g] + rank] = (int32_t)a.vals[i];
-    if (rank + 1 < B && (rank + 1 == kp || a.exact_order)) {
-      if ((uint32_t)a.keys[i + 1] == (uint32_t)key) {  // equal score next to a kept entry
-        if (atomicOr(a.flags + grel, 1u) == 0u) {
-          const unsigned slot = atomicAdd(a.n_repair, 1u);
-          a.repair[slot] = grel;
+  const uint32_t pt = (i / (unsigned)a.P) % a.n;
+  a.seg[a.segstart[(uint32_t)(key >> 32)] + a.ranks[i]] = (key << 32) | pt;
+}
+
+// repair size classes: what one warp's block of shared memory holds
+constexpr unsigned kRepairCap[2] = {880, 7000};
+
+// A tie in bucket b: put off (the caller copies the entries to arena +
+// the returned position) while there is room, else repaired after this chunk
+// (0xffffffff).  A replay is one long chain, so the few hundred of a chunk
+// would leave the GPU waiting for the longest of them chunk after chunk (41 of
+// 205 ms at 1M x 200, 100 tables, 6,303 repairs); all at once they fill it.
+__device__ __forceinline__ unsigned add_repair(const BucketArgs& a, uint32_t b, uint32_t B, uint32_t kp, uint32_t out) {
+  const int c = B <= kRepairCap[0] ? 0 : B <= kRepairCap[1] ? 1 : 2;
+  atomicAdd(a.n_repaired, 1ull);
+  if (B <= a.arena_entries) {
+    const unsigned pos = atomicAdd(a.deferred, B);
+    if (pos <= a.arena_entries - B) {
+      const unsigned i = atomicAdd(a.deferred + 1 + c, 1u);
+      if (i < kRepairItems) {
+        a.items[c][i] = RepairItem{pos, B, kp, out};
+        return pos;
+      }
+      atomicSub(a.deferred + 1 + c, 1u);  // never below the items written
+    } else {
+      atomicSub(a.deferred, B);
+    }
+  }
+  a.repair[c][atomicAdd(a.counters + 3 + c, 1u)] = b;
+  return 0xffffffffu;
+}
+
+// Whether the kept entry at rank r and the next one make the reference's heap
+// order matter: equal scores at the cut, or (exact_order) anywhere before it.
+__device__ __forceinline__ bool tie_matters(const BucketArgs& a, uint32_t r, uint32_t kp, uint32_t B, uint64_t e,
+                                            uint64_t next) {
+  return r < kp && r + 1 < B && (r + 1 == kp || a.exact_order) && (uint32_t)(e >> 32) == (uint32_t)(next >> 32);
+}
+
+// One warp per 32 consecutive buckets: those of up to 32 entries are sorted in
+// registers, one at a time; larger ones go to the list.
+__global__ void __launch_bounds__(256) k_bucket_small(BucketArgs a) {
+  const int lane = threadIdx.x & 31;
+  const unsigned b0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * 32u;
+  if (b0 >= a.nb) return;
+  const unsigned b = b0 + lane;
+  uint32_t B = 0, s0 = 0, o = 0, kp = 0;
+  if (b < a.nb) {
+    B = a.counts[b];
+    bool limited;
+    kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
+    if (kp) {
+      s0 = a.segstart[b];
+      o = a.off[b];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const bool in = kp && B > 32 && (B > kMediumCap) == (c == 1);
+    const unsigned bal = __ballot_sync(kFullMask, in);
+    if (bal) {
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(a.counters + c, (unsigned)__popc(bal));
+      at = __shfl_sync(kFullMask, at, 0) + __popc(bal & ((1u << lane) - 1u));
+      if (in) (c ? a.large : a.medium)[at] = b;
+    }
+  }
+  if (kp && B == 1) a.ids[o] = (int32_t)(uint32_t)a.seg[s0];  // nothing to sort
+  unsigned todo = __ballot_sync(kFullMask, kp && B > 1 && B <= 32);
+  uint64_t next = ~0ull;  // the next bucket's entries, loaded ahead
+  if (todo) {
+    const int src = __ffs(todo) - 1;
+    const uint32_t nB = __shfl_sync(kFullMask, B, src), ns = __shfl_sync(kFullMask, s0, src);
+    if (lane < (int)nB) next = a.seg[ns + lane];
+  }
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const uint32_t cB = __shfl_sync(kFullMask, B, src), co = __shfl_sync(kFullMask, o, src),
+                   ck = __shfl_sync(kFullMask, kp, src);
+    uint64_t e = next;
+    next = ~0ull;
+    if (todo) {
+      const int nsrc = __ffs(todo) - 1;
+      const uint32_t nB = __shfl_sync(kFullMask, B, nsrc), ns = __shfl_sync(kFullMask, s0, nsrc);
+      if (lane < (int)nB) next = a.seg[ns + lane];
+    }
+    // bitonic sort over the lanes (ids differ, so do the entries), no wider
+    // than the bucket
+    for (int k = 2; (k >> 1) < (int)cB; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const uint64_t p = __shfl_xor_sync(kFullMask, e, j);
+        const bool up = (lane & k) == 0 || k == 32;
+        const bool low = (lane & j) == 0;
+        e = (low == up) == (e < p) ? e : p;
+      }
+    // blocks of k lanes alternate in direction: the first one ascends
+    const uint64_t after = __shfl_down_sync(kFullMask, e, 1);
+    if (lane < (int)ck) a.ids[co + lane] = (int32_t)(uint32_t)e;
+    if (__any_sync(kFullMask, tie_matters(a, lane, ck, cB, e, after))) {
+      unsigned pos = 0;
+      if (lane == 0) pos = add_repair(a, b0 + src, cB, ck, co);
+      pos = __shfl_sync(kFullMask, pos, 0);
+      if (pos != 0xffffffffu && lane < (int)cB) a.arena[pos + lane] = e;
+    }
+  }
+}
+
+// One warp per bucket of 33 to kMediumCap entries, sorted in its part of shared
+// memory; warps take the next bucket of the list by themselves.
+__global__ void __launch_bounds__(256) k_bucket_medium(BucketArgs a) {
+  __shared__ uint64_t sm[8][kMediumCap];
+  const int lane = threadIdx.x & 31;
+  uint64_t* e = sm[threadIdx.x >> 5];
+  const unsigned nm = a.counters[0];
+  for (unsigned item = blockIdx.x * 8u + (threadIdx.x >> 5); item < nm; item += gridDim.x * 8u) {
+    const uint32_t b = a.medium[item];
+    const uint32_t B = a.counts[b];
+    bool limited;
+    const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
+    const uint32_t out = a.off[b];
+    const uint64_t* g = a.seg + a.segstart[b];
+    int N = 64;
+    while (N < (int)B) N <<= 1;
+    for (int i = lane; i < N; i += 32) e[i] = i < (int)B ? g[i] : ~0ull;
+    __syncwarp();
+    for (int k = 2; k <= N; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int t = lane; t < N / 2; t += 32) {
+          const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo + j;
+          const uint64_t x = e[lo], y = e[hi];
+          if ((x > y) == ((lo & k) == 0)) {
+            e[lo] = y;
+            e[hi] = x;
+          }
+        }
+        __syncwarp();
+      }
+    bool tie = false;
+    for (uint32_t r = lane; r < kp; r += 32) {
+      a.ids[out + r] = (int32_t)(uint32_t)e[r];
+      tie |= tie_matters(a, r, kp, B, e[r], r + 1 < B ? e[r + 1] : 0ull);
+    }
+    if (__any_sync(kFullMask, tie)) {
+      unsigned pos = 0;
+      if (lane == 0) pos = add_repair(a, b, B, kp, out);
+      pos = __shfl_sync(kFullMask, pos, 0);
+      if (pos != 0xffffffffu)
+        for (uint32_t i = lane; i < B; i += 32) a.arena[pos + i] = e[i];
+    }
+    __syncwarp();
+  }
+}
+
+// Block-wide ascending bitonic sort of N (a power of two) entries: steps whose
+// pairs lie within 64 entries need only the warp that owns them.
+__device__ __forceinline__ void block_sort_entries(uint64_t* e, int N) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int k = 2; k <= N; k <<= 1) {
+    int j = k >> 1;
+    for (; j > 32; j >>= 1) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < N / 2; t += blockDim.x) {
+        const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo + j;
+        const uint64_t x = e[lo], y = e[hi];
+        if ((x > y) == ((lo & k) == 0)) {
+          e[lo] = y;
+          e[hi] = x;
         }
       }
+    }
+    __syncthreads();
+    for (int w = warp * 64; w < N; w += nw * 64)
+      for (int jj = j; jj > 0; jj >>= 1) {
+        const int lo = w + (((lane & ~(jj - 1)) << 1) | (lane & (jj - 1))), hi = lo + jj;
+        if (hi < N) {
+          const uint64_t x = e[lo], y = e[hi];
+          if ((x > y) == ((lo & k) == 0)) {
+            e[lo] = y;
+            e[hi] = x;
+          }
+        }
+        __syncwarp();
+      }
+  }
+  __syncthreads();
+}
+
+constexpr int kLargeSmem = 8192;  // entries sorted in shared memory (64 KB, three blocks per SM)
+
+// Persistent blocks over the list of larger buckets.  A bucket beyond the
+// shared memory is sorted where it lies, padded steps skipped.
+__global__ void __launch_bounds__(256) k_bucket_large(BucketArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint64_t* sm = reinterpret_cast<uint64_t*>(smem_raw);
+  __shared__ unsigned s_item, s_pos;
+  const unsigned nl = a.counters[1];
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = atomicAdd(a.counters + 2, 1u);
+    __syncthreads();
+    const unsigned item = s_item;
+    if (item >= nl) break;
+    const uint32_t b = a.large[item];
+    const uint32_t B = a.counts[b];
+    bool limited;
+    const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
+    uint64_t* g = a.seg + a.segstart[b];
+    int32_t* out = a.ids + a.off[b];
+    uint64_t* e = sm;
+    if (B <= (uint32_t)kLargeSmem) {
+      int N = 64;
+      while (N < (int)B) N <<= 1;
+      for (int i = threadIdx.x; i < N; i += 256) sm[i] = i < (int)B ? g[i] : ~0ull;
+      block_sort_entries(sm, N);
+    } else {
+      // all comparators ascending (mirror form): positions past the end act as
+      // +infinity and never move
+      e = g;
+      uint32_t N = 1;
+      while (N < B) N <<= 1;
+      for (uint32_t k = 2; k <= N; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+          __syncthreads();
+          for (uint32_t t = threadIdx.x; t < N / 2; t += 256) {
+            const uint32_t blk = t / j, r = t - blk * j;
+            const uint32_t lo = j == (k >> 1) ? blk * k + r : blk * 2 * j + r;
+            const uint32_t hi = j == (k >> 1) ? blk * k + k - 1 - r : lo + j;
+            if (hi < B) {
+              const uint64_t x = g[lo], y = g[hi];
+              if (x > y) {
+                g[lo] = y;
+                g[hi] = x;
+              }
+            }
+          }
+        }
+      __syncthreads();
+    }
+    bool tie = false;
+    for (uint32_t r = threadIdx.x; r < kp; r += 256) {
+      out[r] = (int32_t)(uint32_t)e[r];
+      tie |= tie_matters(a, r, kp, B, e[r], r + 1 < B ? e[r + 1] : 0ull);
+    }
+    if (__syncthreads_or(tie)) {
+      if (threadIdx.x == 0) s_pos = add_repair(a, b, B, kp, a.off[b]);
+      __syncthreads();
+      const unsigned pos = s_pos;
+      if (pos != 0xffffffffu)
+        for (uint32_t i = threadIdx.x; i < B; i += 256) a.arena[pos + i] = e[i];
     }
   }
 }
 
 // ---------------------------------------------------------------- tie repair
-constexpr int kRepairSmemEntries = 4096;  // 32 KB of static shared memory
+// A bucket's heap in one array: value and id together, slot i at h[i + 1], so
+// that both children of a slot are one aligned 16-byte load.  The operations
+// are those of fpp_heap.h (priority_queue push and pop on the value only, max
+// first).
+__device__ __forceinline__ void bucket_sift_up(uint2* h, int hole, int top, uint2 e) {
+  int parent = (hole - 1) / 2;
+  while (hole > top) {
+    const uint2 p = h[parent + 1];
+    if (!(__uint_as_float(p.x) < __uint_as_float(e.x))) break;
+    h[hole + 1] = p;
+    hole = parent;
+    parent = (hole - 1) / 2;
+  }
+  h[hole + 1] = e;
+}
 
-struct RepairArgs {
-  const uint64_t* keys;  // sorted
-  const uint32_t* vals;
-  uint32_t* sk;          // scratch ids   (alternate sort buffer, same positions)
-  uint32_t* sv;          // scratch scores
-  const uint32_t* counts;
-  const uint32_t* segstart;
-  const uint32_t* off;
-  unsigned long long gbase;
-  float alpha;
-  int P, minSize;
-  const uint32_t* repair;
-  const unsigned int* n_repair;
-  int32_t* ids;
-};
-
-// One block per bucket: put the bucket's entries back in push order (ascending
-// id, FalconnPP.cpp:75 / :200), then thread 0 replays the priority_queue pushes
-// and the first iLimit pops (FalconnPP.cpp:226-230).
-__global__ void __launch_bounds__(256) k_repair(RepairArgs a) {
-  __shared__ uint32_t s_id[kRepairSmemEntries];
-  __shared__ uint32_t s_sc[kRepairSmemEntries];
-  const unsigned nrep = *a.n_repair;
-  for (unsigned r = blockIdx.x; r < nrep; r += gridDim.x) {
-    const uint32_t grel = a.repair[r];
-    const unsigned long long g = a.gbase + grel;
-    const uint32_t B = a.counts[g];
-    bool limited;
-    const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
-    const uint32_t s0 = a.segstart[grel];
-    const bool in_smem = B <= (uint32_t)kRepairSmemEntries;
-    uint32_t* pid = in_smem ? s_id : a.sk + s0;
-    uint32_t* psc = in_smem ? s_sc : a.sv + s0;
-    for (uint32_t i = threadIdx.x; i < B; i += blockDim.x) {
-      pid[i] = a.vals[s0 + i];
-      psc[i] = ord_key_inv_dev(~(uint32_t)a.keys[s0 + i]);  // float bits of the score
+__device__ __forceinline__ void bucket_pop(uint2* h, int& n) {
+  if (n > 1) {
+    const int len = n - 1;
+    const uint2 last = h[len + 1];
+    int hole = 0, child = 0;
+    while (child < (len - 1) / 2) {
+      child = 2 * (child + 1);
+      const uint4 two = *reinterpret_cast<const uint4*>(h + child);  // slots child - 1, child
+      uint2 c = make_uint2(two.z, two.w);
+      if (__uint_as_float(two.z) < __uint_as_float(two.x)) {
+        c = make_uint2(two.x, two.y);
+        --child;
+      }
+      h[hole + 1] = c;
+      hole = child;
     }
-    __syncthreads();
-    block_bitonic_sort_u32(pid, psc, (int)B);
-    if (threadIdx.x == 0) {
-      float* hv = reinterpret_cast<float*>(psc);
-      int* hi = reinterpret_cast<int*>(pid);
-      int n = 0;
-      for (uint32_t i = 0; i < B; ++i) heap_push<false, int>(hv, hi, n, hv[i], hi[i]);
-      int32_t* out = a.ids + a.off[g];
-      for (uint32_t j = 0; j < kp; ++j) {
-        out[j] = hi[0];
-        heap_pop<false, int>(hv, hi, n);
+    if ((len & 1) == 0 && child == (len - 2) / 2) {
+      child = 2 * (child + 1);
+      h[hole + 1] = h[child];
+      hole = child - 1;
+    }
+    bucket_sift_up(h, hole, 0, last);
+  }
+  --n;
+}
+
+// One warp per bucket, its heap in CAP entries of shared memory (class 2: in
+// the seg array itself): the entries back in push order (ascending id,
+// FalconnPP.cpp:75 / :200), then lane 0 replays the priority_queue pushes and
+// the first iLimit pops (FalconnPP.cpp:226-230).  A replay is one chain of
+// dependent loads (about 45 clocks per level); the SM runs as many as fit its
+// shared memory.
+template <int CLS>
+__global__ void __launch_bounds__(32) k_repair(BucketArgs a, bool deferred) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x;
+  const unsigned nrep = deferred ? a.deferred[1 + CLS] : a.counters[3 + CLS];
+  for (unsigned r = blockIdx.x; r < nrep; r += gridDim.x) {
+    uint32_t B, kp;
+    uint64_t* g;
+    int32_t* out;
+    if (deferred) {
+      const RepairItem it = a.items[CLS][r];
+      B = it.B;
+      kp = it.kp;
+      g = a.arena + it.pos;
+      out = a.ids + it.out;
+    } else {
+      const uint32_t b = a.repair[CLS][r];
+      bool limited;
+      B = a.counts[b];
+      kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
+      g = a.seg + a.segstart[b];
+      out = a.ids + a.off[b];
+    }
+    // entries as (id << 32) | score bits, slot i at e[i + 1]
+    uint64_t* e = CLS == 2 ? g - 1 : reinterpret_cast<uint64_t*>(smem_raw);
+    for (uint32_t i = lane; i < B; i += 32) {
+      const uint64_t x = g[i];
+      e[i + 1] = (x << 32) | ord_key_inv_dev(~(uint32_t)(x >> 32));
+    }
+    __syncwarp();
+    uint32_t N = 1;
+    while (N < B) N <<= 1;
+    for (uint32_t k = 2; k <= N; k <<= 1)
+      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+        for (uint32_t t = lane; t < N / 2; t += 32) {
+          const uint32_t q = t & ~(j - 1), o = t & (j - 1);  // q = j * block
+          const uint32_t lo = 2 * q + o;
+          const uint32_t hi = j == (k >> 1) ? 2 * q + k - 1 - o : lo + j;
+          if (hi < B) {
+            const uint64_t x = e[lo + 1], y = e[hi + 1];
+            if (x > y) {
+              e[lo + 1] = y;
+              e[hi + 1] = x;
+            }
+          }
+        }
+        __syncwarp();
+      }
+    if (lane == 0) {
+      if constexpr (CLS == 2) {
+        // entry i keeps its place as (value, id); no aligned pairs here
+        for (uint32_t i = 0; i < B; ++i) {
+          const uint64_t x = g[i];
+          uint32_t hole = i;
+          const float v = __uint_as_float((uint32_t)x);
+          while (hole > 0) {
+            const uint32_t parent = (hole - 1) / 2;
+            const uint64_t p = g[parent];
+            if (!(__uint_as_float((uint32_t)p) < v)) break;
+            g[hole] = p;
+            hole = parent;
+          }
+          g[hole] = x;
+        }
+        int n = (int)B;
+        for (uint32_t j = 0; j < kp; ++j) {
+          out[j] = (int32_t)(uint32_t)(g[0] >> 32);
+          if (n > 1) {
+            const int len = n - 1;
+            const uint64_t last = g[len];
+            int hole = 0, child = 0;
+            while (child < (len - 1) / 2) {
+              child = 2 * (child + 1);
+              if (__uint_as_float((uint32_t)g[child]) < __uint_as_float((uint32_t)g[child - 1])) --child;
+              g[hole] = g[child];
+              hole = child;
+            }
+            if ((len & 1) == 0 && child == (len - 2) / 2) {
+              child = 2 * (child + 1);
+              g[hole] = g[child - 1];
+              hole = child - 1;
+            }
+            while (hole > 0) {
+              const int parent = (hole - 1) / 2;
+              if (!(__uint_as_float((uint32_t)g[parent]) < __uint_as_float((uint32_t)last))) break;
+              g[hole] = g[parent];
+              hole = parent;
+            }
+            g[hole] = last;
+          }
+          --n;
+        }
+      } else {
+        uint2* h = reinterpret_cast<uint2*>(smem_raw);
+        for (uint32_t i = 0; i < B; ++i) bucket_sift_up(h, (int)i, 0, h[i + 1]);
+        int n = (int)B;
+        for (uint32_t j = 0; j < kp; ++j) {
+          out[j] = (int32_t)h[1].y;
+          bucket_pop(h, n);
+        }
       }
     }
-    __syncthreads();
+    __syncwarp();
   }
 }
 
 // ---------------------------------------------------------------- host side
-template <int FHT>
-static cudaError_t launch_hash(const HashArgs& a, int nsm, cudaStream_t s) {
-  const size_t smem = HashSmem<FHT>::bytes;
-  cudaError_t e = cudaFuncSetAttribute(k_build_hash<FHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int FHT, int KEEP>
+static cudaError_t launch_hash_keep(const HashArgs& a, int nsm, cudaStream_t s) {
+  using SM = HashSmem<FHT, KEEP>;
+  const size_t smem = SM::bytes;
+  cudaError_t e =
+      cudaFuncSetAttribute(k_build_hash<FHT, KEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build_hash<FHT>, 128, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build_hash<FHT, KEEP>, 128, smem);
   if (e != cudaSuccess) return e;
-  const long long groups_needed = (a.n + HashSmem<FHT>::GROUPS - 1) / HashSmem<FHT>::GROUPS;
+  const long long groups_needed = (a.n + SM::GROUPS - 1) / SM::GROUPS;
   const long long grid = std::max(1LL, std::min<long long>((long long)nsm * std::max(per_sm, 1), groups_needed));
-  k_build_hash<FHT><<<(unsigned)grid, 128, smem, s>>>(a);
+  k_build_hash<FHT, KEEP><<<(unsigned)grid, 128, smem, s>>>(a);
   return cudaGetLastError();
+}
+
+template <int FHT>
+static cudaError_t launch_hash(const HashArgs& a, int nsm, cudaStream_t s) {
+  if constexpr (FHT >= 32) {
+    if (a.P == 1) return launch_hash_keep<FHT, 1>(a, nsm, s);
+    if (a.P == 2) return launch_hash_keep<FHT, 2>(a, nsm, s);
+    if (a.P == 3) return launch_hash_keep<FHT, 3>(a, nsm, s);
+  }
+  return launch_hash_keep<FHT, 0>(a, nsm, s);
 }
 
 static cudaError_t dispatch_hash(int fht, const HashArgs& a, int nsm, cudaStream_t s) {
@@ -636,21 +1031,22 @@ static cudaError_t dispatch_hash(int fht, const HashArgs& a, int nsm, cudaStream
   }
 }
 
+// The largest class first: its chains are the longest.
+static void launch_repairs(const BucketArgs& a, int nsm, bool deferred, cudaStream_t s) {
+  k_repair<2><<<(unsigned)nsm * 4, 32, 0, s>>>(a, deferred);
+  k_repair<1><<<(unsigned)nsm * 4, 32, (kRepairCap[1] + 2) * 8, s>>>(a, deferred);
+  k_repair<0><<<(unsigned)nsm * 28, 32, (kRepairCap[0] + 2) * 8, s>>>(a, deferred);
+}
+
 static double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
 void free_index(DeviceIndex& di) {
-  cudaFree(di.Xc);
-  cudaFree(di.center);
-  cudaFree(di.flips);
-  cudaFree(di.tflips);
-  cudaFree(di.bucket_off);
+  cudaFree(di.slab);
   cudaFree(di.ids);
   cudaFree(di.Xlp);
   cudaFree(di.Xlp_scale);
-  cudaFree(di.Xi8);
-  cudaFree(di.i8_norm_max);
   di = DeviceIndex();
 }
 
@@ -668,7 +1064,6 @@ int upload_flips(const Params& P, const HostBits& bits, DeviceIndex& di, cudaStr
           if (bit == 0) hflips[(((size_t)layer * L + l) * 3 + r) * WORDS + i / 32] |= 1u << (i % 32);
         }
   }
-  FPP_CUDA(fpp::dev_malloc(&di.flips, sizeof(uint32_t) * hflips.size()));
   FPP_CUDA(cudaMemcpyAsync(di.flips, hflips.data(), sizeof(uint32_t) * hflips.size(), cudaMemcpyHostToDevice, s));
   if (F == 256) {
     // the tensor-core rotation (batched low-precision form) reads round 2's
@@ -684,7 +1079,6 @@ int upload_flips(const Params& P, const HostBits& bits, DeviceIndex& di, cudaStr
         if ((src[p0 >> 5] >> (p0 & 31)) & 1u) dst[pp >> 5] |= 1u << (pp & 31);
       }
     }
-    FPP_CUDA(fpp::dev_malloc(&di.tflips, sizeof(uint32_t) * htflips.size()));
     FPP_CUDA(cudaMemcpyAsync(di.tflips, htflips.data(), sizeof(uint32_t) * htflips.size(), cudaMemcpyHostToDevice,
                              s));
   }
@@ -710,63 +1104,97 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
 
+  unsigned char* scratch = nullptr;  // everything below but the ids
   float* Xstage = nullptr;
   float* part = nullptr;
   int* d_bad = nullptr;
   uint32_t* counts = nullptr;
-  uint64_t* keys[2] = {nullptr, nullptr};
-  uint32_t* vals[2] = {nullptr, nullptr};
-  uint32_t* hist = nullptr;
-  uint32_t* digit_total = nullptr;
+  uint64_t* keys = nullptr;
+  uint32_t* ranks = nullptr;
+  uint64_t* seg = nullptr;
   uint32_t* segstart = nullptr;
-  uint32_t* flags = nullptr;
-  uint32_t* repair = nullptr;
-  unsigned int* n_repair = nullptr;
+  uint32_t* medium = nullptr;
+  uint32_t* large = nullptr;
+  uint64_t* arena = nullptr;
+  RepairItem* items[3] = {nullptr, nullptr, nullptr};
+  unsigned* deferred = nullptr;
+  uint32_t* repair[3] = {nullptr, nullptr, nullptr};
+  unsigned* counters = nullptr;
   unsigned long long* blk_cnt = nullptr;
   unsigned long long* blk_kept = nullptr;
-  unsigned long long* d_base = nullptr;
+  unsigned long long* totals = nullptr;  // ids before the next chunk, limited buckets, repaired buckets
   unsigned int* d_maxkept = nullptr;
-  unsigned long long* d_limited = nullptr;
+  BucketArgs ba;
   int32_t* ids_cap = nullptr;
   uint64_t ids_capacity = 0;
   int h_bad = 0;
   unsigned long long h_base = 0;
-  long long tables_per_chunk = 0;
-  const long long entry_cap = 1LL << 27;
-  long long max_entries = 0;
-  long long nb_chunk_max = 0;
-  long long nblk_max = 0;
-  int ntiles_max = 0;
+  // 2^24 entries a chunk (336 MB of scratch; the buckets' entries, 134 MB,
+  // about fill L2): larger chunks only cost memory
+  const long long entry_cap = 1LL << 24;
   const long long nchunks_c = (n + kCenterChunk - 1) / kCenterChunk;
+  const long long tables_per_chunk = std::min<long long>(
+      L, opt.tables_per_chunk > 0 ? opt.tables_per_chunk
+                                  : std::max(1LL, std::min<long long>(L, entry_cap / std::max(1LL, n * IP))));
+  const long long max_entries = std::max(1LL, tables_per_chunk * n * IP);
+  const long long nb_chunk_max = tables_per_chunk * (long long)NB;
+  const long long nblk_max = (nb_chunk_max + kScanTile - 1) / kScanTile;
+  // put-off repairs: the size of a small build's entries is enough
+  const unsigned arena_entries = (unsigned)std::min<unsigned long long>(kArenaEntries, (unsigned long long)L * n * IP);
 
   free_index(di);
-  di.ld = ld;
+  if (max_entries >= (1LL << 32) || nb_chunk_max >= (1LL << 32)) {
+    err.code = kErrUnsupported;
+    err.msg = "build: too many entries per table chunk";
+    goto fail;
+  }
+  FPP_CUDA(alloc_index(P, di));
+  {
+    Slab slab;
+    if (!x_on_device) slab.reserve(&Xstage, (size_t)n * d);
+    slab.reserve(&part, (size_t)nchunks_c * d);
+    slab.reserve(&d_bad, 1);
+    slab.reserve(&counts, nb_chunk_max);
+    slab.reserve(&keys, max_entries);
+    slab.reserve(&ranks, max_entries);
+    slab.reserve(&seg, max_entries);
+    slab.reserve(&segstart, nb_chunk_max);
+    // buckets of more than 32 and kMediumCap entries, and those that can need
+    // a repair (two entries or more; by class, more than its lower end)
+    slab.reserve(&medium, std::min(nb_chunk_max, max_entries / 33) + 1);
+    slab.reserve(&large, std::min(nb_chunk_max, max_entries / (long long)kMediumCap) + 1);
+    slab.reserve(&repair[0], std::min(nb_chunk_max, max_entries / 2) + 1);
+    slab.reserve(&repair[1], std::min(nb_chunk_max, max_entries / kRepairCap[0]) + 1);
+    slab.reserve(&repair[2], std::min(nb_chunk_max, max_entries / kRepairCap[1]) + 1);
+    slab.reserve(&arena, arena_entries);
+    for (int c = 0; c < 3; ++c) slab.reserve(&items[c], kRepairItems);
+    slab.reserve(&deferred, 4);
+    slab.reserve(&counters, 8);
+    slab.reserve(&blk_cnt, nblk_max);
+    slab.reserve(&blk_kept, nblk_max);
+    slab.reserve(&totals, 3);
+    slab.reserve(&d_maxkept, 1);
+    FPP_CUDA(slab.alloc(&scratch));
+  }
 
   // 1. centre
   {
     auto t0 = std::chrono::steady_clock::now();
     const float* Xd = X;
     if (!x_on_device) {
-      FPP_CUDA(fpp::dev_malloc(&Xstage, sizeof(float) * n * d));
       FPP_CUDA(cudaMemcpyAsync(Xstage, X, sizeof(float) * n * d, cudaMemcpyHostToDevice, s));
       Xd = Xstage;
     }
-    FPP_CUDA(fpp::dev_malloc(&di.Xc, sizeof(float) * n * ld));
-    FPP_CUDA(fpp::dev_malloc(&di.center, sizeof(float) * d));
-    FPP_CUDA(fpp::dev_malloc(&part, sizeof(float) * nchunks_c * d));
-    FPP_CUDA(fpp::dev_malloc(&d_bad, sizeof(int)));
     FPP_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
     dim3 g1((unsigned)nchunks_c, (unsigned)((d + 255) / 256));
     k_center_partial<<<g1, 256, 0, s>>>(Xd, n, d, part);
     k_center_final<<<(d + 255) / 256, 256, 0, s>>>(part, nchunks_c, n, d, di.center);
-    alloc_screen_rows(P, di, s);
+    if (di.Xi8) FPP_CUDA(cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s));
     k_center_rows<true><<<(unsigned)std::max(1, nsm * 8), 256, 0, s>>>(Xd, n, d, ld, di.center, di.Xc, di.Xi8,
                                                                        i8_row_bytes(d), di.i8_norm_max, d_bad);
     FPP_CUDA(cudaGetLastError());
     FPP_CUDA(cudaMemcpyAsync(&h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));
-    cudaFree(Xstage);
-    Xstage = nullptr;
     if (h_bad) {
       err.code = kErrNonFinite;
       err.msg = "build: the dataset contains NaN or infinite values";
@@ -779,39 +1207,12 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   if (upload_flips(P, bits, di, s, err) != kOk) goto fail;
 
   // 3. hash + sort + compact, a chunk of tables at a time
-  tables_per_chunk = opt.tables_per_chunk > 0 ? opt.tables_per_chunk
-                                               : std::max(1LL, std::min<long long>(L, entry_cap / std::max(1LL, n * IP)));
-  tables_per_chunk = std::min<long long>(tables_per_chunk, L);
-  max_entries = tables_per_chunk * n * IP;
-  nb_chunk_max = tables_per_chunk * (long long)NB;
-  nblk_max = (nb_chunk_max + kScanTile - 1) / kScanTile;
-  ntiles_max = (int)((max_entries + kRsTile - 1) / kRsTile);
-  if (max_entries >= (1LL << 32) || nb_chunk_max >= (1LL << 32)) {
-    err.code = kErrUnsupported;
-    err.msg = "build: too many entries per table chunk";
-    goto fail;
-  }
-  FPP_CUDA(fpp::dev_malloc(&counts, sizeof(uint32_t) * (size_t)L * NB));
-  FPP_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (size_t)L * NB, s));
-  FPP_CUDA(fpp::dev_malloc(&di.bucket_off, sizeof(uint32_t) * ((size_t)L * NB + 1)));
-  for (int i = 0; i < 2; ++i) {
-    FPP_CUDA(fpp::dev_malloc(&keys[i], sizeof(uint64_t) * std::max(1LL, max_entries)));
-    FPP_CUDA(fpp::dev_malloc(&vals[i], sizeof(uint32_t) * std::max(1LL, max_entries)));
-  }
-  FPP_CUDA(fpp::dev_malloc(&hist, sizeof(uint32_t) * 256 * (size_t)std::max(1, ntiles_max)));
-  FPP_CUDA(fpp::dev_malloc(&digit_total, sizeof(uint32_t) * 256));
-  FPP_CUDA(fpp::dev_malloc(&segstart, sizeof(uint32_t) * nb_chunk_max));
-  FPP_CUDA(fpp::dev_malloc(&flags, sizeof(uint32_t) * nb_chunk_max));
-  FPP_CUDA(fpp::dev_malloc(&repair, sizeof(uint32_t) * nb_chunk_max));
-  FPP_CUDA(fpp::dev_malloc(&n_repair, sizeof(unsigned int)));
-  FPP_CUDA(fpp::dev_malloc(&blk_cnt, sizeof(unsigned long long) * nblk_max));
-  FPP_CUDA(fpp::dev_malloc(&blk_kept, sizeof(unsigned long long) * nblk_max));
-  FPP_CUDA(fpp::dev_malloc(&d_base, sizeof(unsigned long long)));
-  FPP_CUDA(fpp::dev_malloc(&d_maxkept, sizeof(unsigned int)));
-  FPP_CUDA(fpp::dev_malloc(&d_limited, sizeof(unsigned long long)));
-  FPP_CUDA(cudaMemsetAsync(d_base, 0, sizeof(unsigned long long), s));
+  FPP_CUDA(cudaMemsetAsync(deferred, 0, sizeof(unsigned) * 4, s));
+  FPP_CUDA(cudaMemsetAsync(totals, 0, sizeof(unsigned long long) * 3, s));
   FPP_CUDA(cudaMemsetAsync(d_maxkept, 0, sizeof(unsigned int), s));
-  FPP_CUDA(cudaMemsetAsync(d_limited, 0, sizeof(unsigned long long), s));
+  FPP_CUDA(cudaFuncSetAttribute(k_bucket_large, cudaFuncAttributeMaxDynamicSharedMemorySize, kLargeSmem * 8));
+  FPP_CUDA(cudaFuncSetAttribute(k_repair<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(kRepairCap[1] + 2) * 8));
 
   for (long long l0 = 0; l0 < L; l0 += tables_per_chunk) {
     const long long l1 = std::min<long long>(L, l0 + tables_per_chunk);
@@ -831,11 +1232,12 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     ha.log2D = log2D;
     ha.P = IP;
     ha.NB = NB;
-    ha.keys = keys[0];
-    ha.vals = vals[0];
+    ha.keys = keys;
+    ha.ranks = ranks;
     ha.counts = counts;
     ha.dump_codes = dump_codes;
     ha.dump_scores = dump_scores;
+    FPP_CUDA(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * nbc, s));
     FPP_CUDA(dispatch_hash(F, ha, nsm, s));
     FPP_CUDA(cudaStreamSynchronize(s));
     st.ms_hash += ms_since(t0);
@@ -843,7 +1245,7 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     // bucket limits and CSR offsets of this chunk
     t0 = std::chrono::steady_clock::now();
     ScanArgs sa;
-    sa.counts = counts + l0 * NB;
+    sa.counts = counts;
     sa.nb = nbc;
     sa.alpha = P.bucket_scale;
     sa.P = IP;
@@ -852,15 +1254,15 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     sa.off = di.bucket_off + l0 * NB;
     sa.blk_cnt = blk_cnt;
     sa.blk_kept = blk_kept;
-    sa.base = d_base;
+    sa.base = totals;
     sa.max_kept = d_maxkept;
-    sa.n_limited = d_limited;
+    sa.n_limited = totals + 1;
     const long long nblk = (nbc + kScanTile - 1) / kScanTile;
     k_scan_reduce<<<(unsigned)nblk, kScanThreads, 0, s>>>(sa);
     k_scan_blocks<<<1, kScanThreads, 0, s>>>(sa, nblk);
     k_scan_down<<<(unsigned)nblk, kScanThreads, 0, s>>>(sa);
     FPP_CUDA(cudaGetLastError());
-    FPP_CUDA(cudaMemcpyAsync(&h_base, d_base, sizeof(h_base), cudaMemcpyDeviceToHost, s));
+    FPP_CUDA(cudaMemcpyAsync(&h_base, totals, sizeof(h_base), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));
     if (h_base >= (1ULL << 32)) {
       err.code = kErrUnsupported;
@@ -868,7 +1270,8 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
       goto fail;
     }
     if (h_base > ids_capacity) {  // grow the 1D table
-      uint64_t cap = std::max<uint64_t>(h_base, ids_capacity * 3 / 2);
+      // what the tables so far kept, for all tables, and a little more
+      uint64_t cap = (uint64_t)((double)h_base / (double)l1 * (double)L * 1.02) + 1024;
       cap = std::min<uint64_t>(std::max<uint64_t>(cap, h_base), std::max<uint64_t>(h_base, (uint64_t)L * n * IP));
       int32_t* nids = nullptr;
       FPP_CUDA(fpp::dev_malloc(&nids, sizeof(int32_t) * cap));
@@ -882,127 +1285,71 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     di.n_ids = h_base;
     st.ms_csr += ms_since(t0);
 
-    // sort the chunk's entries by (bucket, score desc), stable
+    // the entries to their buckets, each bucket sorted, ties repaired
     t0 = std::chrono::steady_clock::now();
-    int bbits = 0;
-    while ((1LL << bbits) < nbc) ++bbits;
-    const int total_bits = 32 + bbits;
-    const int ntiles = (int)((Ne + kRsTile - 1) / kRsTile);
-    int cur = 0;
-    for (int shift = 0; shift < total_bits; shift += 8) {
-      k_rs_hist<<<ntiles, kRsThreads, 0, s>>>(keys[cur], Ne, shift, hist, ntiles);
-      k_rs_scan<<<256, 1024, 0, s>>>(hist, ntiles, digit_total);
-      k_rs_scatter<<<ntiles, kRsThreads, 0, s>>>(keys[cur], vals[cur], keys[cur ^ 1], vals[cur ^ 1], Ne, shift, hist,
-                                                 ntiles, digit_total);
-      cur ^= 1;
-    }
+    ba.keys = keys;
+    ba.ranks = ranks;
+    ba.N = (unsigned)Ne;
+    ba.n = (unsigned)n;
+    ba.P = IP;
+    ba.counts = counts;
+    ba.segstart = segstart;
+    ba.off = di.bucket_off + l0 * NB;
+    ba.nb = (unsigned)nbc;
+    ba.alpha = P.bucket_scale;
+    ba.minSize = P.bucket_minSize;
+    ba.exact_order = opt.exact_bucket_order ? 1 : 0;
+    ba.seg = seg;
+    ba.ids = ids_cap;
+    ba.medium = medium;
+    ba.large = large;
+    ba.arena = arena;
+    for (int c = 0; c < 3; ++c) ba.items[c] = items[c];
+    ba.deferred = deferred;
+    ba.arena_entries = arena_entries;
+    for (int c = 0; c < 3; ++c) ba.repair[c] = repair[c];
+    ba.counters = counters;
+    ba.n_repaired = totals + 2;
+    FPP_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned) * 8, s));
+    k_bucket_scatter<<<(unsigned)((Ne + 255) / 256), 256, 0, s>>>(ba);
+    k_bucket_small<<<(unsigned)((nbc + 255) / 256), 256, 0, s>>>(ba);
+    k_bucket_large<<<(unsigned)nsm * 3, 256, kLargeSmem * 8, s>>>(ba);
+    k_bucket_medium<<<(unsigned)nsm * 6, 256, 0, s>>>(ba);
+    launch_repairs(ba, nsm, false, s);
     FPP_CUDA(cudaGetLastError());
     FPP_CUDA(cudaStreamSynchronize(s));
     st.ms_sort += ms_since(t0);
-
-    t0 = std::chrono::steady_clock::now();
-    FPP_CUDA(cudaMemsetAsync(flags, 0, sizeof(uint32_t) * nbc, s));
-    FPP_CUDA(cudaMemsetAsync(n_repair, 0, sizeof(unsigned int), s));
-    CompactArgs ca;
-    ca.keys = keys[cur];
-    ca.vals = vals[cur];
-    ca.N = Ne;
-    ca.counts = counts;
-    ca.segstart = segstart;
-    ca.off = di.bucket_off;
-    ca.gbase = (unsigned long long)l0 * NB;
-    ca.alpha = P.bucket_scale;
-    ca.P = IP;
-    ca.minSize = P.bucket_minSize;
-    ca.exact_order = opt.exact_bucket_order ? 1 : 0;
-    ca.ids = ids_cap;
-    ca.flags = flags;
-    ca.repair = repair;
-    ca.n_repair = n_repair;
-    k_compact<<<(unsigned)((Ne + 255) / 256), 256, 0, s>>>(ca);
+  }
+  {
+    auto t0 = std::chrono::steady_clock::now();
+    ba.ids = ids_cap;
+    launch_repairs(ba, nsm, true, s);
     FPP_CUDA(cudaGetLastError());
-    unsigned int h_rep = 0;
-    FPP_CUDA(cudaMemcpyAsync(&h_rep, n_repair, sizeof(h_rep), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));
-    if (h_rep) {
-      RepairArgs ra;
-      ra.keys = keys[cur];
-      ra.vals = vals[cur];
-      ra.sk = reinterpret_cast<uint32_t*>(keys[cur ^ 1]);
-      ra.sv = vals[cur ^ 1];
-      ra.counts = counts;
-      ra.segstart = segstart;
-      ra.off = di.bucket_off;
-      ra.gbase = (unsigned long long)l0 * NB;
-      ra.alpha = P.bucket_scale;
-      ra.P = IP;
-      ra.minSize = P.bucket_minSize;
-      ra.repair = repair;
-      ra.n_repair = n_repair;
-      ra.ids = ids_cap;
-      k_repair<<<std::min<unsigned>(h_rep, (unsigned)nsm * 4), 256, 0, s>>>(ra);
-      FPP_CUDA(cudaGetLastError());
-      FPP_CUDA(cudaStreamSynchronize(s));
-    }
-    st.n_repaired += h_rep;
-    st.ms_csr += ms_since(t0);
+    st.ms_sort += ms_since(t0);
   }
   {
     const uint32_t last = (uint32_t)h_base;
     FPP_CUDA(cudaMemcpyAsync(di.bucket_off + (size_t)L * NB, &last, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-    unsigned long long lim = 0;
+    unsigned long long lim[2] = {0, 0};
     FPP_CUDA(cudaMemcpyAsync(&di.max_kept, d_maxkept, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-    FPP_CUDA(cudaMemcpyAsync(&lim, d_limited, sizeof(lim), cudaMemcpyDeviceToHost, s));
+    FPP_CUDA(cudaMemcpyAsync(lim, totals + 1, sizeof(lim), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));
-    st.n_limited = (long long)lim;
+    st.n_limited = (long long)lim[0];
+    st.n_repaired = (long long)lim[1];
     st.points_per_table = (double)h_base / (double)n / (double)L;
   }
   if (ids_cap == nullptr) FPP_CUDA(fpp::dev_malloc(&ids_cap, sizeof(int32_t)));
   di.ids = ids_cap;
   ids_cap = nullptr;
 
-  cudaFree(part);
-  cudaFree(d_bad);
-  cudaFree(counts);
-  for (int i = 0; i < 2; ++i) {
-    cudaFree(keys[i]);
-    cudaFree(vals[i]);
-  }
-  cudaFree(hist);
-  cudaFree(digit_total);
-  cudaFree(segstart);
-  cudaFree(flags);
-  cudaFree(repair);
-  cudaFree(n_repair);
-  cudaFree(blk_cnt);
-  cudaFree(blk_kept);
-  cudaFree(d_base);
-  cudaFree(d_maxkept);
-  cudaFree(d_limited);
+  cudaFree(scratch);
   st.ms_total = ms_since(t_start);
   return kOk;
 
 fail:
   cudaStreamSynchronize(s);
-  cudaFree(Xstage);
-  cudaFree(part);
-  cudaFree(d_bad);
-  cudaFree(counts);
-  for (int i = 0; i < 2; ++i) {
-    cudaFree(keys[i]);
-    cudaFree(vals[i]);
-  }
-  cudaFree(hist);
-  cudaFree(digit_total);
-  cudaFree(segstart);
-  cudaFree(flags);
-  cudaFree(repair);
-  cudaFree(n_repair);
-  cudaFree(blk_cnt);
-  cudaFree(blk_kept);
-  cudaFree(d_base);
-  cudaFree(d_maxkept);
-  cudaFree(d_limited);
+  cudaFree(scratch);
   cudaFree(ids_cap);
   free_index(di);
   return err.code;

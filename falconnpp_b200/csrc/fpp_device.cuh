@@ -136,13 +136,91 @@ template <int FHT, int EL = Geo<FHT>::E>
 __device__ __forceinline__ void hd3_rotate(float (&y)[EL], const uint32_t* flips, int gl) {
   constexpr int WORDS = Geo<FHT>::WORDS;
   constexpr int NW = EL >= 32 ? EL / 32 : 1;  // flip words per lane
+  // rolled: three copies of a round (350 instructions each) are more than the
+  // instruction caches hold beside the callers' code
+  uint32_t w[3][NW];  // loaded ahead of the rounds
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) w[r][k] = flips[r * WORDS + (FHT < 32 ? 0 : gl * NW + k)];
+#pragma unroll 1
+  for (int r = 0; r < 3; ++r) {
+    flip_signs<FHT, EL>(y, w[0]);
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+      w[0][k] = w[1][k];
+      w[1][k] = w[2][k];
+    }
+    fwht_group<FHT, EL>(y, gl);
+  }
+}
+
+// ---------------------------------------------------------------- packed vectors
+// The same rotation on a lane's 32 elements held as 16 register pairs
+// (elements 2j and 2j + 1): packed instructions take the pairs as they are, and
+// 16-byte loads and stores move two of them (with the elements in scalars, the
+// pairs of j and j + 16 above cost a move per element at every load and
+// store).  Here the stage h = 1 is the one inside the pairs.  Rounding is the
+// scalar operations'.
+typedef unsigned long long f2;  // two floats: low word, high word
+
+__device__ __forceinline__ float f2_lo(f2 p) { return __uint_as_float((uint32_t)p); }
+__device__ __forceinline__ float f2_hi(f2 p) { return __uint_as_float((uint32_t)(p >> 32)); }
+__device__ __forceinline__ f2 f2_make(float lo, float hi) {
+  f2 p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+
+template <int FHT>
+__device__ __forceinline__ void fwht_pairs(f2 (&p)[16], int gl) {
+  constexpr int N = 16;
+  constexpr int G = Geo<FHT>::G;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const float a = f2_lo(p[j]), b = f2_hi(p[j]);
+    p[j] = f2_make(__fadd_rn(a, b), __fsub_rn(a, b));
+  }
+#pragma unroll
+  for (int h = 1; h < N; h <<= 1) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (j & h) continue;
+      f2 sum, dif;
+      asm("add.rn.f32x2 %0, %2, %3;\n sub.rn.f32x2 %1, %2, %3;" : "=&l"(sum), "=l"(dif) : "l"(p[j]), "l"(p[j + h]));
+      p[j] = sum;
+      p[j + h] = dif;
+    }
+  }
+#pragma unroll
+  for (int s = 1; s < G; s <<= 1) {
+    const float sg = (gl & s) ? -1.0f : 1.0f;
+    const f2 sgn = f2_make(sg, sg);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float o0 = __shfl_xor_sync(kFullMask, f2_lo(p[j]), s);
+      const float o1 = __shfl_xor_sync(kFullMask, f2_hi(p[j]), s);
+      const f2 o = f2_make(o0, o1);
+      asm("fma.rn.f32x2 %0, %1, %0, %2;" : "+l"(p[j]) : "l"(sgn), "l"(o));  // exact product: one rounding
+    }
+  }
+}
+
+template <int FHT>
+__device__ __forceinline__ void hd3_rotate_pairs(f2 (&p)[16], const uint32_t* flips, int gl) {
+  constexpr int WORDS = Geo<FHT>::WORDS;
+  uint32_t w0 = flips[gl], w1 = flips[WORDS + gl], w2 = flips[2 * WORDS + gl];  // loaded ahead of the rounds
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
-    uint32_t w[NW];
 #pragma unroll
-    for (int k = 0; k < NW; ++k) w[k] = flips[r * WORDS + (FHT < 32 ? 0 : gl * NW + k)];
-    flip_signs<FHT, EL>(y, w);
-    fwht_group<FHT, EL>(y, gl);
+    for (int j = 0; j < 16; ++j) {
+      const uint32_t lo = (uint32_t)p[j] ^ ((w0 << (31 - 2 * j)) & 0x80000000u);
+      const uint32_t hi = (uint32_t)(p[j] >> 32) ^ ((w0 << (30 - 2 * j)) & 0x80000000u);
+      p[j] = f2_make(__uint_as_float(lo), __uint_as_float(hi));
+    }
+    w0 = w1;
+    w1 = w2;
+    fwht_pairs<FHT>(p, gl);
   }
 }
 
@@ -395,6 +473,188 @@ __device__ __forceinline__ bool group_top1_strict(const float (&y)[EL], int gl, 
     out_c[0] = cp_code(wy, owner_gl * E + wpos, log2D);
   }
   return tot == 1 && D >= 2;
+}
+
+// ---------------------------------------------------------------- key selection
+// The largest cnt <= C (2 or 4) coordinates of the group's vector by one u32 key per
+// element, |y| with its low log2(FHT) bits replaced by the position: a sorting
+// network of integer min / max, no branches and no positions to carry.  Keys
+// order the coordinates as their values do wherever two of the cnt best differ
+// above the replaced bits; then the result is exact and strict (`true`, on
+// every lane of the group).  Otherwise (equal or nearly equal values, about
+// one vector in 500 at FHT 256; or a value that is not finite) the caller takes
+// the exact selection.  Issue slots bound the hashing kernels: the insertion of
+// every element into a sorted list of four took about 800 of a warp's 1,700
+// instructions per layer, this takes about 250.
+__device__ __forceinline__ void key_sort2(uint32_t& a, uint32_t& b) {  // a >= b
+  const uint32_t hi = max(a, b);
+  b = min(a, b);
+  a = hi;
+}
+
+// a[0..C) = the C largest of a and b, both descending (b reversed pairs up
+// with a as a bitonic sequence)
+template <int C>
+__device__ __forceinline__ void key_merge(uint32_t (&a)[C], const uint32_t (&b)[C]) {
+  if constexpr (C == 2) {
+    const uint32_t t = min(a[0], b[0]);
+    a[0] = max(a[0], b[0]);
+    a[1] = max(t, max(a[1], b[1]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = max(a[i], b[3 - i]);
+    key_sort2(a[0], a[2]);
+    key_sort2(a[1], a[3]);
+    key_sort2(a[0], a[1]);
+    key_sort2(a[2], a[3]);
+  }
+}
+
+template <int FHT, int C, typename Bits>
+__device__ __forceinline__ bool group_top_keys(Bits bits, int gl, int D, int cnt, uint32_t (&k)[C]) {
+  constexpr int E = Geo<FHT>::E;  // bits(e): the bits of the lane's element e
+  constexpr int G = Geo<FHT>::G;
+  static_assert(E == 32 && (C == 2 || C == 4), "32 elements per lane");
+  constexpr uint32_t kPos = FHT - 1;
+  const uint32_t p0 = (uint32_t)(gl * E);
+  const int lim = D - gl * E;  // elements of this lane that are coordinates (< D)
+#pragma unroll
+  for (int e0 = 0; e0 < E; e0 += C) {
+    uint32_t t[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+      t[i] = (bits(e0 + i) & (0x7fffffffu & ~kPos)) | (p0 + (uint32_t)(e0 + i));
+    if (D < FHT) {
+#pragma unroll
+      for (int i = 0; i < C; ++i)
+        if (e0 + i >= lim) t[i] = 0u;
+    }
+    key_sort2(t[0], t[1]);
+    if constexpr (C == 4) {
+      key_sort2(t[2], t[3]);
+      key_sort2(t[0], t[2]);
+      key_sort2(t[1], t[3]);
+      key_sort2(t[1], t[2]);
+    }
+    if (e0 == 0) {
+#pragma unroll
+      for (int i = 0; i < C; ++i) k[i] = t[i];
+    } else {
+      key_merge<C>(k, t);
+    }
+  }
+#pragma unroll
+  for (int s = 1; s < G; s <<= 1) {
+    uint32_t o[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i) o[i] = __shfl_xor_sync(kFullMask, k[i], s);
+    key_merge<C>(k, o);
+  }
+  bool ok = (k[0] & 0x7f800000u) != 0x7f800000u;
+#pragma unroll
+  for (int i = 1; i < C; ++i) ok = ok && (i >= cnt || (k[i - 1] & ~kPos) != (k[i] & ~kPos));
+  return ok;
+}
+
+// Vectors in shared memory, 32 floats per lane and lanes 36 floats apart (the
+// 16-byte accesses of eight lanes then fall in different banks).
+template <int FHT>
+struct LaneVector {
+  static constexpr int kFloats = Geo<FHT>::G * 36;
+  static __device__ __forceinline__ void store(float* v, const float (&y)[32], int gl) {
+    float4* p = reinterpret_cast<float4*>(v + gl * 36);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) p[e] = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
+  }
+  static __device__ __forceinline__ void store(float* v, const f2 (&p)[16], int gl) {
+    ulonglong2* o = reinterpret_cast<ulonglong2*>(v + gl * 36);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = make_ulonglong2(p[2 * e], p[2 * e + 1]);
+  }
+  static __device__ __forceinline__ void load(const float* v, f2 (&p)[16], int gl) {
+    const ulonglong2* o = reinterpret_cast<const ulonglong2*>(v + gl * 36);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const ulonglong2 x = o[e];
+      p[2 * e] = x.x;
+      p[2 * e + 1] = x.y;
+    }
+  }
+  static __device__ __forceinline__ float& at(float* v, int pos) { return v[(pos >> 5) * 36 + (pos & 31)]; }
+};
+
+// Top-cnt of a stored vector's coordinates in canonical order (value desc,
+// position asc) into out_v / out_c on lane gl == 0, and whether they are
+// strictly decreasing, on every lane: the exact selection where keys cannot
+// tell (rare, so by rounds: each takes the best coordinate after the last).
+template <int FHT>
+__device__ __forceinline__ bool group_top_stored(float* v, int gl, int D, int log2D, int cnt, float* out_v, int* out_c) {
+  constexpr int G = Geo<FHT>::G;
+  float pv = 0.0f;
+  int pr = -1;
+  bool strict = true;
+  for (int t = 0; t < cnt; ++t) {
+    float bv = -1.0f;
+    int br = 0x7fffffff;
+    for (int r = gl; r < D; r += G) {
+      const float x = cp_value(LaneVector<FHT>::at(v, r));
+      if ((t == 0 || cp_better(pv, pr, x, r)) && cp_better(x, r, bv, br)) {
+        bv = x;
+        br = r;
+      }
+    }
+#pragma unroll
+    for (int s = 1; s < G; s <<= 1) {
+      const float ov = __shfl_xor_sync(kFullMask, bv, s);
+      const int orr = __shfl_xor_sync(kFullMask, br, s);
+      if (cp_better(ov, orr, bv, br)) {
+        bv = ov;
+        br = orr;
+      }
+    }
+    if (br == 0x7fffffff) return false;  // not comparable (NaN): the replay decides
+    strict = strict && (t == 0 || pv > bv);
+    pv = bv;
+    pr = br;
+    if (gl == 0) {
+      out_v[t] = bv;
+      out_c[t] = cp_code(LaneVector<FHT>::at(v, br), br, log2D);
+    }
+  }
+  return strict;
+}
+
+// The n (1..4) largest of the sums of two lists, with their pair indexes
+// 4 i + j, in descending order, from lists v1 and v2 of p strictly decreasing
+// values (p = n up to 3 for the build, 2 for the query's n = 2..4).  False
+// where equal sums leave the choice or the order to the reference's heap.
+// Rounded sums are monotone in both arguments, so for n <= 3 only pairs with
+// (i + 1)(j + 1) <= n, and the next ones as ties, can be involved.
+__device__ __forceinline__ bool top_pairs(const float* v1, const float* v2, int p, int n, float (&s)[4], int (&ij)[4]) {
+  s[0] = __fadd_rn(v1[0], v2[0]);
+  ij[0] = 0;
+  if (n == 1) return true;
+  const float s01 = __fadd_rn(v1[0], v2[1]), s10 = __fadd_rn(v1[1], v2[0]), s11 = __fadd_rn(v1[1], v2[1]);
+  const bool a = s01 > s10;
+  s[1] = a ? s01 : s10;
+  ij[1] = a ? 1 : 4;
+  const float x = a ? s10 : s01;  // the other one
+  const int xi = a ? 4 : 1;
+  bool ok = s[0] > s[1] && s01 != s10;
+  if (n == 2) return ok && s[1] > s11 && (p < 3 || (s[1] > __fadd_rn(v1[0], v2[2]) && s[1] > __fadd_rn(v1[2], v2[0])));
+  if (p == 2) {  // all four pairs are known
+    s[2] = x;
+    ij[2] = xi;
+    s[3] = s11;
+    ij[3] = 5;
+    return ok && x > s11;
+  }
+  const float s02 = __fadd_rn(v1[0], v2[2]), s20 = __fadd_rn(v1[2], v2[0]);
+  const float y = a ? s02 : s20, z = a ? s20 : s02;
+  const bool b = x > y;
+  s[2] = b ? x : y;
+  ij[2] = b ? xi : (a ? 2 : 8);
+  return ok && x != y && s[1] > s[2] && s[2] > s11 && s[2] > z;
 }
 
 // Dispatch: the single-pass selection when cnt is small, the round-based one

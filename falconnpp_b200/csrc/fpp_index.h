@@ -4,7 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace fpp {
@@ -57,6 +59,9 @@ struct Params {
 enum RerankMode : int { kRerankFP32 = 0, kRerankBF16 = 1, kRerankFP8 = 2 };
 
 struct DeviceIndex {
+  // one allocation (alloc_index) holds Xc, center, flips, tflips, bucket_off,
+  // Xi8 and i8_norm_max
+  unsigned char* slab = nullptr;
   // centred data, point-major, row stride ld floats (ld = d rounded up to 4)
   float* Xc = nullptr;
   int ld = 0;
@@ -105,9 +110,40 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
 
 void free_index(DeviceIndex& di);
 
-// The int8 screening rows of the centred data di.Xc (asynchronous on s).
-// Only for d <= 512, the batched form's range.  A failed allocation leaves
-// the index without them.
+// The index's arrays whose sizes follow from the parameters, in one allocation
+// (each allocation of the driver's takes a millisecond or so).  The int8
+// screening rows are part of it for d <= 512, the batched form's range; where
+// it does not fit with them, it is made without.
+cudaError_t alloc_index(const Params& P, DeviceIndex& di);
+
+// One allocation cut into 256-byte aligned arrays: reserve() each pointer,
+// then alloc().  All pointers are null after a failure.
+class Slab {
+ public:
+  template <typename T>
+  void reserve(T** p, size_t n) {
+    *p = nullptr;
+    parts_.push_back({reinterpret_cast<void**>(p), total_});
+    total_ += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
+  }
+  size_t bytes() const { return total_; }
+  cudaError_t alloc(unsigned char** base) {
+    const cudaError_t e = dev_malloc(base, total_);
+    if (e != cudaSuccess) {
+      *base = nullptr;
+      return e;
+    }
+    for (auto& p : parts_) *p.first = *base + p.second;
+    return cudaSuccess;
+  }
+
+ private:
+  std::vector<std::pair<void**, size_t>> parts_;
+  size_t total_ = 0;
+};
+
+// The int8 screening rows of the centred data di.Xc (asynchronous on s), if
+// the index has room for them.
 void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s);
 
 // The sign flip words (and, for fhtDim 256, their per-view copy for the

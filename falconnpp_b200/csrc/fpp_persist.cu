@@ -172,15 +172,20 @@ int fpp_load(fpp_index* h, const char* path) {
     h->bfw.release();
   fpp::free_index(h->di);
   h->built = false;
+  fpp::Params P = h->P;
+  P.n_tables = hd.n_tables;
+  P.n_proj = hd.n_proj;
+  P.bucket_minSize = hd.bucket_minSize;
+  P.bucket_scale = hd.bucket_scale;
+  P.iProbes = hd.iProbes;
+  P.seed = hd.seed;
+  P.fhtDim = hd.fhtDim;
   fpp::DeviceIndex di;
-  di.ld = hd.ld;
   di.n_ids = hd.n_ids;
   std::vector<unsigned char> buf(kChunk);
   const uint64_t n = (uint64_t)hd.n_points;
   uint32_t prev = 0, max_kept = 0;
-  bool okr = fpp::dev_malloc(&di.center, sizeof(float) * (size_t)hd.n_features) == cudaSuccess &&
-             fpp::dev_malloc(&di.Xc, sizeof(float) * (size_t)n * hd.ld) == cudaSuccess &&
-             fpp::dev_malloc(&di.bucket_off, sizeof(uint32_t) * (size_t)(hd.n_buckets + 1)) == cudaSuccess &&
+  bool okr = fpp::alloc_index(P, di) == cudaSuccess &&
              fpp::dev_malloc(&di.ids, sizeof(int32_t) * std::max<size_t>(1, (size_t)hd.n_ids)) == cudaSuccess;
   std::string why = okr ? "" : "cannot allocate the index on the device";
   auto any = [](const void*, size_t, size_t) { return true; };
@@ -209,14 +214,6 @@ int fpp_load(fpp_index* h, const char* path) {
     if (!okr) why = "an id outside [0, n_points)";
   }
   fclose(f);
-  fpp::Params P = h->P;
-  P.n_tables = hd.n_tables;
-  P.n_proj = hd.n_proj;
-  P.bucket_minSize = hd.bucket_minSize;
-  P.bucket_scale = hd.bucket_scale;
-  P.iProbes = hd.iProbes;
-  P.seed = hd.seed;
-  P.fhtDim = hd.fhtDim;
   fpp::Error err{0, ""};
   if (okr && fpp::upload_flips(P, bits, di, h->stream, err) != fpp::kOk) {
     okr = false;

@@ -190,11 +190,24 @@ static KernelSel pick_kernel(int fht, int mode, int d, bool tc_only) {
   return pick_kernel_fp8(fht, d, tc_only);
 }
 
+// Blocks per query of a small batch: a cluster helps while SMs would be idle.
+// The fused kernel alone, 1M x 200, FP32, in us with 1 / 2 / 4 / 8 blocks per
+// query: qProbes 10: 1 query 55 / 41 / 33 / 27, 18 queries 55 / 41 / 33 / 33,
+// 37 queries 59 / 43 / 39 / 37, 148 queries 66 / 55, 220 queries 74 / 68;
+// qProbes 2: 1 query 31 / 29 / 25 / 25, 37 queries 33 / 29 / 29 / 33, 148
+// queries 35 / 35.
+static int cluster_size(int nq, int nsm) {
+  if (8LL * nq <= nsm) return 8;
+  if (4LL * nq <= nsm) return 4;
+  if (2LL * nq <= 3LL * nsm) return 2;
+  return 1;
+}
+
 // The plain FP32 form gives the same ids and statistics either way.  Through
 // the batched kernels (shared-memory dedupe, int8 screen, one synchronisation)
-// 10,000 queries at qProbes 10 on 1M x 200 take 3.08 ms from host buffers
+// 10,000 queries at qProbes 10 on 1M x 200 take 2.82 ms from host buffers
 // against 9.05 ms for the three-kernel path, 1,000 on 100K x 200 0.25 against
-// 0.45 ms, one query 0.13 against 0.35 ms, so it is taken wherever it can be.
+// 0.45 ms, one query 0.07 against 0.35 ms, so it is taken wherever it can be.
 // The budget, 2 GiB, is what the fused kernel's per-block lists may use: they
 // are sized from qProbes times the largest bucket, the three-kernel path's
 // from the candidates that the batch has.
@@ -271,6 +284,14 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     return fail(e, "occupancy");
   if (rq.blocks_per_sm > 0) per_sm = std::min(per_sm, rq.blocks_per_sm);
   per_sm = std::max(per_sm, 1);
+  // a batch that leaves SMs without a query: a cluster of blocks per query
+  int cl = 1;
+  KernelSel kc{nullptr, 0};
+  if (split && !big && kmode != kRowsF32 && !rq.blocks_per_sm) {
+    cl = cluster_size(rq.nq, nsm);
+    if (cl > 1) kc = pick_kernel_cluster(kmode, d);
+    if (!kc.fn) cl = 1;
+  }
   // graph mode keeps one grid for every batch size (idle blocks find no work)
   int grid = std::max(1, rq.use_graph ? nsm * per_sm : std::min(rq.nq, nsm * per_sm));
   const long long nwords = (P.n_points + 31) / 32;
@@ -350,7 +371,13 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     bw.ext_cap = ext_need;
     bw.pc_cap = pc_need;
   }
-  const bool vhash = split && rq.tc_hash && F == 256 && di.tflips && L <= 128 && 2 * rq.qprobes_max <= L;
+  // the verified hash gives a query to one block of two warps, about 45 us (55
+  // at qProbes 10) however few the queries; the exact one a group of 8 lanes to
+  // every (query, table), 12 us per 64 groups an SM.  The exact one is faster up
+  // to four of those waves; that is 378 queries at 100 tables, and 256 leave
+  // the verified hash the batches where it is ahead with fewer tables too
+  const bool vhash = split && rq.tc_hash && F == 256 && di.tflips && L <= 128 && 2 * rq.qprobes_max <= L &&
+                     (rq.nq > 256 || (long long)rq.nq * L > 4LL * 64 * nsm);
   if (split) {
     const long long max_groups = (long long)nsm * 64;
     if (rq.stage_timing) {
@@ -550,7 +577,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     }
     cudaEventRecord(bw.tev[1], s);
   }
-  const bool can_graph = rq.use_graph && !rq.dump_probes && !rq.dump_counts;
+  const bool can_graph = rq.use_graph && !rq.dump_probes && !rq.dump_counts && cl == 1;
   BatchKey key{rq.Q, rq.nq, rq.q_k, rq.q_qprobes, rq.k_uniform, rq.qprobes_uniform, rq.k_max, rq.qprobes_max,
                rq.shortlist_mult, rq.out,
                rq.out_stride, rq.out_v, rq.mode, grid, kern, bw.bitset, a.order, a.tflips, s};
@@ -604,7 +631,20 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
       if ((e = cudaGraphLaunch(bw.graph_exec, s)) != cudaSuccess) return fail(e, "graph launch");
     } else {
       if ((e = cudaMemsetAsync(bw.counters, 0, sizeof(unsigned) * 2, s)) != cudaSuccess) return fail(e, "memset");
-      if ((e = cudaLaunchKernel(kern, dim3(grid), dim3(kBThreads), args, ks.smem, s)) != cudaSuccess)
+      if (cl > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(rq.nq * cl));
+        cfg.blockDim = dim3(kBThreads);
+        cfg.dynamicSmemBytes = kc.smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)cl;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if ((e = cudaLaunchKernelExC(&cfg, kc.fn, args)) != cudaSuccess) return fail(e, "cluster launch");
+      } else if ((e = cudaLaunchKernel(kern, dim3(grid), dim3(kBThreads), args, ks.smem, s)) != cudaSuccess)
         return fail(e, "launch");
     }
   }

@@ -3,6 +3,7 @@
 // (fpp_batch_f32.cu, fpp_batch_bf16.cu, fpp_batch_fp8.cu), which instantiate
 // it for fhtDim 32..512 and d <= 512 and are compiled in parallel.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
@@ -1095,6 +1096,275 @@ __global__ void __launch_bounds__(kBThreads, MODE == kRowsF32 ? 2 : 3) k_batch_q
 }
 
 
+// ---------------------------------------------------------------- small batches
+// k_cluster_query — one query per thread-block cluster, for batches that leave
+// most SMs without a query: at one query the fused kernel's block takes 56 us,
+// most of it the latency of its gather and of its rows through one SM (1M x
+// 200, qProbes 10: 9,600 candidates, 2,300 rows).  The cluster's warps share the
+// candidates, a hash set distributed over the blocks' shared memory (an id's
+// home block and slot come from its hash), and the row tiles; the positions,
+// the overflow flag and the score histogram are rank 0's.  Rank 0 then runs the
+// fused kernel's shortlist and top-k on the same arrays, so the results are the
+// fused kernel's.  Starts from k_probe_cut's output, like kHashExt.
+constexpr int kClusterChain = 48;  // probes of one id before the set counts as full
+
+template <int MODE, int VI32>
+__global__ void __launch_bounds__(kBThreads, 3) k_cluster_query(BatchArgs a) {
+  namespace cg = cooperative_groups;
+  static_assert(MODE != kRowsF32, "the FP32 form comes screened");
+  constexpr int GROUPS = kBThreads / 8;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BatchSmem<GROUPS> sm(smem_raw);
+  __shared__ uint32_t hist[256];
+  __shared__ uint32_t s_pre, s_rem;
+  __shared__ unsigned s_cnt, s_u, s_sel, s_ovf, s_bstar, s_above, s_inbin, s_qmax;
+  __shared__ float s_q2, s_r2;
+  __shared__ long long tmp[32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned CL = cluster.num_blocks();  // a power of two
+  const unsigned rank = cluster.block_rank();
+  const int home_shift = 32 - (31 - __clz((int)CL));  // id hash -> home block (32 when CL is 1: unused)
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  const unsigned gw = rank * kBWarps + warp, nw = CL * kBWarps;  // the warp among the cluster's
+  const unsigned qu = blockIdx.x / CL;
+  const int q = a.order ? (int)a.order[qu] : (int)qu;
+  const int k = a.q_k ? a.q_k[q] : a.k_uniform;
+  const int Qp = a.q_qprobes ? a.q_qprobes[q] : a.qprobes_uniform;
+  if (k < 1 || k > a.k_max || Qp < 1 || Qp > a.qprobes_max) {  // uniform over the cluster
+    if (rank == 0) {
+      if (tid == 0) atomicOr(a.status, 2u);
+      for (int j = tid; j < a.out_stride; j += kBThreads) a.out[(size_t)q * a.out_stride + j] = -1;
+    }
+    return;
+  }
+  uint32_t* bits = a.bitset + (size_t)qu * a.nwords;
+  uint32_t* uq = a.uniq + (size_t)qu * a.cap;
+  uint32_t* sc = a.score + (size_t)qu * a.cap;
+  uint32_t* s_hist = sm.hist();
+  for (int i = tid; i < kHT; i += kBThreads) sm.ht[i] = kEmpty;
+  if (tid == 0) {
+    s_u = 0u;
+    s_ovf = 0u;
+    s_qmax = 0u;
+    s_q2 = 0.0f;
+    s_r2 = 0.0f;
+  }
+  __syncthreads();
+  {
+    const float* qv = a.Q + (size_t)q * a.d;
+    float amax = 0.0f;
+    for (int i = tid; i < 1024; i += kBThreads) {
+      const float x = i < a.d ? qv[i] : 0.0f;
+      sm.q[i] = x;
+      amax = fmaxf(amax, fabsf(x));
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(kFullMask, amax, o));
+    if (lane == 0) atomicMax(&s_qmax, __float_as_uint(amax));
+    // the probes' ranges, in every block
+    const size_t pb = (size_t)q * a.qprobes_max;
+    for (int p = tid; p < Qp; p += kBThreads) {
+      const uint32_t pe = a.pc_pe[pb + p];
+      const uint32_t ex = p ? a.pc_pe[pb + p - 1] : 0u;
+      sm.pe()[p] = pe;
+      sm.po()[p] = a.pc_o[pb + p] - ex;
+      if (a.dump_probes && rank == 0) a.dump_probes[(size_t)q * a.qprobes_max + p] = a.pc_g[pb + p];
+    }
+  }
+  cluster.sync();
+  const uint32_t* s_po = sm.po();
+  const uint32_t* s_pe = sm.pe();
+  const uint32_t C = s_pe[Qp - 1];
+  const unsigned cap = (unsigned)a.cap;
+  unsigned* u0 = cluster.map_shared_rank(&s_u, 0);
+  unsigned* ovf0 = cluster.map_shared_rank(&s_ovf, 0);
+  // ---- gather + dedupe: the cluster's warps take steps of kGStep candidates
+  bool use_bitset = false;
+  for (int pass = 0; pass < 2; ++pass) {
+    int lp = 0;
+    uint32_t lend = s_pe[0], loff = s_po[0];
+    for (uint32_t c0 = gw * kGStep; c0 < C; c0 += nw * kGStep) {
+      uint32_t idv[kGPerLane];
+#pragma unroll
+      for (int h = 0; h < kGPerLane; ++h) {
+        const uint32_t i = c0 + h * 32 + lane;
+        idv[h] = kEmpty;
+        if (i < C) {
+          while (i >= lend) {  // ends when i < C = s_pe[Qp - 1]
+            ++lp;
+            lend = s_pe[lp];
+            loff = s_po[lp];
+          }
+          idv[h] = (uint32_t)__ldg(a.ids + (i + loff));
+        }
+      }
+      bool fresh[kGPerLane];
+      if (use_bitset) {
+#pragma unroll
+        for (int h = 0; h < kGPerLane; ++h) {
+          const uint32_t bit = 1u << (idv[h] & 31u);
+          fresh[h] = idv[h] != kEmpty && (atomicOr(bits + (idv[h] >> 5), bit) & bit) == 0u;
+        }
+      } else {
+        // as in the fused kernel, in rounds; the rounds are bounded, and a
+        // chain that does not end in time starts the query over on the bitset
+        uint32_t* home[kGPerLane];
+        uint32_t slot[kGPerLane], old[kGPerLane];
+#pragma unroll
+        for (int h = 0; h < kGPerLane; ++h) {
+          slot[h] = ht_slot(idv[h]);
+          home[h] = CL == 1 ? sm.ht : cluster.map_shared_rank(sm.ht, (idv[h] * 0x9E3779B1u ^ idv[h] * 0x85EBCA6Bu) >> home_shift);
+          old[h] = idv[h] != kEmpty ? atomicCAS(home[h] + slot[h], kEmpty, idv[h]) : kEmpty;
+        }
+        int chain = 0;
+        for (;;) {
+          bool pend = false;
+#pragma unroll
+          for (int h = 0; h < kGPerLane; ++h) pend |= old[h] != kEmpty && old[h] != idv[h];
+          if (!pend) break;
+          if (++chain > kClusterChain) {
+            *ovf0 = 1u;
+            break;
+          }
+#pragma unroll
+          for (int h = 0; h < kGPerLane; ++h)
+            if (old[h] != kEmpty && old[h] != idv[h]) {
+              slot[h] = (slot[h] + ht_step(idv[h])) & (kHT - 1);
+              old[h] = atomicCAS(home[h] + slot[h], kEmpty, idv[h]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < kGPerLane; ++h) fresh[h] = idv[h] != kEmpty && old[h] == kEmpty;
+      }
+      unsigned bal[kGPerLane];
+      unsigned nfresh = 0;
+#pragma unroll
+      for (int h = 0; h < kGPerLane; ++h) {
+        bal[h] = __ballot_sync(kFullMask, fresh[h]);
+        nfresh += __popc(bal[h]);
+      }
+      if (nfresh) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(u0, nfresh);
+        base = __shfl_sync(kFullMask, base, 0);
+        const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+        for (int h = 0; h < kGPerLane; ++h) {
+          const unsigned pos = base + __popc(bal[h] & below);
+          if (fresh[h] && pos < cap) uq[pos] = idv[h];
+          base += __popc(bal[h]);
+        }
+      }
+    }
+    cluster.sync();
+    const bool over = !use_bitset && *ovf0 != 0u;  // the same in every block
+    if (!over) break;
+    cluster.sync();  // every block has read the flag
+    if (rank == 0 && tid == 0) s_u = 0u;
+    use_bitset = true;
+    cluster.sync();
+  }
+  const unsigned U = *u0;
+  int32_t* orow = a.out + (size_t)q * a.out_stride;
+  float* ovrow = a.out_v ? a.out_v + (size_t)q * a.out_stride : nullptr;
+  if (rank == 0 && tid == 0) {
+    if (a.totals) {
+      atomicAdd(&a.totals->cand, (unsigned long long)C);
+      atomicAdd(&a.totals->unique, (unsigned long long)U);
+    }
+    if (a.dump_counts) {
+      a.dump_counts[2 * (size_t)q] = C;
+      a.dump_counts[2 * (size_t)q + 1] = U;
+    }
+  }
+  // ---- first pass over the unique rows, tile by tile over the cluster's warps
+  const float qmax = __uint_as_float(s_qmax);
+  const float qscale = MODE == kRowsFP8 && qmax > 0.0f ? qmax / 448.0f : 1.0f;
+  ScreenArgs scr;
+  bool screen = MODE != kRowsI8;  // whether the first pass runs
+  if (U <= cap) {
+    if constexpr (MODE == kRowsI8) {
+      if (U > 4u * (unsigned)k) {
+        float2 sums = fill_query_parts_i8(sm.q, qmax, sm.qx);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          sums.x += __shfl_xor_sync(kFullMask, sums.x, o);
+          sums.y += __shfl_xor_sync(kFullMask, sums.y, o);
+        }
+        if (lane == 0 && rank == 0) {  // rank 0's sums: every block decides alike
+          atomicAdd(&s_q2, sums.x);
+          atomicAdd(&s_r2, sums.y);
+        }
+      }
+    } else {
+      fill_query_parts<MODE>(sm.q, qscale, sm.qx);
+    }
+    if (rank == 0)
+      for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
+  }
+  cluster.sync();  // the histogram is clear, every block is done with the ranges and the set
+  if (U <= cap) {
+    if constexpr (MODE == kRowsI8) {
+      const float q2 = *cluster.map_shared_rank(&s_q2, 0), r2 = *cluster.map_shared_rank(&s_r2, 0);
+      scr.qs = __fdiv_rn(__fdiv_rn(qmax, 127.0f), 254.0f);
+      scr.qn = sqrtf(q2) * (1.0f + 0x1p-10f);
+      const float smax = scr.qn * __ldg(a.row_norm_max) * 1.01f;
+      screen = U > 4u * (unsigned)k && r2 <= q2 * (0.95f * kScreenQRel * kScreenQRel) && scr.qn > 1e-18f &&
+               smax < 1e30f;
+      if (screen) scr.base = (int)(ord_key(smax) >> 16) - (kHistBins - 1);
+    }
+    if (screen) {
+      uint32_t* hist0 = cluster.map_shared_rank(s_hist, 0);
+      const bool staged = a.nchunk <= 16 && 9 * 16 * a.row_bytes <= (size_t)(4 * kHT) &&
+                          7 * 16 * a.row_bytes <= BatchSmem<GROUPS>::kQ - BatchSmem<GROUPS>::kProbe;
+      unsigned char* st0 = smem_raw + (size_t)warp * 16 * a.row_bytes;
+      unsigned char* st1 = warp < kBWarps - 1 ? smem_raw + BatchSmem<GROUPS>::kProbe + (size_t)warp * 16 * a.row_bytes
+                                              : smem_raw + (size_t)kBWarps * 16 * a.row_bytes;
+      if (staged)
+        rerank_rows_mma_2stage<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, (int)gw,
+                                     (int)nw, lane, hist0, st0, st1, scr);
+      else
+        rerank_rows_mma<MODE>(uq, U, sc, sm.qx, a.Xrows, a.row_bytes, a.nchunk, a.Xscale, qscale, (int)gw, (int)nw,
+                              lane, hist0, scr);
+    }
+  }
+  cluster.sync();
+  if (rank != 0) return;  // nothing of this block is read from here on
+  if (U > cap) {
+    if (tid == 0) atomicOr(a.status, 1u);
+    for (int j = tid; j < k; j += kBThreads) {
+      orow[j] = -1;
+      if (ovrow) ovrow[j] = 0.0f;
+    }
+    for (long long w = tid; w < a.nwords; w += kBThreads) bits[w] = 0u;
+    return;
+  }
+  // ---- shortlist, exact re-score and top-k in rank 0
+  const FinishShared fs{hist, &s_pre, &s_rem, &s_cnt, &s_sel, &s_bstar, &s_above, &s_inbin, tmp};
+  bool bits_dirty = use_bitset;
+  if constexpr (MODE == kRowsI8) {
+    bool done = false;
+    if (screen)
+      done = finish_screened<VI32, GROUPS>(a, sm, sm.top, uq, sc, U, k, scr.base, orow, ovrow, fs, tid, warp, lane);
+    if (!done) {
+      for (int i = tid; i < kHistBins; i += kBThreads) s_hist[i] = 0u;
+      __syncthreads();
+      rerank_rows<kRowsF32, VI32, 1>(uq, U, sc, sm.q, reinterpret_cast<const unsigned char*>(a.Xc), (size_t)a.ld * 4,
+                                     a.ld / 4, nullptr, warp, kBWarps, lane, s_hist);
+      __syncthreads();
+      bits_dirty = finish_query<kRowsF32, VI32, GROUPS>(a, sm, sm.top, uq, sc, U, k, orow, ovrow, use_bitset, bits, fs,
+                                                        tid, warp, lane);
+    }
+  } else {
+    bits_dirty = finish_query<MODE, VI32, GROUPS>(a, sm, sm.top, uq, sc, U, k, orow, ovrow, use_bitset, bits, fs, tid,
+                                                  warp, lane);
+  }
+  if (bits_dirty)
+    for (unsigned i = tid; i < U; i += kBThreads) bits[uq[i] >> 5] = 0u;
+}
+
 struct KernelSel {
   const void* fn;
   size_t smem;
@@ -1127,6 +1397,7 @@ KernelSel pick_kernel_bf16(int fht, int d, bool tc_only);
 KernelSel pick_kernel_fp8(int fht, int d, bool tc_only);
 KernelSel pick_kernel_big(int fht, int mode, int d);  // fpp_batch_big.cu
 KernelSel pick_kernel_ext(int mode, int d, bool big);  // fpp_batch_ext.cu
+KernelSel pick_kernel_cluster(int mode, int d);        // fpp_batch_cluster.cu
 
 inline int vi_of(int d, int epc) {
   const int v = ((d + epc - 1) / epc + 31) / 32;

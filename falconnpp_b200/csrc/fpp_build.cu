@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128, KEEP == 3 ? 5 : 4) k_build_hash(HashArgs 
               ye[2 * j + 1] = f2_hi(y[j]);
             }
             const bool ok = group_top1_strict<FHT>(ye, gl, a.D, a.log2D, lv, lc);
-            if (__all_sync(kFullMask, ok)) {
+            if (__all_sync(kFullMask, ok || !active)) {
               __syncwarp();
               continue;
             }
@@ -314,7 +314,8 @@ __global__ void __launch_bounds__(128, KEEP == 3 ? 5 : 4) k_build_hash(HashArgs 
           constexpr int C = KEEP == 1 ? 2 : 4;
           uint32_t k[C];
           auto bits = [&](int e) { return (uint32_t)(y[e / 2] >> (32 * (e & 1))); };
-          const bool fast = __all_sync(kFullMask, group_top_keys<FHT, C>(bits, gl, a.D, cnt, k));
+          // (a group without a point has ties only)
+          const bool fast = __all_sync(kFullMask, group_top_keys<FHT, C>(bits, gl, a.D, cnt, k) || !active);
           LaneVector<FHT>::store(yv, y, gl);
           __syncwarp();
           if (fast) {
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(128, KEEP == 3 ? 5 : 4) k_build_hash(HashArgs 
                 lc[t] = cp_code(x, pos, a.log2D);
               }
             }
-          } else if (!group_top_stored<FHT>(yv, gl, a.D, a.log2D, cnt, lv, lc) && gl == 0) {
+          } else if (!group_top_stored<FHT>(yv, gl, a.D, a.log2D, cnt, lv, lc) && gl == 0 && active) {
             // the reference's scan, FalconnPP.cpp:103-156
             int n = 0;
             for (int r = 0; r < a.D; ++r) {
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(128, KEEP == 3 ? 5 : 4) k_build_hash(HashArgs 
           }
           hd3_rotate<FHT>(y, flips, gl);
           const bool ok = group_top_cp_checked<FHT>(y, gl, a.D, a.log2D, P, cnt, lv, lc);
-          if (!ok) {  // group-uniform: replay the reference's heap scan
+          if (!ok && active) {  // group-uniform: replay the reference's heap scan
 #pragma unroll
             for (int e = 0; e < E; ++e) yv[gl * E + e] = y[e];
             __syncwarp(gmask);

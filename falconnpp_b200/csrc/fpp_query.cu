@@ -127,7 +127,9 @@ __global__ void __launch_bounds__(128, 4) k_query_hash(QHashArgs a, float* heap_
       int* lc = layer == 0 ? lc1 : lc2;
       if constexpr (C > 2) {
         uint32_t k[C];
-        if (__all_sync(kFullMask, group_top_keys<FHT, C>([&](int e) { return __float_as_uint(y[e]); }, gl, a.D, cnt, k))) {
+        const bool ok =
+            group_top_keys<FHT, C>([&](int e) { return __float_as_uint(y[e]); }, gl, a.D, cnt, k) || !active;
+        if (__all_sync(kFullMask, ok)) {
           LaneVector<FHT>::store(ydump, y, gl);
           __syncwarp();
           if (gl == 0) {
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(128, 4) k_query_hash(QHashArgs a, float* heap_
         }
       }
       const bool ok = group_top_cp_checked<FHT>(y, gl, a.D, a.log2D, m1w, cnt, lv, lc);
-      if (!ok) {
+      if (!ok && active) {  // (a group without an item has ties only)
 #pragma unroll
         for (int e = 0; e < E; ++e) ydump[gl * E + e] = y[e];
         __syncwarp(gmask);

@@ -50,6 +50,41 @@ def test_isotropic_data_and_big_lists():
     _check(X, Q, 12, 64, 20, 1500)
 
 
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("nq", [1, 18, 19, 37, 38, 222, 223])
+def test_small_batches(nq, precision):
+    """Clusters of 8, 4, 2 blocks per query and none: the results of the same
+    queries inside a large batch."""
+    import torch
+    X = synth.mixture(30000, 200, n_centres=16, seed=0)
+    Q = synth.mixture(600, 200, n_centres=16, seed=1)
+    g = capi.Index(*X.shape)
+    g.set_index_param(12, 64, 400, 0.05, 2, 8, 42)
+    g.build(X)
+    g.set_query_form(1, precision, 2)
+    dq = torch.from_numpy(Q).cuda()
+    # qProbes 1: few candidates; 6; 300: more unique ids than a set's chains take
+    for k, qp in ((1, 1), (20, 6), (50, 300)):
+        got, val = [], []
+        for n in (600, nq):
+            ids = torch.full((n, k), -7, dtype=torch.int32, device="cuda")
+            v = torch.zeros((n, k), dtype=torch.float32, device="cuda")
+            g.query_batched(dq.data_ptr(), n, None, None, k, qp, ids.data_ptr(), k, v.data_ptr())
+            got.append(ids.cpu().numpy()[:nq])
+            val.append(v.cpu().numpy()[:nq])
+        assert np.array_equal(got[0], got[1]), (k, qp)
+        assert np.array_equal(val[0].view(np.uint32), val[1].view(np.uint32)), (k, qp)
+    if precision == 0:
+        g.set_qprobes(6)
+        assert np.array_equal(g.query_dump(Q[:nq], 20, 6)["topk"], got_plain(g, Q[:nq]))
+    g.close()
+
+
+def got_plain(g, Q):
+    g.set_query_form(0, 0, 4)
+    return g.query(Q, 20)
+
+
 def test_data_that_defeats_the_screen():
     X = synth.p0_integer(6000, 32, xmax=3)
     _check(X, synth.p0_queries(40, 32, qmax=2), 8, 32, 10, 40)

@@ -336,6 +336,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     }
     if ((e = cudaMemsetAsync(bw.bitset, 0, sizeof(uint32_t) * (size_t)grid * nwords, s)) != cudaSuccess)
       return fail(e, "memset");
+    if ((e = cudaMemsetAsync(bw.counters, 0, sizeof(BatchCounters), s)) != cudaSuccess) return fail(e, "memset");
     bw.hheap_cap = heap_cap;
     bw.list_cap = list_cap;
     bw.probe_cap = probe_cap;
@@ -347,13 +348,24 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   }
   grid = std::min(grid, bw.grid);
   const long long ext_stride = (long long)L * std::max(mmax, 1);
+  // The verified hash: its GEMM and its check take about 40 us however few the
+  // queries; the exact one gives a group of 8 lanes to every (query, table), 12
+  // us per 64 groups an SM.  The exact one is faster up to four of those waves;
+  // that is 378 queries at 100 tables, and 256 leave the verified hash the
+  // batches where it is ahead with fewer tables too.
+  const bool vhash = split && rq.tc_hash && (di.hmat || (F == 256 && di.tflips)) && L <= 128 &&
+                     2 * rq.qprobes_max <= L && (rq.nq > 256 || (long long)rq.nq * L > 4LL * 64 * nsm);
+  // scratch of its GEMM, for up to 32,768 queries at a time (66 MB at 100 tables of 256)
+  const long long hash_nq = vhash && di.hmat ? std::min<long long>(rq.nq, 32768) : 0;
+  const long long hash_need = hash_nq * 2 * L * (D / 128), hq_need = hash_nq * hmat_ld(d);
   // per-batch buffers: lists of the hash, processing order, probe cuts
   const bool pcut = split && !big;
   const long long ext_need = split ? (long long)rq.nq * ext_stride : 0;
   const long long pc_need = pcut ? (long long)rq.nq * rq.qprobes_max : 0;
-  if (!bw.bslab || bw.batch_cap < rq.nq || bw.ext_cap < ext_need || bw.pc_cap < pc_need) {
+  if (!bw.bslab || bw.batch_cap < rq.nq || bw.ext_cap < ext_need || bw.pc_cap < pc_need || bw.hash_cap < hash_need ||
+      bw.hq_cap < hq_need) {
     cudaFree(bw.bslab);
-    bw.batch_cap = bw.ext_cap = bw.pc_cap = 0;
+    bw.batch_cap = bw.ext_cap = bw.pc_cap = bw.hash_cap = bw.hq_cap = 0;
     Slab slab;
     slab.reserve(&bw.okey, (size_t)rq.nq);
     slab.reserve(&bw.order, (size_t)rq.nq);
@@ -364,20 +376,19 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     slab.reserve(&bw.pc_o, (size_t)pc_need);
     slab.reserve(&bw.pc_pe, (size_t)pc_need);
     slab.reserve(&bw.pc_n, (size_t)rq.nq);
+    if (hash_need) {
+      slab.reserve(&bw.hq, (size_t)hq_need);
+      slab.reserve(&bw.htmax, (size_t)hash_need);
+    }
     if ((e = slab.alloc(&bw.bslab)) != cudaSuccess) return fail(e, "alloc");
     if ((e = cudaMemsetAsync(bw.ohist, 0, sizeof(uint32_t) * kOrderMaxBins, s)) != cudaSuccess)
       return fail(e, "memset");
     bw.batch_cap = rq.nq;
     bw.ext_cap = ext_need;
     bw.pc_cap = pc_need;
+    bw.hash_cap = hash_need;
+    bw.hq_cap = hq_need;
   }
-  // the verified hash gives a query to one block of two warps, about 45 us (55
-  // at qProbes 10) however few the queries; the exact one a group of 8 lanes to
-  // every (query, table), 12 us per 64 groups an SM.  The exact one is faster up
-  // to four of those waves; that is 378 queries at 100 tables, and 256 leave
-  // the verified hash the batches where it is ahead with fewer tables too
-  const bool vhash = split && rq.tc_hash && F == 256 && di.tflips && L <= 128 && 2 * rq.qprobes_max <= L &&
-                     (rq.nq > 256 || (long long)rq.nq * L > 4LL * 64 * nsm);
   if (split) {
     const long long max_groups = (long long)nsm * 64;
     if (rq.stage_timing) {
@@ -390,15 +401,21 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     // host queries: up to four chunks copied on the copy stream, each hashed
     // as soon as it lands.  The hash launches of one stream run one after
     // the other, so a chunk that is not a whole number of waves of hash
-    // blocks leaves SMs idle at its end: with the verified hash the first
-    // chunks are one full wave each and the last takes the rest (the same
-    // number of waves as one launch over the batch); otherwise quarters.
+    // blocks leaves SMs idle at its end: with the verified hash of one block
+    // per query the first chunks are one full wave each and the last takes the
+    // rest (the same number of waves as one launch over the batch); with the
+    // matrices a small first chunk starts the pipeline and a modest last one
+    // ends it; otherwise quarters.
     long long cut[5] = {0, 0, 0, 0, 0};
     int nch = (rq.Q_host && rq.copy_stream && rq.copy_stream != s && rq.nq >= 4096) ? 4 : 1;
     if (nch > 1) {
-      const long long wq = vhash ? hash_verified_wave_queries() : 0;
+      const long long wq = vhash && !di.hmat ? hash_verified_wave_queries() : 0;
       if (wq > 0) nch = (int)std::min<long long>(4, rq.nq / wq);
-      for (int c = 0; c <= nch; ++c) cut[c] = wq > 0 ? (c < nch ? c * wq : rq.nq) : (long long)rq.nq * c / nch;
+      const int part[5] = {0, 12, 40, 70, 100};
+      for (int c = 0; c <= nch; ++c)
+        cut[c] = wq > 0              ? (c < nch ? c * wq : rq.nq)
+                 : vhash && di.hmat  ? (long long)rq.nq * part[c] / 100
+                                     : (long long)rq.nq * c / nch;
     }
     if (nch <= 1) {
       nch = 1;
@@ -432,7 +449,8 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
       const int* qq = rq.q_qprobes ? rq.q_qprobes + q0 : nullptr;
       e = vhash ? hash_lists_verified(P, di, rq.Q + q0 * d, (int)(q1 - q0), qq, rq.qprobes_max,
                                       bw.ext_lv + q0 * ext_stride, bw.ext_lb + q0 * ext_stride, ext_stride,
-                                      rq.stage_timing ? &bw.counters->tc_exact : nullptr, s)
+                                      rq.stage_timing ? &bw.counters->tc_exact : nullptr,
+                                      HashScratch{bw.hq, bw.htmax, &bw.counters->pipe, hash_nq}, s)
                 : hash_lists(P, di, rq.Q + q0 * d, (int)(q1 - q0), qq, rq.qprobes_max, bw.ext_lv + q0 * ext_stride,
                              bw.ext_lb + q0 * ext_stride, ext_stride, bw.hheap_v, bw.hheap_i, max_groups, s);
       if (e != cudaSuccess) return fail(e, "hash kernel");
@@ -672,6 +690,12 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     if ((e = cudaMemcpyAsync(&hc, bw.counters, sizeof(hc), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
       return fail(e, "status");
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return fail(e, "batch kernel");
+    if (hc.pipe) {
+      cudaMemsetAsync(&bw.counters->pipe, 0, sizeof(unsigned), s);
+      err.code = kErrDevice;
+      err.msg = "batch query: a block of the hash gave up waiting on its pipeline";
+      return err.code;
+    }
     res.overflow = (hc.status & 1u) != 0;
     res.bad_params = (hc.status & 2u) != 0;
     if (totals) res.totals = hc.totals;

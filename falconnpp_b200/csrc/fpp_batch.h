@@ -52,9 +52,9 @@ struct BatchTotals {
 };
 
 // Device words of a batch: the first four 32-bit words (work counter, status,
-// re-hashed tables, unused), then the totals.
+// re-hashed tables, status of the hash's tensor-core pipeline), then the totals.
 struct BatchCounters {
-  unsigned work, status, tc_exact, pad;
+  unsigned work, status, tc_exact, pipe;
   BatchTotals totals;
 };
 
@@ -130,6 +130,10 @@ struct BatchWorkspace {
   float* ext_lv = nullptr;
   uint32_t* ext_lb = nullptr;
   long long batch_cap = 0, ext_cap = 0, pc_cap = 0;  // queries, list and probe entries that bslab holds
+  // verified hash with the rotations as matrices: FP16 queries, magnitudes
+  uint16_t* hq = nullptr;
+  float* htmax = nullptr;
+  long long hash_cap = 0, hq_cap = 0;
   float* hheap_v = nullptr;
   int* hheap_i = nullptr;
   long long hheap_cap = 0;

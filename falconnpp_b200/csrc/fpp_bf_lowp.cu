@@ -148,7 +148,7 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
 // kind::f16 (BF16 x BF16) or kind::f8f6f4 (E4M3 x E4M3), FP32 accumulator,
 // both operands K-major, M = N = 128.
 template <int MODE>
-__host__ __device__ constexpr uint32_t umma_idesc() {
+__host__ __device__ constexpr uint32_t umma_idesc() {  // (kind::f16 with type bits 0: FP16 x FP16)
   return (1u << 4) | (MODE == kRowsBF16 ? ((1u << 7) | (1u << 10)) : 0u) | ((uint32_t)(kTile >> 3) << 17) |
          ((uint32_t)(kTile >> 4) << 24);
 }
@@ -520,7 +520,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 // MODE kScanBound: BF16 rows with a bound of their error (row_err, times the
 // query's norm): the sample pass takes lower bounds of the exact score and the
 // collect pass compares upper bounds.
+//
+// MODE kScanHash: FP16 rows, the sample pass alone over every row tile, with
+// magnitudes: tmax gets the largest |score| of each tile (launch_hash_scan).
 constexpr int kScanBound = 4;
+constexpr int kScanHash = 5;
 constexpr int kScanThreads = 352;                 // producer, 2 issuers, 2 x 4 epilogue warps
 constexpr int kScanHalves = 2;
 constexpr int kScanTileQ = kScanHalves * kTile;  // queries per CTA
@@ -602,7 +606,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 template <int MODE>
 __device__ __forceinline__ void umma_elect(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumulate) {
   const uint32_t idesc = umma_idesc<MODE>();
-  if constexpr (MODE == kRowsBF16) {
+  if constexpr (MODE != kRowsFP8) {
     asm volatile(
         "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n elect.sync _|e, 0xffffffff;\n"
         " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n"
@@ -650,9 +654,10 @@ __device__ __forceinline__ float scan_value(float v, float row, float f) {
 template <int MODE, bool COLLECT>
 __global__ void __launch_bounds__(kScanThreads, 1)
     k_bf_scan(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap xmap, ScanTileArgs a) {
-  constexpr int kRow = MODE == kRowsFP8 ? kRowsFP8 : kRowsBF16;
-  constexpr bool kScaled = MODE != kRowsBF16;
-  using C = BfCfg<kRow>;
+  // the MMAs' operand type (kScanHash: FP16, the 2-byte layout of BF16)
+  constexpr int kRow = MODE == kRowsFP8 ? kRowsFP8 : MODE == kScanHash ? kScanHash : kRowsBF16;
+  constexpr bool kScaled = MODE == kRowsFP8 || MODE == kScanBound;
+  using C = BfCfg<MODE == kRowsFP8 ? kRowsFP8 : kRowsBF16>;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* q_smem = base;  // [half][box]
@@ -863,6 +868,10 @@ __global__ void __launch_bounds__(kScanThreads, 1)
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj)
             if (c * 32 + jj >= nvalid) v[jj] = -INFINITY;
+        }
+        if (MODE == kScanHash) {
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) v[jj] = fabsf(v[jj]);
         }
         float m4[4];
 #pragma unroll
@@ -1451,6 +1460,38 @@ extern "C" int fpp_bruteforce_topk_lowp(fpp_index* h, const float* d_queries, in
   if (st) return set_last_error(FPP_ERR_DEVICE, "bruteforce_lowp: a block gave up waiting on its pipeline");
   return clear_last_error();
 }
+
+// ---------------------------------------------------------------- query hash
+namespace fpp {
+
+cudaError_t launch_hash_scan(const void* qrows, int nq, const void* matrix, int rows, int d, int ld, float* tmax,
+                             unsigned* status, int nsm, cudaStream_t s) {
+  CUtensorMap qmap, xmap;
+  const int inner = (d + 7) & ~7;
+  if (!make_map(&qmap, qrows, nq, inner, ld * 2, 2) || !make_map(&xmap, matrix, rows, inner, ld * 2, 2))
+    return cudaErrorInvalidValue;
+  ScanTileArgs a = {};
+  a.n = rows;
+  a.nq = nq;
+  a.kbytes = ((d * 2 + 31) / 32) * 32;
+  a.boxes = (a.kbytes + kBoxBytes - 1) / kBoxBytes;
+  a.stages = std::min(kScanMaxStages, 13 - kScanHalves * a.boxes);
+  a.tmax = tmax;
+  a.status = status;
+  a.xstride = 1;
+  a.row_tiles = rows / kTile;
+  a.qtiles = (nq + kScanTileQ - 1) / kScanTileQ;
+  a.block_tiles = a.row_tiles;  // the matrix stays in L2
+  const size_t smem = 1024 + (size_t)(kScanHalves * a.boxes + a.stages) * kBoxTileBytes;
+  const void* kern = (const void*)&k_bf_scan<kScanHash, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&qmap, &xmap, &a};
+  return cudaLaunchKernel(kern, dim3((unsigned)std::min<long long>(nsm, (long long)a.row_tiles * a.qtiles)),
+                          dim3(kScanThreads), args, smem, s);
+}
+
+}  // namespace fpp
 
 // ---------------------------------------------------------------- FP64 ground truth
 namespace fpp {

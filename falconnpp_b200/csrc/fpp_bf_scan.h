@@ -7,6 +7,13 @@
 
 namespace fpp {
 
+// The largest |q . row| of every 128 rows of a matrix of `rows` (a multiple of
+// 128) FP16 rows of d elements, zeros up to `ld` (a multiple of 8, at most 256),
+// for nq FP16 queries of the same layout: tmax[q][rows / 128], FP32 accumulation.  status
+// bit 0 is raised if a CTA gave up waiting.  Asynchronous.
+cudaError_t launch_hash_scan(const void* qrows, int nq, const void* matrix, int rows, int d, int ld, float* tmax,
+                             unsigned* status, int nsm, cudaStream_t s);
+
 // Subtracted from a threshold: more than the absolute error that products and
 // sums below FP32's normal range can add (norms are at most 1e15).
 constexpr float kTruthSlack = 1e-34f;

@@ -19,6 +19,7 @@
 //      (score desc, id asc) — ties at the iLimit cut, and (by default) ties
 //      inside the kept prefix — k_repair replays the reference's max-heap on
 //      that bucket's entries and rewrites its ids in the reference's order.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -179,7 +180,7 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
   const size_t nb = (size_t)P.n_tables * 4 * P.n_proj * P.n_proj;
   di.ld = (P.n_features + 3) & ~3;
   cudaError_t e = cudaSuccess;
-  for (bool i8 = d <= 512;; i8 = false) {
+  for (bool extra = true;; extra = false) {
     Slab slab;
     slab.reserve(&di.Xc, n * di.ld);
     slab.reserve(&di.center, d);
@@ -188,17 +189,68 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
     slab.reserve(&di.bucket_off, nb + 1);
     di.Xi8 = nullptr;
     di.i8_norm_max = nullptr;
-    if (i8) {
+    di.hmat = nullptr;
+    di.hmat_err = nullptr;
+    if (extra && d <= 512) {
       slab.reserve(&di.Xi8, n * i8_row_bytes(P.n_features));
       slab.reserve(&di.i8_norm_max, 1);
     }
+    if (extra && hmat_fits(P)) {
+      slab.reserve(&di.hmat, (size_t)2 * P.n_tables * P.n_proj * hmat_ld(P.n_features));
+      slab.reserve(&di.hmat_err, 1);
+    }
     e = slab.alloc(&di.slab);
-    if (e == cudaSuccess || !i8) break;
+    if (e == cudaSuccess || !extra) break;
     cudaGetLastError();
     size_t have = 0, all = 0;
     if (cudaMemGetInfo(&have, &all) != cudaSuccess || have >= slab.bytes()) break;  // not for want of room
   }
   return e;
+}
+
+// One group of FHT / 32 lanes per (table, layer, basis vector): the vector's
+// rotation, exact in FP32 (integers), is a column of the layer's matrix.
+template <int FHT>
+__global__ void __launch_bounds__(128) k_hash_matrix(const uint32_t* __restrict__ flips, int L, int D, int d, int ld,
+                                                     uint16_t* __restrict__ out, float* __restrict__ err) {
+  constexpr int G = Geo<FHT>::G;
+  const int gl = threadIdx.x & (G - 1);
+  const long long item = (long long)blockIdx.x * (128 / G) + threadIdx.x / G;
+  const bool act = item < (long long)2 * L * d;
+  const int v = act ? (int)(item / d) : 0;  // 2 l + layer
+  const int j = act ? (int)(item - (long long)v * d) : 0;
+  f2 y[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    y[i] = f2_make(gl * 32 + 2 * i == j ? 1.0f : 0.0f, gl * 32 + 2 * i + 1 == j ? 1.0f : 0.0f);
+  hd3_rotate_pairs<FHT>(y, flips + ((size_t)((v & 1) * L + (v >> 1)) * 3) * Geo<FHT>::WORDS, gl);
+  float worst = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    const float x = i & 1 ? f2_hi(y[i / 2]) : f2_lo(y[i / 2]);
+    const int r = gl * 32 + i;
+    const __half h = __float2half_rn(x);
+    if (act && r < D) {
+      out[((size_t)v * D + r) * ld + j] = __half_as_ushort(h);
+      worst = fmaxf(worst, fabsf(x - __half2float(h)));
+    }
+  }
+  worst = __uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(worst)));
+  if ((threadIdx.x & 31) == 0 && worst > 0.0f) atomicMax(reinterpret_cast<unsigned*>(err), __float_as_uint(worst));
+}
+
+cudaError_t make_hash_matrix(const Params& P, DeviceIndex& di, cudaStream_t s) {
+  if (!di.hmat) return cudaSuccess;
+  const int L = P.n_tables, D = P.n_proj, d = P.n_features, ld = hmat_ld(d);
+  cudaError_t e = cudaMemsetAsync(di.hmat, 0, sizeof(uint16_t) * (size_t)2 * L * D * ld, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(di.hmat_err, 0, sizeof(float), s);
+  if (e != cudaSuccess) return e;
+  const long long items = (long long)2 * L * d, per = 128 / (P.fhtDim / 32);
+  const unsigned grid = (unsigned)((items + per - 1) / per);
+  if (P.fhtDim == 128) k_hash_matrix<128><<<grid, 128, 0, s>>>(di.flips, L, D, d, ld, di.hmat, di.hmat_err);
+  if (P.fhtDim == 256) k_hash_matrix<256><<<grid, 128, 0, s>>>(di.flips, L, D, d, ld, di.hmat, di.hmat_err);
+  if (P.fhtDim == 512) k_hash_matrix<512><<<grid, 128, 0, s>>>(di.flips, L, D, d, ld, di.hmat, di.hmat_err);
+  return cudaGetLastError();
 }
 
 void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
@@ -1206,6 +1258,7 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
 
   // 2. random signs -> flip words [2][L][3][WORDS]
   if (upload_flips(P, bits, di, s, err) != kOk) goto fail;
+  FPP_CUDA(make_hash_matrix(P, di, s));
 
   // 3. hash + sort + compact, a chunk of tables at a time
   FPP_CUDA(cudaMemsetAsync(deferred, 0, sizeof(unsigned) * 4, s));

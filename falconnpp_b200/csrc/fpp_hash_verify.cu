@@ -1,7 +1,9 @@
 // fpp_hash_verify.cu — the query hash of the batched form with the rotation
 // on the tensor cores and the reference's FP32 arithmetic wherever it can
-// decide a probe (k_query_hash_verified).  fhtDim 256, one probe per table
-// (2 qProbes <= L).
+// decide a probe; one probe per table (2 qProbes <= L).  Two forms: the
+// rotations as matrices (the second half of this file), wherever the index
+// holds them (DeviceIndex::hmat), and k_query_hash_verified, for fhtDim 256
+// with n_proj < 128 or an index without room for the matrices:
 //
 // One block of two warps per query (the warps split the tables, and block
 // barriers join them; half-query work units keep the last wave short):
@@ -48,6 +50,7 @@
 
 #include <algorithm>
 
+#include "fpp_bf_scan.h"
 #include "fpp_device.cuh"
 #include "fpp_query.h"
 #include "fpp_tc_rotate.cuh"
@@ -284,6 +287,247 @@ __global__ void __launch_bounds__(kVThreads, 8) k_query_hash_verified(VerifyArgs
   }
 }
 
+// ---------------------------------------------------------------- rotations as one product
+// The same verification from the rotations as dense matrices: HD3 is linear, so
+// the 2 L n_proj coordinates of a query are one matrix-vector product, and a
+// batch's are a GEMM of K = d on the tcgen05 tensor cores (k_bf_scan, mode
+// kScanHash), whose epilogue keeps only each layer's largest magnitude.  The
+// weights are integers of standard deviation FHT (exact in FP16 up to 2,048),
+// so the error is nearly the query's own rounding alone, and the tables that
+// have to be hashed in FP32 are little more than the probed ones: 3 of 100 at
+// qProbes 2 and 11.5 at 10, against 10 and 35 of the three-round rotation,
+// which rounds to FP16 six times.
+//   1. k_hash_rows: the queries as FP16, scaled by a power of two to a norm in
+//      [128, 256) (values below FP16's normal range, taken as lost, are then
+//      nothing beside the rest);
+//   2. the GEMM: largest magnitude of every 128 coordinates;
+//   3. k_hash_check: per query, s~ = v1~ + v2~ of every table, the qProbes-th
+//      largest, and the FP32 hash of every table within 2 delta of it (and of
+//      table 0, whose bucket orders the batch); the tie rule as above.
+// The bound, per layer and relative to ||x||: ||M_r|| (e_x + 2^-13 + 2^-18) +
+// e_M, with ||M_r|| <= FHT^1.5, e_x the query's actual rounding error, 2^-13
+// the accumulation (at most 17 truncations of 2^-23 of the sum of magnitudes in
+// each of the 16 steps of 16 products), 2^-18 the exact path's own rounding and
+// e_M = sqrt(d) times the largest error of a weight.  delta per table = 2
+// layers x 1.05 x that.
+// 10,000 queries, 100 tables of 256 coordinates, d 200, qProbes 2 / 10 / 40:
+// 291 / 352 / 575 us (k_query_hash_verified: 567 / 750 / 1,130), of which the
+// rows take 9 and the product 200 (its MMAs alone 95).
+
+// Scale of a query of norm n: 2^e with n 2^e in [128, 256).
+__device__ __forceinline__ float hash_scale(float nrm) {
+  int ex = 0;
+  frexpf(nrm, &ex);  // nrm in [2^(ex-1), 2^ex)
+  return __int_as_float((127 + 8 - ex) << 23);
+}
+__device__ __forceinline__ bool hash_norm_ok(float nrm) { return nrm > 0x1p-60f && nrm < 0x1p60f; }
+
+// The norm as both kernels compute it (one warp, the same order).
+__device__ __forceinline__ float warp_norm(const float* x, int d, int lane) {
+  float ss = 0.0f;
+  for (int i = lane; i < d; i += 32) {
+    const float v = __ldg(x + i);
+    ss = fmaf(v, v, ss);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(kFullMask, ss, o);
+  return sqrtf(ss);
+}
+
+__global__ void __launch_bounds__(256) k_hash_rows(const float* __restrict__ Q, int nq, int d, int ld,
+                                                   __half* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (q >= nq) return;
+  const float* x = Q + (size_t)q * d;
+  const float nrm = warp_norm(x, d, lane);
+  const float s = hash_norm_ok(nrm) ? hash_scale(nrm) : 0.0f;  // such a query is hashed exactly
+  for (int i = lane; i < ld; i += 32)
+    out[(size_t)q * ld + i] = __float2half_rn(i < d && s > 0.0f ? __ldg(x + i) * s : 0.0f);
+}
+
+struct CheckArgs {
+  VerifyArgs v;
+  const float* tmax;  // [nq][2 L parts], parts = D / 128 maxima per layer
+  int parts;
+  const float* merr;  // the largest rounding error of a weight
+};
+
+constexpr int kCheckWarps = 4;  // per block
+
+template <int FHT>
+struct __align__(16) CheckSmem {
+  static constexpr int GROUPS = 32 / Geo<FHT>::G;
+  float x[LaneVector<FHT>::kFloats];
+  float sv[kVMaxL];
+  uint32_t sb[kVMaxL];
+  int rl[kVMaxL];
+  float ydump[GROUPS][FHT];
+  float lv[GROUPS][2];
+  int lc[GROUPS][2];
+  float hv[GROUPS];
+  int hi[GROUPS];
+};
+
+// exact_tables for any FHT, with pairs, by one warp.
+template <int FHT>
+__device__ __forceinline__ void check_tables(const VerifyArgs& a, CheckSmem<FHT>& sm, int lane,
+                                             const uint32_t (&mask)[4]) {
+  constexpr int G = Geo<FHT>::G;
+  constexpr int PER_WARP = 32 / G;
+  int base = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if ((mask[j] >> lane) & 1u) sm.rl[base + __popc(mask[j] & ((1u << lane) - 1u))] = lane + 32 * j;
+    base += __popc(mask[j]);
+  }
+  __syncwarp();
+  const int nr = base;
+  const int gl = lane & (G - 1);
+  const int grp = lane / G;
+  const unsigned gmask = G == 32 ? kFullMask : (((1u << G) - 1u) << (lane & ~(G - 1)));
+  for (int r0 = 0; r0 < nr; r0 += PER_WARP) {
+    const int r = r0 + grp;
+    const bool act = r < nr;
+    const int l = sm.rl[act ? r : r0];
+#pragma unroll 1
+    for (int layer = 0; layer < 2; ++layer) {
+      f2 y[16];
+      LaneVector<FHT>::load(sm.x, y, gl);
+      hd3_rotate_pairs<FHT>(y, a.flips + ((size_t)(layer * a.L + l) * 3) * Geo<FHT>::WORDS, gl);
+      float ye[32];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        ye[2 * j] = f2_lo(y[j]);
+        ye[2 * j + 1] = f2_hi(y[j]);
+      }
+      float* ov = &sm.lv[grp][layer];
+      int* oc = &sm.lc[grp][layer];
+      const bool ok = group_top1_strict<FHT>(ye, gl, a.D, a.log2D, ov, oc);
+      __syncwarp();
+      if (!ok) {
+        // a tie for the best coordinate: the reference's scan
+        float* yd = sm.ydump[grp];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) yd[gl * 32 + e] = ye[e];
+        __syncwarp(gmask);
+        if (gl == 0) replay_layer_topp(yd, a.D, a.log2D, 1, &sm.hv[grp], &sm.hi[grp], ov, oc);
+        __syncwarp(gmask);
+      }
+    }
+    __syncwarp();
+    if (gl == 0 && act) {
+      sm.sv[l] = __fadd_rn(sm.lv[grp][0], sm.lv[grp][1]);
+      sm.sb[l] = (uint32_t)l * a.NB + (uint32_t)(sm.lc[grp][0] * 2 * a.D + sm.lc[grp][1]);
+    }
+    __syncwarp();
+  }
+}
+
+// One warp per query: about three tables are hashed again at qProbes 2, and the
+// rest is reductions of a warp (a block of two warps per query, one of them
+// mostly waiting: 136 us for 10,000 queries; this: 80).
+template <int FHT>
+__global__ void __launch_bounds__(32 * kCheckWarps, 16 / kCheckWarps) k_hash_check(CheckArgs c) {
+  const VerifyArgs& a = c.v;
+  __shared__ __align__(16) CheckSmem<FHT> sm_all[kCheckWarps];
+  const int lane = threadIdx.x & 31;
+  const int q = blockIdx.x * kCheckWarps + (threadIdx.x >> 5);
+  if (q >= a.nq) return;  // warps work alone
+  CheckSmem<FHT>& sm = sm_all[threadIdx.x >> 5];
+  const int L = a.L;
+  const float* x = a.Q + (size_t)q * a.d;
+  for (int i = lane; i < FHT; i += 32) LaneVector<FHT>::at(sm.x, i) = i < a.d ? __ldg(x + i) : 0.0f;
+  const float nrm = warp_norm(x, a.d, lane);
+  bool all = !hash_norm_ok(nrm);
+  uint32_t valid[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int lo = 32 * j;
+    valid[j] = L - lo >= 32 ? kFullMask : (L - lo <= 0 ? 0u : (1u << (L - lo)) - 1u);
+  }
+  const int qp = min(max(a.q_qprobes ? __ldg(a.q_qprobes + q) : a.qp_max, 1), a.qp_max);
+  uint32_t first[4] = {valid[0], valid[1], valid[2], valid[3]};
+  if (!all) {
+    const float scale = hash_scale(nrm);
+    const float inv = 1.0f / scale;  // a power of two
+    // the rounding error of the scaled query
+    float rr = 0.0f;
+    for (int i = lane; i < a.d; i += 32) {
+      const float v = __ldg(x + i) * scale;
+      const float h = __half2float(__float2half_rn(v));
+      const float r = fabsf(h) < 0x1p-14f ? fmaxf(fabsf(v), fabsf(v - h)) : v - h;
+      rr = fmaf(r, r, rr);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) rr += __shfl_xor_sync(kFullMask, rr, o);
+    constexpr float kNormM = FHT == 128 ? 1448.2f : FHT == 256 ? 4096.0f : 11585.3f;  // FHT^1.5
+    const float nx = nrm * scale * (1.0f + 0x1p-10f);
+    const float ex = sqrtf(rr) * (1.0f + 0x1p-10f) + 0x1p-20f;
+    const float layer = kNormM * (ex + (nx + ex) * (0x1p-13f + 0x1p-18f)) +
+                        sqrtf((float)a.d) * 1.01f * __ldg(c.merr) * (nx + ex);
+    const float delta = 2.0f * 1.05f * layer * inv;
+    const float* t = c.tmax + (size_t)q * (2 * L * c.parts);
+    for (int l = lane; l < L; l += 32) {
+      float v1 = 0.0f, v2 = 0.0f;
+      for (int p = 0; p < c.parts; ++p) {
+        v1 = fmaxf(v1, __ldg(t + (size_t)(2 * l) * c.parts + p));
+        v2 = fmaxf(v2, __ldg(t + (size_t)(2 * l + 1) * c.parts + p));
+      }
+      sm.sv[l] = (v1 + v2) * inv;
+      sm.sb[l] = (uint32_t)l * a.NB;  // below the cut: never probed
+    }
+    __syncwarp();
+    bool fin = true;
+    for (int i = lane; i < L; i += 32) fin = fin && isfinite(sm.sv[i]);
+    fin = __all_sync(kFullMask, fin);
+    if (!fin) {
+      all = true;
+    } else {
+      const float thr = __uint_as_float(warp_pth_largest(sm.sv, L, qp, lane)) - 2.0f * delta;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = lane + 32 * j;
+        first[j] = __ballot_sync(kFullMask, i < L && sm.sv[i < L ? i : 0] >= thr) & valid[j];
+      }
+      first[0] |= 1u;
+    }
+  }
+  __syncwarp();  // every approximate score has been read before exact ones replace them
+  check_tables<FHT>(a, sm, lane, first);
+  if (!all) {
+    const uint32_t e_cut = warp_pth_largest(sm.sv, L, qp, lane);
+    int ge = 0;
+    for (int i = lane; i < L; i += 32) ge += score_key(sm.sv[i]) >= e_cut ? 1 : 0;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) ge += __shfl_xor_sync(kFullMask, ge, o);
+    if (ge > qp) {
+      uint32_t rest[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rest[j] = valid[j] & ~first[j];
+      __syncwarp();
+      check_tables<FHT>(a, sm, lane, rest);
+      all = true;
+    }
+  }
+  if (a.n_exact && lane == 0) {
+    unsigned n = 0;
+    if (all) {
+      n = (unsigned)L;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) n += (unsigned)__popc(first[j]);
+    }
+    atomicAdd(a.n_exact, n);
+  }
+  float* ov = a.list_v + (size_t)q * a.stride;
+  uint32_t* ob = a.list_b + (size_t)q * a.stride;
+  for (int i = lane; i < L; i += 32) {
+    ov[i] = sm.sv[i];
+    ob[i] = sm.sb[i];
+  }
+}
+
 }  // namespace
 
 long long hash_verified_wave_queries() {
@@ -297,9 +541,9 @@ long long hash_verified_wave_queries() {
 
 cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const float* Q, int nq, const int* q_qprobes,
                                 int qp_max, float* list_v, uint32_t* list_b, long long stride, unsigned* n_exact,
-                                cudaStream_t s) {
+                                const HashScratch& scr, cudaStream_t s) {
   const int L = P.n_tables, D = P.n_proj;
-  if (P.fhtDim != kVFht || !di.tflips || L < 1 || L > kVMaxL || qp_max < 1 || 2 * qp_max > L || stride < L)
+  if ((!di.hmat && (P.fhtDim != kVFht || !di.tflips)) || L < 1 || L > kVMaxL || qp_max < 1 || 2 * qp_max > L || stride < L)
     return cudaErrorInvalidValue;
   if (nq <= 0) return cudaSuccess;
   int log2D = 0;
@@ -320,6 +564,29 @@ cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const fl
   a.list_b = list_b;
   a.stride = stride;
   a.n_exact = n_exact;
+  if (di.hmat) {
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int ld = hmat_ld(P.n_features);
+    for (int q0 = 0, n = 0; q0 < nq; q0 += n) {
+      n = (int)std::min<long long>(scr.nq, nq - q0);
+      a.Q = Q + (size_t)q0 * P.n_features;
+      a.q_qprobes = q_qprobes ? q_qprobes + q0 : nullptr;
+      a.list_v = list_v + q0 * stride;
+      a.list_b = list_b + q0 * stride;
+      k_hash_rows<<<(n + 7) / 8, 256, 0, s>>>(a.Q, n, P.n_features, ld, reinterpret_cast<__half*>(scr.rows));
+      const cudaError_t e = launch_hash_scan(scr.rows, n, di.hmat, 2 * L * D, P.n_features, ld, scr.tmax, scr.status, nsm, s);
+      if (e != cudaSuccess) return e;
+      a.nq = n;
+      const unsigned grid = (unsigned)((n + kCheckWarps - 1) / kCheckWarps);
+      const CheckArgs c{a, scr.tmax, D / 128, di.hmat_err};
+      if (P.fhtDim == 128) k_hash_check<128><<<grid, 32 * kCheckWarps, 0, s>>>(c);
+      if (P.fhtDim == 256) k_hash_check<256><<<grid, 32 * kCheckWarps, 0, s>>>(c);
+      if (P.fhtDim == 512) k_hash_check<512><<<grid, 32 * kCheckWarps, 0, s>>>(c);
+    }
+    return cudaGetLastError();
+  }
   k_query_hash_verified<<<(unsigned)nq, kVThreads, 0, s>>>(a);
   return cudaGetLastError();
 }

@@ -60,7 +60,7 @@ enum RerankMode : int { kRerankFP32 = 0, kRerankBF16 = 1, kRerankFP8 = 2 };
 
 struct DeviceIndex {
   // one allocation (alloc_index) holds Xc, center, flips, tflips, bucket_off,
-  // Xi8 and i8_norm_max
+  // Xi8, i8_norm_max, hmat and hmat_err
   unsigned char* slab = nullptr;
   // centred data, point-major, row stride ld floats (ld = d rounded up to 4)
   float* Xc = nullptr;
@@ -82,7 +82,19 @@ struct DeviceIndex {
   // the form then scores every candidate in FP32), and the largest row norm
   unsigned char* Xi8 = nullptr;      // [n][i8_row_bytes(d)]
   float* i8_norm_max = nullptr;
+  // the rotations as matrices (null: not available): row (2 l + layer) n_proj
+  // + r holds coordinate r of layer and table l as a vector of FP16 weights,
+  // hmat_ld(d) of them; and the largest rounding error of a weight
+  uint16_t* hmat = nullptr;
+  float* hmat_err = nullptr;
 };
+
+// Whether the query hash can use hmat, and its row length.
+inline bool hmat_fits(const Params& P) {
+  return P.n_tables <= 128 && P.n_proj >= 128 && (P.fhtDim == 128 || P.fhtDim == 256 || P.fhtDim == 512) &&
+         P.n_features <= 256;
+}
+inline int hmat_ld(int d) { return (d + 7) & ~7; }  // (rows of a multiple of 64 bytes: the same time)
 
 // Bytes of an int8 screening row: an 8-byte head and d elements, padded to 16.
 inline int i8_row_bytes(int d) { return (d + 8 + 15) & ~15; }
@@ -112,8 +124,8 @@ void free_index(DeviceIndex& di);
 
 // The index's arrays whose sizes follow from the parameters, in one allocation
 // (each allocation of the driver's takes a millisecond or so).  The int8
-// screening rows are part of it for d <= 512, the batched form's range; where
-// it does not fit with them, it is made without.
+// screening rows (for d <= 512, the batched form's range) and the hash matrix are part of
+// it; where it does not fit with them, it is made without.
 cudaError_t alloc_index(const Params& P, DeviceIndex& di);
 
 // One allocation cut into 256-byte aligned arrays: reserve() each pointer,
@@ -141,6 +153,9 @@ class Slab {
   std::vector<std::pair<void**, size_t>> parts_;
   size_t total_ = 0;
 };
+
+// di.hmat from the flip words, if the index has room for it (asynchronous on s).
+cudaError_t make_hash_matrix(const Params& P, DeviceIndex& di, cudaStream_t s);
 
 // The int8 screening rows of the centred data di.Xc (asynchronous on s), if
 // the index has room for them.

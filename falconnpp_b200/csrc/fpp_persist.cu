@@ -225,7 +225,7 @@ int fpp_load(fpp_index* h, const char* path) {
   }
   di.max_kept = max_kept;
   fpp::make_screen_rows(P, di, h->stream);
-  if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
+  if (fpp::make_hash_matrix(P, di, h->stream) != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess) {
     fpp::free_index(di);
     return fail(FPP_ERR_CUDA, "load: the device failed");
   }

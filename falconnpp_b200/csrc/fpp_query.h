@@ -83,14 +83,24 @@ cudaError_t hash_lists(const Params& P, const DeviceIndex& di, const float* Q, i
                        float* list_v, uint32_t* list_b, long long stride, float* heap_v, int* heap_i,
                        long long max_groups, cudaStream_t s);
 
-// The same lists for fhtDim 256 when every query keeps one probe per table
-// (2 qp_max <= L, L <= 128): the rotations on the tensor cores, and an exact
+// Scratch of hash_lists_verified with di.hmat, for `nq` queries at a time: FP16
+// rows (nq x hmat_ld), magnitudes (nq x 2 L n_proj / 128), and a status word
+// (bit 0: a CTA gave up waiting).
+struct HashScratch {
+  uint16_t* rows = nullptr;
+  float* tmax = nullptr;
+  unsigned* status = nullptr;
+  long long nq = 0;
+};
+
+// The same lists when every query keeps one probe per table (2 qp_max <= L, L
+// <= 128), with di.hmat or for fhtDim 256: the rotations on the tensor cores, and an exact
 // FP32 re-hash of every table whose score can reach the probe cut (ties at
 // the cut: of every table), so the probe cut selects the same probes with the
 // same scores.  n_exact (device, nullable) += the tables re-hashed.
 cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const float* Q, int nq, const int* q_qprobes,
                                 int qp_max, float* list_v, uint32_t* list_b, long long stride, unsigned* n_exact,
-                                cudaStream_t s);
+                                const HashScratch& scr, cudaStream_t s);
 
 // Queries k_query_hash_verified takes in one full wave of its blocks on the
 // current device (SMs x resident blocks x queries per block); 0 if unknown.

@@ -598,7 +598,8 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   const bool can_graph = rq.use_graph && !rq.dump_probes && !rq.dump_counts && cl == 1;
   BatchKey key{rq.Q, rq.nq, rq.q_k, rq.q_qprobes, rq.k_uniform, rq.qprobes_uniform, rq.k_max, rq.qprobes_max,
                rq.shortlist_mult, rq.out,
-               rq.out_stride, rq.out_v, rq.mode, grid, kern, bw.bitset, a.order, a.tflips, s};
+               rq.out_stride, rq.out_v, rq.mode, grid, kern, bw.bitset, a.order, a.tflips,
+               bw.bslab, a.Xrows, a.Xscale, s};
   // same launch shape (kernel, grid, stream, scratch): the captured graph is
   // replayed, with the kernel node's arguments updated when they changed
   const bool same_shape = bw.graph_exec && bw.key.kern == key.kern && bw.key.grid == key.grid &&

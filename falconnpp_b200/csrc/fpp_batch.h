@@ -85,12 +85,17 @@ struct BatchKey {
   uint32_t* bitset;
   const uint32_t* order;
   const uint32_t* tflips;
+  // the buffers that a call outside the graph may have moved since
+  const unsigned char* bslab;
+  const unsigned char* rows;
+  const float* scale;
   cudaStream_t stream;
   bool operator==(const BatchKey& o) const {
     return Q == o.Q && nq == o.nq && q_k == o.q_k && q_qprobes == o.q_qprobes && k_uniform == o.k_uniform &&
            qprobes_uniform == o.qprobes_uniform && k_max == o.k_max && qprobes_max == o.qprobes_max && shortlist_mult == o.shortlist_mult && out == o.out &&
            out_stride == o.out_stride && out_v == o.out_v && mode == o.mode && grid == o.grid && kern == o.kern &&
-           bitset == o.bitset && order == o.order && tflips == o.tflips && stream == o.stream;
+           bitset == o.bitset && order == o.order && tflips == o.tflips &&
+           bslab == o.bslab && rows == o.rows && scale == o.scale && stream == o.stream;
   }
 };
 

@@ -203,3 +203,35 @@ def test_host_queries_equal_device_queries(precision):
             assert np.array_equal(host, out.cpu().numpy())
             assert np.array_equal(host, g.query(Q, 10))  # the query buffer is reused safely
     g.close()
+
+
+@pytest.mark.parametrize("between", ["plain", "rows"])
+def test_graph_after_a_call_that_moves_its_buffers(between):
+    """A replayed graph after a call outside it that reallocated the per-batch
+    buffers (a larger plain batch) or the low-precision rows (a small batch of
+    another precision): the results of the first call."""
+    import torch
+    X = synth.mixture(20000, 64, n_centres=16, seed=0)
+    Q = synth.mixture(6000, 64, n_centres=16, seed=1)
+    g = capi.Index(*X.shape)
+    g.set_index_param(12, 64, 100, 0.05, 2, 8, 42)
+    g.build(X)
+    g.set_qprobes(6)
+    g.set_option("use_graph", 1)
+    dq = torch.from_numpy(Q).cuda()
+    got = []
+    for call in range(2):
+        g.set_query_form(1, 2, 4)
+        ids = torch.full((600, 10), -7, dtype=torch.int32, device="cuda") if call == 0 else ids.fill_(-7)
+        torch.cuda.synchronize()
+        g.query_batched(dq.data_ptr(), 600, None, None, 10, 6, ids.data_ptr(), 10)
+        got.append(ids.cpu().numpy().copy())
+        if between == "plain":
+            g.set_query_form(0, 0, 4)
+            g.query(Q, 10)
+        else:
+            g.set_query_form(1, 1, 4)
+            small = torch.zeros((8, 10), dtype=torch.int32, device="cuda")
+            g.query_batched(dq.data_ptr(), 8, None, None, 10, 6, small.data_ptr(), 10)
+    g.close()
+    assert np.array_equal(got[0], got[1])

@@ -351,6 +351,7 @@ struct CheckArgs {
   const float* tmax;  // [nq][2 L parts], parts = D / 128 maxima per layer
   int parts;
   const float* merr;  // the largest rounding error of a weight
+  const unsigned* status;  // not 0: a CTA of the product gave up, every table is hashed exactly
 };
 
 constexpr int kCheckWarps = 4;  // per block
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(32 * kCheckWarps, 16 / kCheckWarps) k_hash_che
   const float* x = a.Q + (size_t)q * a.d;
   for (int i = lane; i < FHT; i += 32) LaneVector<FHT>::at(sm.x, i) = i < a.d ? __ldg(x + i) : 0.0f;
   const float nrm = warp_norm(x, a.d, lane);
-  bool all = !hash_norm_ok(nrm);
+  bool all = !hash_norm_ok(nrm) || *c.status;
   uint32_t valid[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -580,7 +581,7 @@ cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const fl
       if (e != cudaSuccess) return e;
       a.nq = n;
       const unsigned grid = (unsigned)((n + kCheckWarps - 1) / kCheckWarps);
-      const CheckArgs c{a, scr.tmax, D / 128, di.hmat_err};
+      const CheckArgs c{a, scr.tmax, D / 128, di.hmat_err, scr.status};
       if (P.fhtDim == 128) k_hash_check<128><<<grid, 32 * kCheckWarps, 0, s>>>(c);
       if (P.fhtDim == 256) k_hash_check<256><<<grid, 32 * kCheckWarps, 0, s>>>(c);
       if (P.fhtDim == 512) k_hash_check<512><<<grid, 32 * kCheckWarps, 0, s>>>(c);

@@ -85,7 +85,7 @@ cudaError_t hash_lists(const Params& P, const DeviceIndex& di, const float* Q, i
 
 // Scratch of hash_lists_verified with di.hmat, for `nq` queries at a time: FP16
 // rows (nq x hmat_ld), magnitudes (nq x 2 L n_proj / 128), and a status word
-// (bit 0: a CTA gave up waiting).
+// (bit 0: a CTA gave up waiting; while it is set, every table is hashed exactly).
 struct HashScratch {
   uint16_t* rows = nullptr;
   float* tmax = nullptr;

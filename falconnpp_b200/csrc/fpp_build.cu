@@ -179,7 +179,12 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
   const size_t words = (size_t)2 * P.n_tables * 3 * (P.fhtDim < 32 ? 1 : P.fhtDim / 32);
   const size_t nb = (size_t)P.n_tables * 4 * P.n_proj * P.n_proj;
   di.ld = (P.n_features + 3) & ~3;
+  // the optional arrays stay out where they could take the room of what a build
+  // or query needs after them: ids (growing), host data, low-precision rows
+  const size_t later = (size_t)8 * P.n_tables * P.iProbes * n + 8 * n * d + ((size_t)1 << 30);
   cudaError_t e = cudaSuccess;
+  size_t have = 0, all = 0;
+  const bool known = cudaMemGetInfo(&have, &all) == cudaSuccess;
   for (bool extra = true;; extra = false) {
     Slab slab;
     slab.reserve(&di.Xc, n * di.ld);
@@ -199,11 +204,9 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
       slab.reserve(&di.hmat, (size_t)2 * P.n_tables * P.n_proj * hmat_ld(P.n_features));
       slab.reserve(&di.hmat_err, 1);
     }
+    if (extra && known && have < slab.bytes() + later) continue;
     e = slab.alloc(&di.slab);
-    if (e == cudaSuccess || !extra) break;
-    cudaGetLastError();
-    size_t have = 0, all = 0;
-    if (cudaMemGetInfo(&have, &all) != cudaSuccess || have >= slab.bytes()) break;  // not for want of room
+    break;
   }
   return e;
 }

@@ -79,6 +79,18 @@ int check_query_params(const fpp_index* h, int n_queries, int k) {
   return FPP_OK;
 }
 
+// A plain query that ran out of memory on the batched kernels: their scratch
+// (at most the 2 GiB of plain_through_batch, and the batch's lists) is given
+// back, and the three-kernel path, which sizes its own from the candidates
+// found, takes the call.  With 8 GiB free it was not for want of room.
+bool plain_falls_back(fpp_index* h, int rc) {
+  if (rc != FPP_ERR_OUT_OF_MEMORY) return false;
+  cudaGetLastError();
+  h->bw.release();
+  size_t have = 0, all = 0;
+  return cudaMemGetInfo(&have, &all) == cudaSuccess && have < ((size_t)8 << 30);
+}
+
 std::string int2str(int x) {
   std::stringstream ss;
   ss << x;
@@ -395,7 +407,8 @@ int fpp_query(fpp_index* h, const float* queries, int n_queries, int n_neighbors
   const auto t0 = std::chrono::high_resolution_clock::now();
   fpp::Error err{0, ""};
   const bool plain = h->form == 0;
-  if (n_queries > 0 && (!plain || fpp::plain_through_batch(P, h->di, n_queries))) {
+  bool batched = n_queries > 0 && (!plain || fpp::plain_through_batch(P, h->di, n_queries));
+  if (batched) {
     // stage the queries and results through the workspace
     size_t capq = h->ws.cap_Qd, capo = h->ws.cap_out;
     cudaError_t e = cudaSuccess;
@@ -417,8 +430,10 @@ int fpp_query(fpp_index* h, const float* queries, int n_queries, int n_neighbors
     if (!h->cstream && cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking) != cudaSuccess)
       h->cstream = nullptr;
     rc = run_batched(h, h->ws.Qd, n_queries, n_neighbors, h->ws.out, h->stream, plain, queries, out, h->cstream);
-    if (rc) return rc;
-  } else {
+    if (rc && !(plain && plain_falls_back(h, rc))) return rc;
+    batched = rc == FPP_OK;
+  }
+  if (!batched) {
     rc = fpp::query_index(P, h->di, queries, false, n_queries, n_neighbors, out, false, h->ws, h->qst, h->stream,
                           err, nullptr);
     if (rc) return fail(rc, err.msg);
@@ -456,8 +471,8 @@ int fpp_query_device(fpp_index* h, const float* d_queries, int n_queries, int n_
   fpp::Error err{0, ""};
   if (h->form == 1 || fpp::plain_through_batch(h->P, h->di, n_queries)) {
     rc = run_batched(h, d_queries, n_queries, n_neighbors, d_out, s, h->form == 0);
-    if (rc) return rc;
-    return ok();
+    if (rc == FPP_OK) return ok();
+    if (h->form == 1 || !plain_falls_back(h, rc)) return rc;
   }
   rc = fpp::query_index(h->P, h->di, d_queries, true, n_queries, n_neighbors, d_out, true, h->ws, h->qst, s, err,
                         nullptr);

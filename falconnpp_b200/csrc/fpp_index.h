@@ -125,7 +125,7 @@ void free_index(DeviceIndex& di);
 // The index's arrays whose sizes follow from the parameters, in one allocation
 // (each allocation of the driver's takes a millisecond or so).  The int8
 // screening rows (for d <= 512, the batched form's range) and the hash matrix are part of
-// it; where it does not fit with them, it is made without.
+// it; where memory is short, it is made without.
 cudaError_t alloc_index(const Params& P, DeviceIndex& di);
 
 // One allocation cut into 256-byte aligned arrays: reserve() each pointer,

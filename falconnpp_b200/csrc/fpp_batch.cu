@@ -66,7 +66,16 @@ __global__ void k_rows_fp8(const float* __restrict__ Xc, long long n, int ld, in
 // queries in flight at the same time then probe overlapping buckets and rows,
 // which stay in L2.  Each query is computed independently, so the order
 // changes no result.
-constexpr int kOrderMaxBins = 1024;  // 2 * n_proj codes
+//
+// A mixed batch (per-query qProbes) is first grouped by the power of two below
+// qProbes, the largest first: a query of 80 probes runs six times as long as
+// one of 5, and one that starts last leaves the other blocks idle.  Eight
+// classes; within a class the codes as above, in pairs where the bins need it.
+// qProbes from {1, 5, 10, 20, 80}, FP8, 444 blocks, by codes alone / so: 450
+// queries 215 / 222 us (the two launches), 600: 266 / 253, 1,000: 376 / 330,
+// 2,047: 685 / 643, 10,000: 2,609 / 2,563; hence the line at 592.
+constexpr int kOrderMaxBins = 4096;
+constexpr int kOrderClasses = 8;
 
 template <int FHT>
 __global__ void __launch_bounds__(256) k_order_key(const float* __restrict__ Q, int nq, int d,
@@ -97,26 +106,42 @@ __global__ void __launch_bounds__(256) k_order_key(const float* __restrict__ Q, 
 // the histogram zeroed for the next batch
 __global__ void __launch_bounds__(1024) k_order_scatter(const uint32_t* __restrict__ key, int nq, int bins,
                                                         uint32_t* __restrict__ hist, uint32_t* __restrict__ order) {
+  constexpr int B = kOrderMaxBins / 1024;  // bins per thread
   __shared__ uint32_t off[kOrderMaxBins];
   __shared__ long long tmp[32];
   const int t = threadIdx.x;
-  const uint32_t h = t < bins ? hist[t] : 0u;
+  uint32_t h[B];
+  uint32_t sum = 0;
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const int b = t * B + i;
+    h[i] = b < bins ? hist[b] : 0u;
+    if (b < bins) hist[b] = 0u;
+    sum += h[i];
+  }
   long long tot;
-  const long long ex = block_exclusive_scan((long long)h, tmp, &tot);
-  if (t < bins) {
-    off[t] = (uint32_t)ex;
-    hist[t] = 0u;
+  uint32_t ex = (uint32_t)block_exclusive_scan((long long)sum, tmp, &tot);
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    off[t * B + i] = ex;
+    ex += h[i];
   }
   __syncthreads();
   for (int q = t; q < nq; q += blockDim.x) order[atomicAdd(&off[key[q]], 1u)] = (uint32_t)q;
 }
 
 // the key from the exact lists: the first-layer code of table 0's best bucket
-__global__ void k_order_key_ext(const uint32_t* __restrict__ lb, int nq, long long stride, int twoD,
-                                uint32_t* __restrict__ key, uint32_t* __restrict__ hist) {
+// (>> shift), in a mixed batch below the class of the query's qProbes
+__global__ void k_order_key_ext(const uint32_t* __restrict__ lb, int nq, long long stride, int twoD, int shift,
+                                const int* __restrict__ q_qprobes, int qp_max, uint32_t* __restrict__ key,
+                                uint32_t* __restrict__ hist) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nq) return;
-  const uint32_t c = lb[(size_t)q * stride] / (uint32_t)twoD;  // table 0: global id = c1 * 2D + c2
+  uint32_t c = (lb[(size_t)q * stride] / (uint32_t)twoD) >> shift;  // table 0: global id = c1 * 2D + c2
+  if (q_qprobes) {
+    const int qp = min(max(q_qprobes[q], 1), qp_max);
+    c += (uint32_t)min(__clz(qp) - __clz(qp_max), kOrderClasses - 1) * (uint32_t)(twoD >> shift);
+  }
   key[q] = c;
   atomicAdd(hist + c, 1u);
 }
@@ -467,11 +492,19 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   int log2D = 0;
   while ((1 << log2D) < D) ++log2D;
   const void* okern = order_key_kernel(F);
-  const bool reorder = rq.reorder && okern && rq.nq >= 2 * grid && 2 * D <= kOrderMaxBins;
+  // (mixed: from a third of a second wave on)
+  const bool mixed = split && rq.q_qprobes;
+  const bool reorder =
+      rq.reorder && okern && (mixed ? 3LL * rq.nq >= 4LL * grid : rq.nq >= 2 * grid) && 2 * D <= kOrderMaxBins;
   if (reorder && split) {
-    k_order_key_ext<<<(rq.nq + 255) / 256, 256, 0, s>>>(bw.ext_lb, rq.nq, ext_stride, 2 * D, bw.okey, bw.ohist);
+    int shift = 0;
+    while (mixed && kOrderClasses * ((2 * D) >> shift) > kOrderMaxBins) ++shift;
+    k_order_key_ext<<<(rq.nq + 255) / 256, 256, 0, s>>>(bw.ext_lb, rq.nq, ext_stride, 2 * D, shift,
+                                                        mixed ? rq.q_qprobes : nullptr, rq.qprobes_max, bw.okey,
+                                                        bw.ohist);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "order key launch");
-    k_order_scatter<<<1, 1024, 0, s>>>(bw.okey, rq.nq, 2 * D, bw.ohist, bw.order);
+    k_order_scatter<<<1, 1024, 0, s>>>(bw.okey, rq.nq, (mixed ? kOrderClasses : 1) * ((2 * D) >> shift), bw.ohist,
+                                       bw.order);
     if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "order scatter launch");
   } else if (reorder) {
     const int per_block = 256 / (F / 32);

@@ -235,3 +235,25 @@ def test_graph_after_a_call_that_moves_its_buffers(between):
             g.query_batched(dq.data_ptr(), 8, None, None, 10, 6, small.data_ptr(), 10)
     g.close()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("D,nq", [(64, 592), (256, 700), (512, 2100)])
+def test_mixed_order_changes_nothing(D, nq):
+    """Mixed batches grouped by qProbes (every class, powers of two and their
+    neighbours; codes whole and in pairs): the results in call order."""
+    import torch
+    X = synth.mixture(20000, 64, n_centres=16, seed=0)
+    Q = synth.mixture(nq, 64, n_centres=16, seed=1)
+    g = _index(X, 8, D, 60, 0.05, 2)
+    g.set_query_form(1, 0, 4)
+    qps = torch.from_numpy(np.random.default_rng(5).choice([1, 2, 3, 4, 7, 8, 127, 128, 255, 300], nq).astype(np.int32)).cuda()
+    dq = torch.from_numpy(Q).cuda()
+    got = []
+    for reorder in (1, 0):
+        g.set_option("reorder_queries", reorder)
+        ids = torch.full((nq, 10), -7, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        g.query_batched(dq.data_ptr(), nq, None, qps.data_ptr(), 10, 300, ids.data_ptr(), 10)
+        got.append(ids.cpu().numpy())
+    g.close()
+    assert np.array_equal(got[0], got[1])

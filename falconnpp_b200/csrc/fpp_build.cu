@@ -31,6 +31,7 @@
 
 #include "fpp_device.cuh"
 #include "fpp_index.h"
+#include "fpp_stage.h"
 
 namespace fpp {
 
@@ -1146,8 +1147,8 @@ fail:
 }
 
 int build_index(const Params& P, const float* X, bool x_on_device, const HostBits& bits,
-                const BuildOptions& opt, DeviceIndex& di, BuildStats& st, cudaStream_t s, Error& err,
-                int32_t* dump_codes, float* dump_scores) {
+                const BuildOptions& opt, HostStage& stage, DeviceIndex& di, BuildStats& st, cudaStream_t s,
+                Error& err, int32_t* dump_codes, float* dump_scores) {
   const auto t_start = std::chrono::steady_clock::now();
   const long long n = P.n_points;
   const int d = P.n_features, L = P.n_tables, D = P.n_proj, F = P.fhtDim, IP = P.iProbes;
@@ -1238,7 +1239,7 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     auto t0 = std::chrono::steady_clock::now();
     const float* Xd = X;
     if (!x_on_device) {
-      FPP_CUDA(cudaMemcpyAsync(Xstage, X, sizeof(float) * n * d, cudaMemcpyHostToDevice, s));
+      FPP_CUDA(stage.copy(Xstage, X, sizeof(float) * n * d, s));
       Xd = Xstage;
     }
     FPP_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), s));

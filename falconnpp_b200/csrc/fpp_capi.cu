@@ -119,7 +119,7 @@ int do_build(fpp_index* h, const float* X, bool on_device, cudaStream_t s, int32
   h->built = false;
   fpp::Error err{0, ""};
   h->bst = fpp::BuildStats();
-  const int rc = fpp::build_index(P, X, on_device, h->bits, h->opt, h->di, h->bst, s, err, dcodes, dscores);
+  const int rc = fpp::build_index(P, X, on_device, h->bits, h->opt, h->stage, h->di, h->bst, s, err, dcodes, dscores);
   if (rc == FPP_OK && codes_host) {
     cudaMemcpy(codes_host, dcodes, sizeof(int32_t) * ncodes, cudaMemcpyDeviceToHost);
     cudaMemcpy(scores_host, dscores, sizeof(float) * ncodes, cudaMemcpyDeviceToHost);
@@ -275,6 +275,7 @@ void fpp_destroy(fpp_index* h) {
     h->ws.release();
     h->bw.release();
     h->bfw.release();
+    h->stage.release();
     fpp::free_index(h->di);
     if (h->stream) cudaStreamDestroy(h->stream);
     if (h->cstream) cudaStreamDestroy(h->cstream);
@@ -333,6 +334,7 @@ int fpp_clear(fpp_index* h) {
   h->ws.release();
   h->bw.release();
     h->bfw.release();
+  h->stage.release();
   fpp::free_index(h->di);
   h->bits = fpp::HostBits();
   h->built = false;

@@ -8,6 +8,7 @@
 #include "fpp_batch.h"
 #include "fpp_index.h"
 #include "fpp_query.h"
+#include "fpp_stage.h"
 
 struct fpp_index {
   fpp::Params P;
@@ -19,6 +20,7 @@ struct fpp_index {
   fpp::QueryStats qst;
   fpp::BatchWorkspace bw;
   fpp::BfWorkspace bfw;
+  fpp::HostStage stage;     // pageable data on its way to a build
   int form = 0;             // 0 plain three-kernel path, 1 batched fused kernel
   int precision = 0;        // batched form: 0 FP32 (exact), 1 BF16, 2 FP8-E4M3
   int shortlist_mult = 4;   // batched low precision: FP32 re-score of shortlist_mult * k

@@ -116,9 +116,11 @@ struct BuildOptions {
   int tables_per_chunk = 0;        // 0 = automatic
 };
 
+class HostStage;  // fpp_stage.h
+
 int build_index(const Params& P, const float* X, bool x_on_device, const HostBits& bits,
-                const BuildOptions& opt, DeviceIndex& di, BuildStats& st, cudaStream_t s, Error& err,
-                int32_t* dump_codes, float* dump_scores);
+                const BuildOptions& opt, HostStage& stage, DeviceIndex& di, BuildStats& st, cudaStream_t s,
+                Error& err, int32_t* dump_codes, float* dump_scores);
 
 void free_index(DeviceIndex& di);
 

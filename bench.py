@@ -380,17 +380,14 @@ def run_ours(args, w, rank, world, local_rank):
         plain_stats = (st[1], st[0], None)
         idx.set_query_form(form, prec, mult)
     U, C, _ = plain_stats
-    lpb = {0: 4 * d, 1: 2 * ((d + 7) // 8 * 8), 2: (d + 15) // 16 * 16 + 4}[prec]
+    # FP32 (plain, too) reads every candidate's int8 screening row, and the FP32
+    # rows of the top k at least
+    lpb = {0: (d + 8 + 15) // 16 * 16 if d <= 512 else 4 * d, 1: 2 * ((d + 7) // 8 * 8), 2: (d + 15) // 16 * 16 + 4}[prec]
     common = C * 4 + nq * chosen * 8 + nq * (4 * d + 4 * k)
-    if form == 0:
-        kern = "k_gather_rerank"
-        bytes_per_launch = U * 4 * d + common
-        launch_s = plain_stats[2]
-    else:
-        kern = "k_batch_query"
-        short = 0 if prec == 0 else nq * min(mult * k, 1024) * 4 * ((d + 3) // 4 * 4)
-        bytes_per_launch = U * lpb + short + common
-        launch_s = statistics.mean(hr["rerank_ms"]) / 1000.0
+    kern = "k_batch_query"
+    short = nq * min((1 if prec == 0 else mult) * k, 1024) * 4 * ((d + 3) // 4 * 4)
+    bytes_per_launch = U * lpb + short + common
+    launch_s = statistics.mean(hr["rerank_ms"]) / 1000.0
     achieved = bytes_per_launch / launch_s / 1e9
     traffic = None
     prof = os.path.join(ROOT, "profiles", f"{kern}.traffic.json")
@@ -401,10 +398,9 @@ def run_ours(args, w, rank, world, local_rank):
         traffic = traffic * U if traffic else None
 
     # the hash kernel of the batched form.  With one probe per table (2 qProbes
-    # <= L, fhtDim 256, L <= 128) it is k_query_hash_verified: rotations on the
-    # tensor cores, and the reference's FP32 arithmetic for every table whose
-    # score can reach the probe cut (the share below); otherwise the exact FP32
-    # k_query_hash, against the FP32 add rate (6 FWHT of fhtDim * log2(fhtDim)
+    # <= L, L <= 128) it is the rotations as one product on the tensor cores, and
+    # the reference's FP32 arithmetic for every table whose score can reach the
+    # probe cut (the share below); otherwise the exact FP32 k_query_hash, against the FP32 add rate (6 FWHT of fhtDim * log2(fhtDim)
     # add/sub per (query, table)).  Both give the exact hash's lists.
     fht = 1 << max(0, (max(w["D"], d) - 1).bit_length())
     adds = nq * w["L"] * 6 * fht * (fht.bit_length() - 1)
@@ -414,8 +410,9 @@ def run_ours(args, w, rank, world, local_rank):
         mhz = clk.summary().get("sm_mhz") or 1965.0
         peak_adds = 148 * 128 * mhz * 1e6 / 1e12  # FP32 lanes x clock, T add/s (nominal)
         verified = hr["rehashed"] > 0
-        hash_kernel = {"kernel": "k_query_hash_verified (tensor-core rotation, FP32 re-hash of the tables "
-                                 "that can reach the probe cut)" if verified else "k_query_hash (exact FP32)",
+        hash_kernel = {"kernel": "k_bf_scan<kScanHash> + k_hash_check (rotations as one tensor-core product, "
+                                 "FP32 re-hash of the tables that can reach the probe cut)"
+                       if verified else "k_query_hash (exact FP32)",
                        "ms": round(hms, 4),
                        "order_and_probe_cut_ms": round(statistics.mean(hr["prep_ms"]), 4),
                        "fused_kernel_ms": round(launch_s * 1e3, 4)}

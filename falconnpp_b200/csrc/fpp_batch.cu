@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <algorithm>
 #include <vector>
@@ -541,6 +542,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     if ((e = probe_cut_lists(pa, rq.nq, s)) != cudaSuccess) return fail(e, "probe cut launch");
   }
   BatchArgs a;
+  memset(&a, 0, sizeof(a));  // padding too: a graph's arguments are compared as bytes
   a.Xc = di.Xc;
   a.ld = di.ld;
   if (kmode == kRowsI8) {
@@ -629,16 +631,14 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     cudaEventRecord(bw.tev[1], s);
   }
   const bool can_graph = rq.use_graph && !rq.dump_probes && !rq.dump_counts && cl == 1;
-  BatchKey key{rq.Q, rq.nq, rq.q_k, rq.q_qprobes, rq.k_uniform, rq.qprobes_uniform, rq.k_max, rq.qprobes_max,
-               rq.shortlist_mult, rq.out,
-               rq.out_stride, rq.out_v, rq.mode, grid, kern, bw.bitset, a.order, a.tflips,
-               bw.bslab, a.Xrows, a.Xscale, s};
-  // same launch shape (kernel, grid, stream, scratch): the captured graph is
-  // replayed, with the kernel node's arguments updated when they changed
-  const bool same_shape = bw.graph_exec && bw.key.kern == key.kern && bw.key.grid == key.grid &&
-                          bw.key.stream == key.stream && bw.key.bitset == key.bitset;
+  // same launch (kernel, grid, stream; the memset node's counters live as long
+  // as the graph): the captured graph is replayed, with the kernel node's
+  // arguments updated when any of them changed
+  const bool same_shape =
+      bw.graph_exec && bw.graph_kern == kern && bw.graph_grid == grid && bw.graph_stream == s;
+  const unsigned char* abytes = reinterpret_cast<const unsigned char*>(&a);
   if (can_graph && same_shape) {
-    if (!(bw.key == key)) {
+    if (memcmp(bw.graph_args.data(), &a, sizeof(a)) != 0) {
       cudaKernelNodeParams kp = {};
       kp.func = const_cast<void*>(kern);
       kp.gridDim = dim3(grid);
@@ -647,7 +647,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
       kp.kernelParams = args;
       if ((e = cudaGraphExecKernelNodeSetParams(bw.graph_exec, bw.graph_knode, &kp)) != cudaSuccess)
         return fail(e, "graph update");
-      bw.key = key;
+      bw.graph_args.assign(abytes, abytes + sizeof(a));
     }
     if ((e = cudaGraphLaunch(bw.graph_exec, s)) != cudaSuccess) return fail(e, "graph launch");
     res.graph_replayed = true;
@@ -673,13 +673,21 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
       e = cudaGraphInstantiate(&bw.graph_exec, graph, 0);
       if (bw.graph) cudaGraphDestroy(bw.graph);
       bw.graph = graph;  // kept alive: the kernel node handle belongs to it
-      if (e != cudaSuccess) return fail(e, "graph instantiate");
+      if (e != cudaSuccess) {
+        bw.graph_exec = nullptr;
+        return fail(e, "graph instantiate");
+      }
       if (!bw.graph_knode) {
+        cudaGraphExecDestroy(bw.graph_exec);
+        bw.graph_exec = nullptr;
         err.code = kErrCuda;
         err.msg = "batch query: captured graph has no kernel node";
         return err.code;
       }
-      bw.key = key;
+      bw.graph_kern = kern;
+      bw.graph_grid = grid;
+      bw.graph_stream = s;
+      bw.graph_args.assign(abytes, abytes + sizeof(a));
       if ((e = cudaGraphLaunch(bw.graph_exec, s)) != cudaSuccess) return fail(e, "graph launch");
     } else {
       if ((e = cudaMemsetAsync(bw.counters, 0, sizeof(unsigned) * 2, s)) != cudaSuccess) return fail(e, "memset");

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "fpp_index.h"
 
 namespace fpp {
@@ -71,34 +73,6 @@ struct BatchResult {
   long long tc_exact = 0;           // with stage_timing: tables the verified hash re-hashed in FP32
 };
 
-struct BatchKey {
-  const float* Q;
-  int nq;
-  const int* q_k;
-  const int* q_qprobes;
-  int k_uniform, qprobes_uniform, k_max, qprobes_max, shortlist_mult;
-  int32_t* out;
-  int out_stride;
-  float* out_v;
-  int mode, grid;
-  const void* kern;
-  uint32_t* bitset;
-  const uint32_t* order;
-  const uint32_t* tflips;
-  // the buffers that a call outside the graph may have moved since
-  const unsigned char* bslab;
-  const unsigned char* rows;
-  const float* scale;
-  cudaStream_t stream;
-  bool operator==(const BatchKey& o) const {
-    return Q == o.Q && nq == o.nq && q_k == o.q_k && q_qprobes == o.q_qprobes && k_uniform == o.k_uniform &&
-           qprobes_uniform == o.qprobes_uniform && k_max == o.k_max && qprobes_max == o.qprobes_max && shortlist_mult == o.shortlist_mult && out == o.out &&
-           out_stride == o.out_stride && out_v == o.out_v && mode == o.mode && grid == o.grid && kern == o.kern &&
-           bitset == o.bitset && order == o.order && tflips == o.tflips &&
-           bslab == o.bslab && rows == o.rows && scale == o.scale && stream == o.stream;
-  }
-};
-
 // Per-block scratch of the batched kernel (kept between calls) and the cached graph.
 struct BatchWorkspace {
   unsigned char* slab = nullptr;   // the per-block scratch and the counters
@@ -152,7 +126,12 @@ struct BatchWorkspace {
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphNode_t graph_knode = nullptr;
-  BatchKey key{};
+  // what the captured nodes hold: the launch, and the kernel node's arguments
+  // byte for byte (BatchArgs): every pointer and stride, whichever call moved it
+  const void* graph_kern = nullptr;
+  int graph_grid = 0;
+  cudaStream_t graph_stream = nullptr;
+  std::vector<unsigned char> graph_args;
   void release();
 };
 

@@ -1,0 +1,55 @@
+"""The batched form's workspace over calls of changing shape on one handle:
+a replayed graph after calls outside it have moved the buffers inside the
+per-batch allocation (its base address may stay the same), against the first
+call's results."""
+import numpy as np
+import pytest
+
+from falconnpp_b200 import capi, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _index(L=12, D=64, qp=6):
+    X = synth.mixture(20000, 64, n_centres=16, seed=0)
+    g = capi.Index(*X.shape)
+    g.set_index_param(L, D, 100, 0.05, 2, 8, 42)
+    g.build(X)
+    g.set_qprobes(qp)
+    return g
+
+
+def _batched(g, dq, nq, k, qp, ids):
+    ids.fill_(-7)
+    import torch
+    torch.cuda.synchronize()
+    g.query_batched(dq.data_ptr(), nq, None, None, k, qp, ids.data_ptr(), k)
+    return ids.cpu().numpy().copy()
+
+
+@pytest.mark.parametrize("form,nq,qp", [(0, 601, 6), (0, 640, 6), (0, 700, 6), (0, 880, 6), (1, 222, 20), (1, 200, 26)])
+def test_graph_after_calls_that_move_buffers_within_the_allocation(form, nq, qp):
+    # 600 queries: less than two waves, so the graph's node has no order array;
+    # the call between (a plain query, or a small batch on clusters, which takes
+    # no graph) needs a few per cent more of the per-batch buffers
+    import torch
+    Q = synth.mixture(900, 64, n_centres=16, seed=1)
+    dq = torch.from_numpy(Q).cuda()
+    ids = torch.zeros((600, 10), dtype=torch.int32, device="cuda")
+    small = torch.zeros((nq, 10), dtype=torch.int32, device="cuda")
+    g = _index()
+    g.query_dump(Q, 10, 6)  # the query buffers of host calls are in place
+    g.set_option("use_graph", 1)
+    g.set_query_form(1, 2, 4)
+    first = _batched(g, dq, 600, 10, 6, ids)
+    for _ in range(3):
+        if form == 0:
+            g.set_query_form(0, 0, 4)
+            g.set_qprobes(qp)
+            g.query(Q[:nq], 10)
+            g.set_qprobes(6)
+            g.set_query_form(1, 2, 4)
+        else:
+            _batched(g, dq, nq, 10, qp, small)
+        assert np.array_equal(_batched(g, dq, 600, 10, 6, ids), first)
+    g.close()

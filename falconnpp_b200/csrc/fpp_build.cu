@@ -29,6 +29,7 @@
 #include <chrono>
 #include <vector>
 
+#include "fpp_arena.h"
 #include "fpp_device.cuh"
 #include "fpp_index.h"
 #include "fpp_stage.h"
@@ -616,6 +617,7 @@ struct BucketArgs {
   struct RepairItem* items[3];
   unsigned* deferred;
   unsigned arena_entries;
+  unsigned max_items;  // per class
 };
 
 // A bucket whose ties the reference's heap decides: B entries (in any order),
@@ -645,27 +647,29 @@ constexpr unsigned kRepairCap[2] = {880, 7000};
 
 // A tie in bucket b: put off (the caller copies the entries to arena +
 // the returned position) while there is room, else repaired after this chunk
-// (0xffffffff).  A replay is one long chain, so the few hundred of a chunk
+// (kArenaFull).  A replay is one long chain, so the few hundred of a chunk
 // would leave the GPU waiting for the longest of them chunk after chunk (41 of
 // 205 ms at 1M x 200, 100 tables, 6,303 repairs); all at once they fill it.
 __device__ __forceinline__ unsigned add_repair(const BucketArgs& a, uint32_t b, uint32_t B, uint32_t kp, uint32_t out) {
   const int c = B <= kRepairCap[0] ? 0 : B <= kRepairCap[1] ? 1 : 2;
   atomicAdd(a.n_repaired, 1ull);
-  if (B <= a.arena_entries) {
-    const unsigned pos = atomicAdd(a.deferred, B);
-    if (pos <= a.arena_entries - B) {
-      const unsigned i = atomicAdd(a.deferred + 1 + c, 1u);
-      if (i < kRepairItems) {
-        a.items[c][i] = RepairItem{pos, B, kp, out};
-        return pos;
-      }
-      atomicSub(a.deferred + 1 + c, 1u);  // never below the items written
-    } else {
-      atomicSub(a.deferred, B);
+  auto reserve = [](unsigned* used, unsigned want, unsigned cap) {
+    return arena_reserve(
+        want, cap, [=] { return *(volatile unsigned*)used; },
+        [=](unsigned expect, unsigned value) { return atomicCAS(used, expect, value); });
+  };
+  unsigned* items = a.deferred + 1 + c;
+  if (*(volatile unsigned*)items < a.max_items) {  // else the class is full for good
+    const unsigned pos = reserve(a.deferred, B, a.arena_entries);
+    // (the last item may go to another warp meanwhile: then the range stays unused)
+    const unsigned i = pos == kArenaFull ? kArenaFull : reserve(items, 1u, a.max_items);
+    if (i != kArenaFull) {
+      a.items[c][i] = RepairItem{pos, B, kp, out};
+      return pos;
     }
   }
   a.repair[c][atomicAdd(a.counters + 3 + c, 1u)] = b;
-  return 0xffffffffu;
+  return kArenaFull;
 }
 
 // Whether the kept entry at rank r and the next one make the reference's heap
@@ -739,7 +743,7 @@ __global__ void __launch_bounds__(256) k_bucket_small(BucketArgs a) {
       unsigned pos = 0;
       if (lane == 0) pos = add_repair(a, b0 + src, cB, ck, co);
       pos = __shfl_sync(kFullMask, pos, 0);
-      if (pos != 0xffffffffu && lane < (int)cB) a.arena[pos + lane] = e;
+      if (pos != kArenaFull && lane < (int)cB) a.arena[pos + lane] = e;
     }
   }
 }
@@ -783,7 +787,7 @@ __global__ void __launch_bounds__(256) k_bucket_medium(BucketArgs a) {
       unsigned pos = 0;
       if (lane == 0) pos = add_repair(a, b, B, kp, out);
       pos = __shfl_sync(kFullMask, pos, 0);
-      if (pos != 0xffffffffu)
+      if (pos != kArenaFull)
         for (uint32_t i = lane; i < B; i += 32) a.arena[pos + i] = e[i];
     }
     __syncwarp();
@@ -884,7 +888,7 @@ __global__ void __launch_bounds__(256) k_bucket_large(BucketArgs a) {
       if (threadIdx.x == 0) s_pos = add_repair(a, b, B, kp, a.off[b]);
       __syncthreads();
       const unsigned pos = s_pos;
-      if (pos != 0xffffffffu)
+      if (pos != kArenaFull)
         for (uint32_t i = threadIdx.x; i < B; i += 256) a.arena[pos + i] = e[i];
     }
   }
@@ -1197,7 +1201,11 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   const long long nb_chunk_max = tables_per_chunk * (long long)NB;
   const long long nblk_max = (nb_chunk_max + kScanTile - 1) / kScanTile;
   // put-off repairs: the size of a small build's entries is enough
-  const unsigned arena_entries = (unsigned)std::min<unsigned long long>(kArenaEntries, (unsigned long long)L * n * IP);
+  const unsigned arena_entries = (unsigned)std::min<unsigned long long>(
+      opt.repair_arena > 0 ? std::min<unsigned>(kArenaEntries, opt.repair_arena) : kArenaEntries,
+      (unsigned long long)L * n * IP);
+  const unsigned max_items =
+      opt.repair_items > 0 ? std::min<unsigned>(kRepairItems, opt.repair_items) : kRepairItems;
 
   free_index(di);
   if (max_entries >= (1LL << 32) || nb_chunk_max >= (1LL << 32)) {
@@ -1365,6 +1373,7 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     for (int c = 0; c < 3; ++c) ba.items[c] = items[c];
     ba.deferred = deferred;
     ba.arena_entries = arena_entries;
+    ba.max_items = max_items;
     for (int c = 0; c < 3; ++c) ba.repair[c] = repair[c];
     ba.counters = counters;
     ba.n_repaired = totals + 2;

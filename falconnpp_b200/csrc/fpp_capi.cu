@@ -5,6 +5,7 @@
 // codes instead of undefined behaviour, and the verbose side effects of
 // query2Layers_1D (src/FalconnPP.cpp:682-703).
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -367,6 +368,9 @@ int fpp_set_option(fpp_index* h, const char* key, long long value) {
   } else if (!strcmp(key, "tables_per_chunk")) {
     if (value < 0) return fail(FPP_ERR_INVALID_ARGUMENT, "set_option: tables_per_chunk must be >= 0");
     h->opt.tables_per_chunk = (int)value;
+  } else if (!strcmp(key, "repair_arena") || !strcmp(key, "repair_items")) {
+    if (value < 0 || value > INT_MAX) return fail(FPP_ERR_INVALID_ARGUMENT, std::string("set_option: bad ") + key);
+    (key[7] == 'a' ? h->opt.repair_arena : h->opt.repair_items) = (int)value;
   } else {
     return fail(FPP_ERR_INVALID_ARGUMENT, std::string("set_option: unknown key ") + key);
   }

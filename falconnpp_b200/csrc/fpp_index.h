@@ -114,6 +114,8 @@ struct HostBits {
 struct BuildOptions {
   bool exact_bucket_order = true;  // replay ties inside kept prefixes too
   int tables_per_chunk = 0;        // 0 = automatic
+  int repair_arena = 0;            // put-off tie repairs: entries, and buckets per
+  int repair_items = 0;            // size class, at most (0 = automatic)
 };
 
 class HostStage;  // fpp_stage.h

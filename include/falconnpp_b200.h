@@ -105,6 +105,9 @@ int fpp_get_stats(fpp_index* h, int kind, double* out, int n);
 /* Tuning and test switches: "exact_bucket_order" (default 1: bucket contents
  * in the reference's heap order even among equal scores; 0: ascending id among
  * equal scores, the kept set is identical either way), "tables_per_chunk",
+ * "repair_arena" and "repair_items" (test switches: how many bucket entries,
+ * and how many buckets of each size class, a build puts off to one tie-repair
+ * launch at its end; 0 = automatic; the tables are the same either way),
  * "stage_timing" (0/1: CUDA events around each query kernel), "use_graph"
  * (0/1: batched form captured into a CUDA graph and replayed for repeated
  * shapes; the stream must not be the legacy default stream), "blocks_per_sm"

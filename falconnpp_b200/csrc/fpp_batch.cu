@@ -197,9 +197,16 @@ fail:
   return err.code;
 }
 
-void BatchWorkspace::release() {
+void BatchWorkspace::drop_graph() {
   if (graph_exec) cudaGraphExecDestroy(graph_exec);
   if (graph) cudaGraphDestroy(graph);
+  graph_exec = nullptr;
+  graph = nullptr;
+  graph_knode = nullptr;
+}
+
+void BatchWorkspace::release() {
+  drop_graph();
   cudaFree(slab);
   cudaFree(bslab);
   for (auto& ev : tev)
@@ -207,6 +214,83 @@ void BatchWorkspace::release() {
   for (auto& ev : cev)
     if (ev) cudaEventDestroy(ev);
   *this = BatchWorkspace();
+}
+
+cudaError_t BatchWorkspace::grow_block(const Block& n, cudaStream_t s) {
+  const Block& h = block;
+  if (slab && h.bits >= n.bits && h.uniq >= n.uniq && h.dump >= n.dump && h.heap >= n.heap && h.hheap >= n.hheap &&
+      h.list >= n.list && h.probe >= n.probe && h.layer >= n.layer && h.replay >= n.replay)
+    return cudaSuccess;
+  const Block both{std::max(h.bits, n.bits),   std::max(h.uniq, n.uniq),   std::max(h.dump, n.dump),
+                   std::max(h.heap, n.heap),   std::max(h.hheap, n.hheap), std::max(h.list, n.list),
+                   std::max(h.probe, n.probe), std::max(h.layer, n.layer), std::max(h.replay, n.replay)};
+  drop_graph();  // its memset node names the counters
+  cudaFree(slab);
+  slab = nullptr;
+  block = Block();
+  size_t tried = 0;
+  cudaError_t e = cudaSuccess;
+  for (const Block* b : {&both, &n}) {
+    Slab sl;
+    sl.reserve(&bitset, (size_t)b->bits);
+    sl.reserve(&uniq, (size_t)b->uniq);
+    sl.reserve(&score, (size_t)b->uniq);
+    sl.reserve(&gdump, (size_t)b->dump);
+    sl.reserve(&gheap_v, (size_t)b->heap);
+    sl.reserve(&gheap_i, (size_t)b->heap);
+    sl.reserve(&counters, 1);
+    sl.reserve(&hheap_v, (size_t)b->hheap);
+    sl.reserve(&hheap_i, (size_t)b->hheap);
+    sl.reserve(&glv, (size_t)b->list);
+    sl.reserve(&glb, (size_t)b->list);
+    sl.reserve(&gprobe, (size_t)b->probe);
+    sl.reserve(&gpo, (size_t)b->probe);
+    sl.reserve(&gpe, (size_t)b->probe);
+    sl.reserve(&ggv, (size_t)b->layer);
+    sl.reserve(&ggc, (size_t)b->layer);
+    sl.reserve(&grhv, (size_t)b->replay);
+    sl.reserve(&grhi, (size_t)b->replay);
+    if (sl.bytes() == tried) return e;  // nothing else to give back
+    tried = sl.bytes();
+    if ((e = sl.alloc(&slab)) != cudaSuccess) continue;
+    block = *b;
+    if ((e = cudaMemsetAsync(bitset, 0, sizeof(uint32_t) * (size_t)b->bits, s)) == cudaSuccess)
+      e = cudaMemsetAsync(counters, 0, sizeof(BatchCounters), s);
+    return e;
+  }
+  return e;
+}
+
+cudaError_t BatchWorkspace::grow_batch(const Batch& n, cudaStream_t s) {
+  const Batch& h = batch;
+  if (bslab && h.nq >= n.nq && h.ext >= n.ext && h.pc >= n.pc && h.hash >= n.hash && h.hq >= n.hq) return cudaSuccess;
+  const Batch both{std::max(h.nq, n.nq), std::max(h.ext, n.ext), std::max(h.pc, n.pc), std::max(h.hash, n.hash),
+                   std::max(h.hq, n.hq)};
+  cudaFree(bslab);
+  bslab = nullptr;
+  batch = Batch();
+  size_t tried = 0;
+  cudaError_t e = cudaSuccess;
+  for (const Batch* b : {&both, &n}) {
+    Slab sl;
+    sl.reserve(&okey, (size_t)b->nq);
+    sl.reserve(&order, (size_t)b->nq);
+    sl.reserve(&ohist, (size_t)kOrderMaxBins);
+    sl.reserve(&ext_lv, (size_t)b->ext);
+    sl.reserve(&ext_lb, (size_t)b->ext);
+    sl.reserve(&pc_g, (size_t)b->pc);
+    sl.reserve(&pc_o, (size_t)b->pc);
+    sl.reserve(&pc_pe, (size_t)b->pc);
+    sl.reserve(&pc_n, (size_t)b->nq);
+    sl.reserve(&hq, (size_t)b->hq);
+    sl.reserve(&htmax, (size_t)b->hash);
+    if (sl.bytes() == tried) return e;
+    tried = sl.bytes();
+    if ((e = sl.alloc(&bslab)) != cudaSuccess) continue;
+    batch = *b;
+    return cudaMemsetAsync(ohist, 0, sizeof(uint32_t) * kOrderMaxBins, s);
+  }
+  return e;
 }
 
 static KernelSel pick_kernel(int fht, int mode, int d, bool tc_only) {
@@ -326,53 +410,19 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   const int groups = grid * (kBThreads / (F < 32 ? 1 : F / 32));
   const long long list_cap = big ? (long long)L * mmax : 0;
   const long long probe_cap = big ? rq.qprobes_max : 0;
-  const long long heap_cap = split ? (long long)nsm * 64 * std::max(mmax, 1) : 0;  // pair heaps of the hash kernel
-  // (re)allocate per-block scratch when the shape grows, in one piece
-  if (!bw.bitset || bw.grid < grid || bw.nwords != nwords || bw.cap < cap || bw.fht < F || bw.mmax < mmax ||
-      bw.list_cap < list_cap || bw.probe_cap < probe_cap || bw.hheap_cap < heap_cap) {
-    bw.release();
-    Slab slab;
-    slab.reserve(&bw.bitset, (size_t)grid * nwords);
-    slab.reserve(&bw.uniq, (size_t)grid * cap);
-    slab.reserve(&bw.score, (size_t)grid * cap);
-    slab.reserve(&bw.gdump, (size_t)groups * F);
-    slab.reserve(&bw.gheap_v, (size_t)groups * std::max(mmax, 1));
-    slab.reserve(&bw.gheap_i, (size_t)groups * std::max(mmax, 1));
-    slab.reserve(&bw.counters, 1);
-    if (heap_cap) {
-      slab.reserve(&bw.hheap_v, heap_cap);
-      slab.reserve(&bw.hheap_i, heap_cap);
-    }
-    if (big) {
-      const size_t gl = (size_t)grid * list_cap, gp = (size_t)grid * probe_cap;
-      const size_t gg = (size_t)groups * 2 * (kBigM1 + 1), gr = (size_t)groups * kBigM1;
-      slab.reserve(&bw.glv, gl);
-      slab.reserve(&bw.glb, gl);
-      slab.reserve(&bw.gprobe, gp);
-      slab.reserve(&bw.gpo, gp);
-      slab.reserve(&bw.gpe, gp);
-      slab.reserve(&bw.ggv, gg);
-      slab.reserve(&bw.ggc, gg);
-      slab.reserve(&bw.grhv, gr);
-      slab.reserve(&bw.grhi, gr);
-    }
-    if ((e = slab.alloc(&bw.slab)) != cudaSuccess) {
-      bw = BatchWorkspace();
-      return fail(e, "alloc");
-    }
-    if ((e = cudaMemsetAsync(bw.bitset, 0, sizeof(uint32_t) * (size_t)grid * nwords, s)) != cudaSuccess)
-      return fail(e, "memset");
-    if ((e = cudaMemsetAsync(bw.counters, 0, sizeof(BatchCounters), s)) != cudaSuccess) return fail(e, "memset");
-    bw.hheap_cap = heap_cap;
-    bw.list_cap = list_cap;
-    bw.probe_cap = probe_cap;
-    bw.grid = grid;
-    bw.nwords = nwords;
-    bw.cap = cap;
-    bw.fht = F;
-    bw.mmax = std::max(mmax, 1);
+  BatchWorkspace::Block blk;
+  blk.bits = grid * nwords;
+  blk.uniq = grid * cap;
+  blk.dump = (long long)groups * F;
+  blk.heap = (long long)groups * std::max(mmax, 1);
+  if (split) blk.hheap = (long long)nsm * 64 * std::max(mmax, 1);  // pair heaps of the hash kernel
+  if (big) {
+    blk.list = grid * list_cap;
+    blk.probe = grid * probe_cap;
+    blk.layer = (long long)groups * 2 * (kBigM1 + 1);
+    blk.replay = (long long)groups * kBigM1;
   }
-  grid = std::min(grid, bw.grid);
+  if ((e = bw.grow_block(blk, s)) != cudaSuccess) return fail(e, "alloc");
   const long long ext_stride = (long long)L * std::max(mmax, 1);
   // The verified hash: its GEMM and its check take about 40 us however few the
   // queries; the exact one gives a group of 8 lanes to every (query, table), 12
@@ -383,38 +433,15 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
                      2 * rq.qprobes_max <= L && (rq.nq > 256 || (long long)rq.nq * L > 4LL * 64 * nsm);
   // scratch of its GEMM, for up to 32,768 queries at a time (66 MB at 100 tables of 256)
   const long long hash_nq = vhash && di.hmat ? std::min<long long>(rq.nq, 32768) : 0;
-  const long long hash_need = hash_nq * 2 * L * (D / 128), hq_need = hash_nq * hmat_ld(d);
   // per-batch buffers: lists of the hash, processing order, probe cuts
   const bool pcut = split && !big;
-  const long long ext_need = split ? (long long)rq.nq * ext_stride : 0;
-  const long long pc_need = pcut ? (long long)rq.nq * rq.qprobes_max : 0;
-  if (!bw.bslab || bw.batch_cap < rq.nq || bw.ext_cap < ext_need || bw.pc_cap < pc_need || bw.hash_cap < hash_need ||
-      bw.hq_cap < hq_need) {
-    cudaFree(bw.bslab);
-    bw.batch_cap = bw.ext_cap = bw.pc_cap = bw.hash_cap = bw.hq_cap = 0;
-    Slab slab;
-    slab.reserve(&bw.okey, (size_t)rq.nq);
-    slab.reserve(&bw.order, (size_t)rq.nq);
-    slab.reserve(&bw.ohist, (size_t)kOrderMaxBins);
-    slab.reserve(&bw.ext_lv, (size_t)ext_need);
-    slab.reserve(&bw.ext_lb, (size_t)ext_need);
-    slab.reserve(&bw.pc_g, (size_t)pc_need);
-    slab.reserve(&bw.pc_o, (size_t)pc_need);
-    slab.reserve(&bw.pc_pe, (size_t)pc_need);
-    slab.reserve(&bw.pc_n, (size_t)rq.nq);
-    if (hash_need) {
-      slab.reserve(&bw.hq, (size_t)hq_need);
-      slab.reserve(&bw.htmax, (size_t)hash_need);
-    }
-    if ((e = slab.alloc(&bw.bslab)) != cudaSuccess) return fail(e, "alloc");
-    if ((e = cudaMemsetAsync(bw.ohist, 0, sizeof(uint32_t) * kOrderMaxBins, s)) != cudaSuccess)
-      return fail(e, "memset");
-    bw.batch_cap = rq.nq;
-    bw.ext_cap = ext_need;
-    bw.pc_cap = pc_need;
-    bw.hash_cap = hash_need;
-    bw.hq_cap = hq_need;
-  }
+  BatchWorkspace::Batch bat;
+  bat.nq = rq.nq;
+  bat.ext = split ? (long long)rq.nq * ext_stride : 0;
+  bat.pc = pcut ? (long long)rq.nq * rq.qprobes_max : 0;
+  bat.hash = hash_nq * 2 * L * (D / 128);
+  bat.hq = hash_nq * hmat_ld(d);
+  if ((e = bw.grow_batch(bat, s)) != cudaSuccess) return fail(e, "alloc");
   if (split) {
     const long long max_groups = (long long)nsm * 64;
     if (rq.stage_timing) {
@@ -586,14 +613,14 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   a.out_stride = rq.out_stride;
   a.out_v = rq.out_v;
   a.bitset = bw.bitset;
-  a.nwords = bw.nwords;
+  a.nwords = nwords;
   a.uniq = bw.uniq;
   a.score = bw.score;
-  a.cap = bw.cap;
+  a.cap = cap;
   a.gdump = bw.gdump;
   a.gheap_v = bw.gheap_v;
   a.gheap_i = bw.gheap_i;
-  a.mmax = bw.mmax;
+  a.mmax = std::max(mmax, 1);
   a.work = &bw.counters->work;
   a.status = &bw.counters->status;
   a.totals = totals;
@@ -601,11 +628,11 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   a.tflips = (!big && rq.tc_rotation && rq.mode != kRowsF32 && F == 256) ? di.tflips : nullptr;
   a.glv = bw.glv;
   a.glb = bw.glb;
-  a.list_cap = bw.list_cap;
+  a.list_cap = list_cap;
   a.gprobe = bw.gprobe;
   a.gpo = bw.gpo;
   a.gpe = bw.gpe;
-  a.probe_cap = bw.probe_cap;
+  a.probe_cap = probe_cap;
   a.ggv = bw.ggv;
   a.ggc = bw.ggc;
   a.grhv = bw.grhv;
@@ -653,10 +680,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     res.graph_replayed = true;
   } else {
     if (can_graph) {
-      if (bw.graph_exec) {
-        cudaGraphExecDestroy(bw.graph_exec);
-        bw.graph_exec = nullptr;
-      }
+      bw.drop_graph();
       cudaGraph_t graph = nullptr;
       if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return fail(e, "capture");
       cudaMemsetAsync(bw.counters, 0, sizeof(unsigned) * 2, s);
@@ -671,7 +695,6 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
           if (cudaGraphNodeGetType(nodes[i], &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) bw.graph_knode = nodes[i];
         }
       e = cudaGraphInstantiate(&bw.graph_exec, graph, 0);
-      if (bw.graph) cudaGraphDestroy(bw.graph);
       bw.graph = graph;  // kept alive: the kernel node handle belongs to it
       if (e != cudaSuccess) {
         bw.graph_exec = nullptr;

@@ -73,34 +73,40 @@ struct BatchResult {
   long long tc_exact = 0;           // with stage_timing: tables the verified hash re-hashed in FP32
 };
 
-// Per-block scratch of the batched kernel (kept between calls) and the cached graph.
+// Scratch of the batched kernels, kept between calls, and the cached graph.
+// Strides follow from each call's own shape; what is kept is room, in elements
+// per array, and every array only grows, so calls of changing shapes settle on
+// one allocation (cudaFree waits for the whole device).
 struct BatchWorkspace {
-  unsigned char* slab = nullptr;   // the per-block scratch and the counters
-  unsigned char* bslab = nullptr;  // the per-batch buffers (order, ext_, pc_)
-  uint32_t* bitset = nullptr;
-  long long nwords = 0;
+  // per-block scratch and the counters
+  struct Block {
+    long long bits = 0, uniq = 0, dump = 0, heap = 0, hheap = 0, list = 0, probe = 0, layer = 0, replay = 0;
+  };
+  // per-batch buffers: queries, list, probe and hash entries
+  struct Batch {
+    long long nq = 0, ext = 0, pc = 0, hash = 0, hq = 0;
+  };
+  unsigned char* slab = nullptr;   // holds `block`
+  unsigned char* bslab = nullptr;  // holds `batch`
+  Block block;
+  Batch batch;
+  uint32_t* bitset = nullptr;  // zero between calls
   uint32_t* uniq = nullptr;
   uint32_t* score = nullptr;
-  long long cap = 0;
   float* gdump = nullptr;
   float* gheap_v = nullptr;
   int* gheap_i = nullptr;
-  int mmax = 0;
-  int fht = 0;
-  int grid = 0;
   BatchCounters* counters = nullptr;
   // query order: key per query, histogram of the keys, the permutation
   uint32_t* okey = nullptr;
-  uint32_t* ohist = nullptr;
+  uint32_t* ohist = nullptr;  // zero between calls
   uint32_t* order = nullptr;
   // big-list form scratch (see BatchArgs)
   float* glv = nullptr;
   uint32_t* glb = nullptr;
-  long long list_cap = 0;
   uint32_t* gprobe = nullptr;
   uint32_t* gpo = nullptr;
   uint32_t* gpe = nullptr;
-  long long probe_cap = 0;
   float* ggv = nullptr;
   int* ggc = nullptr;
   float* grhv = nullptr;
@@ -108,15 +114,12 @@ struct BatchWorkspace {
   // split hash: per-query lists and the hash kernel's pair-heap scratch
   float* ext_lv = nullptr;
   uint32_t* ext_lb = nullptr;
-  long long batch_cap = 0, ext_cap = 0, pc_cap = 0;  // queries, list and probe entries that bslab holds
+  float* hheap_v = nullptr;
+  int* hheap_i = nullptr;
   // verified hash with the rotations as matrices: FP16 queries, magnitudes
   uint16_t* hq = nullptr;
   float* htmax = nullptr;
-  long long hash_cap = 0, hq_cap = 0;
-  float* hheap_v = nullptr;
-  int* hheap_i = nullptr;
-  long long hheap_cap = 0;
-  // split hash with small lists: k_probe_cut's output per processing slot
+  // split hash with small lists: k_probe_cut's output per query
   uint32_t* pc_g = nullptr;
   uint32_t* pc_o = nullptr;
   uint32_t* pc_pe = nullptr;
@@ -133,6 +136,11 @@ struct BatchWorkspace {
   cudaStream_t graph_stream = nullptr;
   std::vector<unsigned char> graph_args;
   void release();
+  void drop_graph();
+  // Room for at least these: with what is held already where it fits in memory,
+  // else for these alone (the other shapes' room is given back).
+  cudaError_t grow_block(const Block& need, cudaStream_t s);
+  cudaError_t grow_batch(const Batch& need, cudaStream_t s);
 };
 
 // Scratch of the brute-force low-precision block kernels (fpp_bf_lowp.cu):

@@ -53,3 +53,42 @@ def test_graph_after_calls_that_move_buffers_within_the_allocation(form, nq, qp)
             _batched(g, dq, nq, 10, qp, small)
         assert np.array_equal(_batched(g, dq, 600, 10, 6, ids), first)
     g.close()
+
+
+def test_calls_of_changing_shape_settle_on_one_allocation():
+    # few queries with many candidates and long lists, many with few, big lists,
+    # mixed batches, plain and batched, in turn: after one round of all of them
+    # nothing is allocated any more (an allocation would fail here), and every
+    # result stays the first round's
+    import torch
+    Q = synth.mixture(2000, 64, n_centres=16, seed=1)
+    dq = torch.from_numpy(Q).cuda()
+    qps = torch.from_numpy(np.random.default_rng(0).integers(1, 41, 2000).astype(np.int32)).cuda()
+    ids = torch.zeros((2000, 10), dtype=torch.int32, device="cuda")
+    g = _index()
+
+    def device(nq, qp, mixed=False, graph=0):
+        g.set_query_form(1, 2, 4)
+        g.set_option("use_graph", graph)
+        ids.fill_(-7)
+        torch.cuda.synchronize()
+        g.query_batched(dq.data_ptr(), nq, None, qps.data_ptr() if mixed else None, 10, qp, ids.data_ptr(), 10)
+        return ids.cpu().numpy().copy()
+
+    def plain(nq, qp):
+        g.set_query_form(0, 0, 4)
+        g.set_qprobes(qp)
+        return g.query(Q[:nq], 10)
+
+    calls = [lambda: device(1, 60), lambda: device(2000, 2), lambda: device(900, 40, mixed=True),
+             lambda: device(30, 1500), lambda: plain(1, 1100), lambda: plain(2000, 3),
+             lambda: device(1000, 6, graph=1), lambda: device(223, 25), lambda: plain(300, 6)]
+    first = [c() for c in calls]
+    try:
+        for order in (range(len(calls)), reversed(range(len(calls)))):
+            for i in order:
+                g.set_option("inject_alloc_failure", 1)
+                assert np.array_equal(calls[i](), first[i]), i
+    finally:
+        g.set_option("inject_alloc_failure", 0)
+    g.close()

@@ -4,7 +4,7 @@
 //   1. centring: per-dimension chunked FP32 sums -> mean -> x - mean, stored
 //      point-major in HBM (FalconnPP.cpp:33-34);
 //   2. k_build_hash: one group of FHT/32 lanes per point holds the point in
-//      registers and, for every table of the chunk, runs 2 layers x 3 x
+//      shared memory and, for every table of the chunk, runs 2 layers x 3 x
 //      (sign flip + shuffle FWHT), picks the top-iProbes cross-polytope codes
 //      per layer and combines the two layers (FalconnPP.cpp:75-201).  Each
 //      (table, point) emits iProbes (bucket, score, id) entries;
@@ -12,9 +12,9 @@
 //      min(bucket_minSize, B) (FalconnPP.cpp:233-242), give CSR offsets, and
 //      the bucket sizes the places of a chunk's entries, bucket by bucket;
 //   4. every entry goes to its bucket's place, then each bucket is sorted by
-//      (score desc, id asc) on its own (a warp for up to 32 entries, a block's
-//      shared memory above), replacing the per-bucket max-heaps; its first
-//      iLimit ids are the 1D table's;
+//      (score desc, id asc) on its own (a warp for up to 512 entries, a block's
+//      shared memory for up to 8,192, tiles and merge passes above), replacing
+//      the per-bucket max-heaps; its first iLimit ids are the 1D table's;
 //   5. where equal scores make the reference's heap order differ from
 //      (score desc, id asc) — ties at the iLimit cut, and (by default) ties
 //      inside the kept prefix — k_repair replays the reference's max-heap on
@@ -492,6 +492,7 @@ struct ScanArgs {
   unsigned long long* base;   // in: ids before this chunk; out: after
   unsigned int* max_kept;
   unsigned long long* n_limited;
+  unsigned long long* max_count;  // entries of the chunk's largest bucket
 };
 
 constexpr int kScanThreads = 1024;
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(ScanArgs a) {
   __shared__ long long tmp[32];
   const long long t0 = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   long long sc = 0, sk = 0, lim = 0;
-  unsigned mk = 0;
+  unsigned mk = 0, mc = 0;
   for (int i = 0; i < kScanItems; ++i) {
     const long long g = t0 + i;
     if (g < a.nb) {
@@ -513,6 +514,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(ScanArgs a) {
       sk += k;
       lim += limited;
       mk = max(mk, k);
+      mc = max(mc, B);
     }
   }
   long long tc, tk;
@@ -526,6 +528,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(ScanArgs a) {
     atomicAdd(a.n_limited, (unsigned long long)tl);
   }
   if (mk) atomicMax(a.max_kept, mk);
+  mc = __reduce_max_sync(kFullMask, mc);
+  if ((threadIdx.x & 31) == 0 && mc) atomicMax(a.max_count, (unsigned long long)mc);
 }
 
 // single block: exclusive scan of the block sums, adds the running base
@@ -603,11 +607,14 @@ struct BucketArgs {
   int exact_order;
   uint64_t* seg;
   int32_t* ids;
-  // work lists of the chunk: buckets of 33 to kMediumCap entries, larger ones,
-  // and the buckets to repair now, by size class; counters: [0] medium, [1]
-  // large, [2] next large, [3 + c] repairs of class c
+  // work lists of the chunk: buckets of 33 to kMediumCap entries, of up to
+  // kTileCap, and larger ones with the tiles that make them up, and the buckets
+  // to repair now, by size class; counters: [0] medium, [1] large, [2] next
+  // large, [3 + c] repairs of class c, [6] tiles, [7] huge
   uint32_t* medium;
   uint32_t* large;
+  uint32_t* huge;
+  uint2* tiles;  // bucket, tile
   uint32_t* repair[3];
   unsigned* counters;
   unsigned long long* n_repaired;  // over all chunks
@@ -627,6 +634,7 @@ struct RepairItem {
 };
 
 constexpr unsigned kMediumCap = 512;
+constexpr unsigned kTileCap = 8192;  // entries a block sorts in shared memory (64 KB, three blocks per SM)
 constexpr unsigned kArenaEntries = 1u << 23;
 constexpr unsigned kRepairItems = 1u << 16;  // per class
 
@@ -698,7 +706,7 @@ __global__ void __launch_bounds__(256) k_bucket_small(BucketArgs a) {
   }
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const bool in = kp && B > 32 && (B > kMediumCap) == (c == 1);
+    const bool in = kp && B > 32 && B <= kTileCap && (B > kMediumCap) == (c == 1);
     const unsigned bal = __ballot_sync(kFullMask, in);
     if (bal) {
       unsigned at = 0;
@@ -706,6 +714,11 @@ __global__ void __launch_bounds__(256) k_bucket_small(BucketArgs a) {
       at = __shfl_sync(kFullMask, at, 0) + __popc(bal & ((1u << lane) - 1u));
       if (in) (c ? a.large : a.medium)[at] = b;
     }
+  }
+  if (kp && B > kTileCap) {
+    a.huge[atomicAdd(a.counters + 7, 1u)] = b;
+    const unsigned nt = (B - 1) / kTileCap + 1, at = atomicAdd(a.counters + 6, nt);
+    for (unsigned t = 0; t < nt; ++t) a.tiles[at + t] = make_uint2(b, t);
   }
   if (kp && B == 1) a.ids[o] = (int32_t)(uint32_t)a.seg[s0];  // nothing to sort
   unsigned todo = __ballot_sync(kFullMask, kp && B > 1 && B <= 32);
@@ -828,10 +841,28 @@ __device__ __forceinline__ void block_sort_entries(uint64_t* e, int N) {
   __syncthreads();
 }
 
-constexpr int kLargeSmem = 8192;  // entries sorted in shared memory (64 KB, three blocks per SM)
+// The kept ids of a sorted bucket, and its repair where a tie asks for one; by
+// the whole block.
+__device__ __forceinline__ void finish_bucket(const BucketArgs& a, uint32_t b, uint32_t B, const uint64_t* e,
+                                              unsigned* s_pos) {
+  bool limited;
+  const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
+  int32_t* out = a.ids + a.off[b];
+  bool tie = false;
+  for (uint32_t r = threadIdx.x; r < kp; r += 256) {
+    out[r] = (int32_t)(uint32_t)e[r];
+    tie |= tie_matters(a, r, kp, B, e[r], r + 1 < B ? e[r + 1] : 0ull);
+  }
+  if (__syncthreads_or(tie)) {
+    if (threadIdx.x == 0) *s_pos = add_repair(a, b, B, kp, a.off[b]);
+    __syncthreads();
+    const unsigned pos = *s_pos;
+    if (pos != kArenaFull)
+      for (uint32_t i = threadIdx.x; i < B; i += 256) a.arena[pos + i] = e[i];
+  }
+}
 
-// Persistent blocks over the list of larger buckets.  A bucket beyond the
-// shared memory is sorted where it lies, padded steps skipped.
+// Persistent blocks over the list of buckets that fit a block's shared memory.
 __global__ void __launch_bounds__(256) k_bucket_large(BucketArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* sm = reinterpret_cast<uint64_t*>(smem_raw);
@@ -845,52 +876,98 @@ __global__ void __launch_bounds__(256) k_bucket_large(BucketArgs a) {
     if (item >= nl) break;
     const uint32_t b = a.large[item];
     const uint32_t B = a.counts[b];
-    bool limited;
-    const uint32_t kp = kept_of(B, a.alpha, a.P, a.minSize, &limited);
-    uint64_t* g = a.seg + a.segstart[b];
-    int32_t* out = a.ids + a.off[b];
-    uint64_t* e = sm;
-    if (B <= (uint32_t)kLargeSmem) {
-      int N = 64;
-      while (N < (int)B) N <<= 1;
-      for (int i = threadIdx.x; i < N; i += 256) sm[i] = i < (int)B ? g[i] : ~0ull;
-      block_sort_entries(sm, N);
-    } else {
-      // all comparators ascending (mirror form): positions past the end act as
-      // +infinity and never move
-      e = g;
-      uint32_t N = 1;
-      while (N < B) N <<= 1;
-      for (uint32_t k = 2; k <= N; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          __syncthreads();
-          for (uint32_t t = threadIdx.x; t < N / 2; t += 256) {
-            const uint32_t blk = t / j, r = t - blk * j;
-            const uint32_t lo = j == (k >> 1) ? blk * k + r : blk * 2 * j + r;
-            const uint32_t hi = j == (k >> 1) ? blk * k + k - 1 - r : lo + j;
-            if (hi < B) {
-              const uint64_t x = g[lo], y = g[hi];
-              if (x > y) {
-                g[lo] = y;
-                g[hi] = x;
-              }
-            }
-          }
-        }
-      __syncthreads();
+    const uint64_t* g = a.seg + a.segstart[b];
+    int N = 64;
+    while (N < (int)B) N <<= 1;
+    for (int i = threadIdx.x; i < N; i += 256) sm[i] = i < (int)B ? g[i] : ~0ull;
+    block_sort_entries(sm, N);
+    finish_bucket(a, b, B, sm, &s_pos);
+  }
+}
+
+// Buckets beyond that (few codes, or thousands of points in one direction):
+// tiles of kTileCap entries sorted by a block each, then merged in passes over
+// all tiles, so that a bucket's sort takes the whole GPU.  1M x 32, 10 tables
+// of 4 / 16 / 64 buckets, sorts and repairs: 452 / 98 / 32 ms with one block
+// per bucket in global memory, 95 / 23 / 8 ms so (the rest is heap replays).
+__global__ void __launch_bounds__(256) k_tile_sort(BucketArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint64_t* sm = reinterpret_cast<uint64_t*>(smem_raw);
+  const unsigned nt = a.counters[6];
+  for (unsigned item = blockIdx.x; item < nt; item += gridDim.x) {
+    const uint2 it = a.tiles[item];
+    const uint32_t o = it.y * kTileCap;
+    const int m = (int)min(a.counts[it.x] - o, kTileCap);
+    uint64_t* g = a.seg + a.segstart[it.x] + o;
+    int N = 64;
+    while (N < m) N <<= 1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < N; i += 256) sm[i] = i < m ? g[i] : ~0ull;
+    block_sort_entries(sm, N);
+    for (int i = threadIdx.x; i < m; i += 256) g[i] = sm[i];
+  }
+}
+
+// How many of the first k entries of the merge of x[0..nx) and y[0..ny) are x's.
+__device__ __forceinline__ uint32_t merge_split(const uint64_t* x, uint32_t nx, const uint64_t* y, uint32_t ny,
+                                                uint32_t k) {
+  uint32_t lo = k > ny ? k - ny : 0u, hi = min(k, nx);
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (x[mid] < y[k - 1 - mid])
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
+}
+
+// One pass: sorted runs of w entries in pairs, from src to dst; a block writes
+// kTileCap places of its bucket.  Entries of a bucket differ (their ids do), so
+// an entry's place is its index plus its rank in the other run.
+__global__ void __launch_bounds__(256) k_tile_merge(BucketArgs a, const uint64_t* src, uint64_t* dst, uint32_t w) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint64_t* sm = reinterpret_cast<uint64_t*>(smem_raw);
+  __shared__ uint32_t s_split[2];
+  const unsigned nt = a.counters[6];
+  for (unsigned item = blockIdx.x; item < nt; item += gridDim.x) {
+    const uint2 it = a.tiles[item];
+    const uint32_t B = a.counts[it.x], s0 = a.segstart[it.x];
+    const uint32_t o0 = it.y * kTileCap, o1 = o0 + min(B - o0, kTileCap);
+    const uint32_t p0 = (uint32_t)(o0 / (2ull * w) * (2ull * w));  // the pair of runs
+    const uint32_t nx = min(B - p0, w), ny = min(B - p0 - nx, w);
+    const uint64_t* x = src + s0 + p0;
+    const uint64_t* y = x + nx;
+    __syncthreads();
+    if (threadIdx.x < 2) s_split[threadIdx.x] = merge_split(x, nx, y, ny, (threadIdx.x ? o1 : o0) - p0);
+    __syncthreads();
+    const uint32_t x0 = s_split[0], y0 = o0 - p0 - x0;
+    const uint32_t cx = s_split[1] - x0, cy = o1 - o0 - cx;
+    for (uint32_t i = threadIdx.x; i < cx + cy; i += 256) sm[i] = i < cx ? x[x0 + i] : y[y0 + i - cx];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < cx + cy; i += 256) {
+      const uint64_t e = sm[i];
+      uint32_t lo = i < cx ? cx : 0u, hi = i < cx ? cx + cy : cx;  // the other run
+      const uint32_t from = lo;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (sm[mid] < e)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      dst[s0 + o0 + (i < cx ? i : i - cx) + (lo - from)] = e;
     }
-    bool tie = false;
-    for (uint32_t r = threadIdx.x; r < kp; r += 256) {
-      out[r] = (int32_t)(uint32_t)e[r];
-      tie |= tie_matters(a, r, kp, B, e[r], r + 1 < B ? e[r + 1] : 0ull);
-    }
-    if (__syncthreads_or(tie)) {
-      if (threadIdx.x == 0) s_pos = add_repair(a, b, B, kp, a.off[b]);
-      __syncthreads();
-      const unsigned pos = s_pos;
-      if (pos != kArenaFull)
-        for (uint32_t i = threadIdx.x; i < B; i += 256) a.arena[pos + i] = e[i];
-    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_bucket_huge(BucketArgs a, const uint64_t* sorted) {
+  __shared__ unsigned s_pos;
+  const unsigned nh = a.counters[7];
+  for (unsigned item = blockIdx.x; item < nh; item += gridDim.x) {
+    const uint32_t b = a.huge[item];
+    __syncthreads();
+    finish_bucket(a, b, a.counts[b], sorted + a.segstart[b], &s_pos);
   }
 }
 
@@ -937,16 +1014,27 @@ __device__ __forceinline__ void bucket_pop(uint2* h, int& n) {
   --n;
 }
 
-// One warp per bucket, its heap in CAP entries of shared memory (class 2: in
-// the seg array itself): the entries back in push order (ascending id,
-// FalconnPP.cpp:75 / :200), then lane 0 replays the priority_queue pushes and
-// the first iLimit pops (FalconnPP.cpp:226-230).  A replay is one chain of
-// dependent loads (about 45 clocks per level); the SM runs as many as fit its
-// shared memory.
+// One warp per bucket, its heap in CAP entries of shared memory (class 2: a
+// block of 1,024 threads, and the seg array itself): the entries back in push
+// order (ascending id, FalconnPP.cpp:75 / :200), then one thread replays the
+// priority_queue pushes and the first iLimit pops (FalconnPP.cpp:226-230).  A
+// replay is one chain of dependent loads (about 45 clocks per level); the SM
+// runs as many as fit its shared memory.  100,000 equal points, 10
+// tables: 16 ms; 75 ms with one warp here and one block per bucket's sort.
 template <int CLS>
-__global__ void __launch_bounds__(32) k_repair(BucketArgs a, bool deferred) {
+constexpr int kRepairThreads = CLS == 2 ? 1024 : 32;
+
+template <int CLS>
+__global__ void __launch_bounds__(kRepairThreads<CLS>) k_repair(BucketArgs a, bool deferred) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr uint32_t T = kRepairThreads<CLS>;
   const int lane = threadIdx.x;
+  auto sync = [] {
+    if constexpr (CLS == 2)
+      __syncthreads();
+    else
+      __syncwarp();
+  };
   const unsigned nrep = deferred ? a.deferred[1 + CLS] : a.counters[3 + CLS];
   for (unsigned r = blockIdx.x; r < nrep; r += gridDim.x) {
     uint32_t B, kp;
@@ -968,16 +1056,16 @@ __global__ void __launch_bounds__(32) k_repair(BucketArgs a, bool deferred) {
     }
     // entries as (id << 32) | score bits, slot i at e[i + 1]
     uint64_t* e = CLS == 2 ? g - 1 : reinterpret_cast<uint64_t*>(smem_raw);
-    for (uint32_t i = lane; i < B; i += 32) {
+    for (uint32_t i = lane; i < B; i += T) {
       const uint64_t x = g[i];
       e[i + 1] = (x << 32) | ord_key_inv_dev(~(uint32_t)(x >> 32));
     }
-    __syncwarp();
+    sync();
     uint32_t N = 1;
     while (N < B) N <<= 1;
-    for (uint32_t k = 2; k <= N; k <<= 1)
+    for (uint32_t k = 2; k && k <= N; k <<= 1)  // (k wraps to 0 past 2^31)
       for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-        for (uint32_t t = lane; t < N / 2; t += 32) {
+        for (uint32_t t = lane; t < N / 2; t += T) {
           const uint32_t q = t & ~(j - 1), o = t & (j - 1);  // q = j * block
           const uint32_t lo = 2 * q + o;
           const uint32_t hi = j == (k >> 1) ? 2 * q + k - 1 - o : lo + j;
@@ -989,7 +1077,7 @@ __global__ void __launch_bounds__(32) k_repair(BucketArgs a, bool deferred) {
             }
           }
         }
-        __syncwarp();
+        sync();
       }
     if (lane == 0) {
       if constexpr (CLS == 2) {
@@ -1045,7 +1133,7 @@ __global__ void __launch_bounds__(32) k_repair(BucketArgs a, bool deferred) {
         }
       }
     }
-    __syncwarp();
+    sync();
   }
 }
 
@@ -1094,7 +1182,7 @@ static cudaError_t dispatch_hash(int fht, const HashArgs& a, int nsm, cudaStream
 
 // The largest class first: its chains are the longest.
 static void launch_repairs(const BucketArgs& a, int nsm, bool deferred, cudaStream_t s) {
-  k_repair<2><<<(unsigned)nsm * 4, 32, 0, s>>>(a, deferred);
+  k_repair<2><<<(unsigned)nsm * 2, kRepairThreads<2>, 0, s>>>(a, deferred);
   k_repair<1><<<(unsigned)nsm * 4, 32, (kRepairCap[1] + 2) * 8, s>>>(a, deferred);
   k_repair<0><<<(unsigned)nsm * 28, 32, (kRepairCap[0] + 2) * 8, s>>>(a, deferred);
 }
@@ -1176,6 +1264,8 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   uint32_t* segstart = nullptr;
   uint32_t* medium = nullptr;
   uint32_t* large = nullptr;
+  uint32_t* huge = nullptr;
+  uint2* tiles = nullptr;
   uint64_t* arena = nullptr;
   RepairItem* items[3] = {nullptr, nullptr, nullptr};
   unsigned* deferred = nullptr;
@@ -1183,13 +1273,15 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   unsigned* counters = nullptr;
   unsigned long long* blk_cnt = nullptr;
   unsigned long long* blk_kept = nullptr;
-  unsigned long long* totals = nullptr;  // ids before the next chunk, limited buckets, repaired buckets
+  // ids before the next chunk, limited buckets, repaired buckets, the chunk's largest bucket
+  unsigned long long* totals = nullptr;
   unsigned int* d_maxkept = nullptr;
   BucketArgs ba;
   int32_t* ids_cap = nullptr;
   uint64_t ids_capacity = 0;
   int h_bad = 0;
-  unsigned long long h_base = 0;
+  unsigned long long h_totals[4] = {0, 0, 0, 0};
+  unsigned long long& h_base = h_totals[0];
   // 2^24 entries a chunk (336 MB of scratch; the buckets' entries, 134 MB,
   // about fill L2): larger chunks only cost memory
   const long long entry_cap = 1LL << 24;
@@ -1224,10 +1316,13 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     slab.reserve(&ranks, max_entries);
     slab.reserve(&seg, max_entries);
     slab.reserve(&segstart, nb_chunk_max);
-    // buckets of more than 32 and kMediumCap entries, and those that can need
-    // a repair (two entries or more; by class, more than its lower end)
+    // buckets of more than 32, kMediumCap and kTileCap entries (the last with
+    // their tiles), and those that can need a repair (two entries or more; by
+    // class, more than its lower end)
     slab.reserve(&medium, std::min(nb_chunk_max, max_entries / 33) + 1);
     slab.reserve(&large, std::min(nb_chunk_max, max_entries / (long long)kMediumCap) + 1);
+    slab.reserve(&huge, max_entries / kTileCap + 1);
+    slab.reserve(&tiles, 2 * (max_entries / kTileCap) + 1);
     slab.reserve(&repair[0], std::min(nb_chunk_max, max_entries / 2) + 1);
     slab.reserve(&repair[1], std::min(nb_chunk_max, max_entries / kRepairCap[0]) + 1);
     slab.reserve(&repair[2], std::min(nb_chunk_max, max_entries / kRepairCap[1]) + 1);
@@ -1237,7 +1332,7 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     slab.reserve(&counters, 8);
     slab.reserve(&blk_cnt, nblk_max);
     slab.reserve(&blk_kept, nblk_max);
-    slab.reserve(&totals, 3);
+    slab.reserve(&totals, 4);
     slab.reserve(&d_maxkept, 1);
     FPP_CUDA(slab.alloc(&scratch));
   }
@@ -1274,9 +1369,11 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
 
   // 3. hash + sort + compact, a chunk of tables at a time
   FPP_CUDA(cudaMemsetAsync(deferred, 0, sizeof(unsigned) * 4, s));
-  FPP_CUDA(cudaMemsetAsync(totals, 0, sizeof(unsigned long long) * 3, s));
+  FPP_CUDA(cudaMemsetAsync(totals, 0, sizeof(unsigned long long) * 4, s));
   FPP_CUDA(cudaMemsetAsync(d_maxkept, 0, sizeof(unsigned int), s));
-  FPP_CUDA(cudaFuncSetAttribute(k_bucket_large, cudaFuncAttributeMaxDynamicSharedMemorySize, kLargeSmem * 8));
+  FPP_CUDA(cudaFuncSetAttribute(k_bucket_large, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileCap * 8));
+  FPP_CUDA(cudaFuncSetAttribute(k_tile_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileCap * 8));
+  FPP_CUDA(cudaFuncSetAttribute(k_tile_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileCap * 8));
   FPP_CUDA(cudaFuncSetAttribute(k_repair<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(kRepairCap[1] + 2) * 8));
 
@@ -1323,12 +1420,14 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     sa.base = totals;
     sa.max_kept = d_maxkept;
     sa.n_limited = totals + 1;
+    sa.max_count = totals + 3;
+    FPP_CUDA(cudaMemsetAsync(totals + 3, 0, sizeof(unsigned long long), s));
     const long long nblk = (nbc + kScanTile - 1) / kScanTile;
     k_scan_reduce<<<(unsigned)nblk, kScanThreads, 0, s>>>(sa);
     k_scan_blocks<<<1, kScanThreads, 0, s>>>(sa, nblk);
     k_scan_down<<<(unsigned)nblk, kScanThreads, 0, s>>>(sa);
     FPP_CUDA(cudaGetLastError());
-    FPP_CUDA(cudaMemcpyAsync(&h_base, totals, sizeof(h_base), cudaMemcpyDeviceToHost, s));
+    FPP_CUDA(cudaMemcpyAsync(h_totals, totals, sizeof(h_totals), cudaMemcpyDeviceToHost, s));
     FPP_CUDA(cudaStreamSynchronize(s));
     if (h_base >= (1ULL << 32)) {
       err.code = kErrUnsupported;
@@ -1369,6 +1468,8 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     ba.ids = ids_cap;
     ba.medium = medium;
     ba.large = large;
+    ba.huge = huge;
+    ba.tiles = tiles;
     ba.arena = arena;
     for (int c = 0; c < 3; ++c) ba.items[c] = items[c];
     ba.deferred = deferred;
@@ -1380,8 +1481,20 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     FPP_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned) * 8, s));
     k_bucket_scatter<<<(unsigned)((Ne + 255) / 256), 256, 0, s>>>(ba);
     k_bucket_small<<<(unsigned)((nbc + 255) / 256), 256, 0, s>>>(ba);
-    k_bucket_large<<<(unsigned)nsm * 3, 256, kLargeSmem * 8, s>>>(ba);
+    k_bucket_large<<<(unsigned)nsm * 3, 256, kTileCap * 8, s>>>(ba);
     k_bucket_medium<<<(unsigned)nsm * 6, 256, 0, s>>>(ba);
+    if (h_totals[3] > kTileCap) {
+      // the hashed entries are in their buckets: their array is the other one
+      // of the merges (either holds the buckets' entries in some order, which
+      // is all a repair needs)
+      k_tile_sort<<<(unsigned)nsm * 3, 256, kTileCap * 8, s>>>(ba);
+      uint64_t *src = seg, *dst = keys;
+      for (uint64_t w = kTileCap; w < h_totals[3]; w <<= 1) {
+        k_tile_merge<<<(unsigned)nsm * 3, 256, kTileCap * 8, s>>>(ba, src, dst, (uint32_t)w);
+        std::swap(src, dst);
+      }
+      k_bucket_huge<<<(unsigned)nsm, 256, 0, s>>>(ba, src);
+    }
     launch_repairs(ba, nsm, false, s);
     FPP_CUDA(cudaGetLastError());
     FPP_CUDA(cudaStreamSynchronize(s));

@@ -56,14 +56,15 @@ int derived_fht_dim(int n_features, int n_proj) {
 }
 
 // ---------------------------------------------------------------- centring
-__global__ void k_center_partial(const float* __restrict__ X, long long n, int d, float* __restrict__ part) {
+// xs: floats from one point of X to the next
+__global__ void k_center_partial(const float* __restrict__ X, long long n, int d, int xs, float* __restrict__ part) {
   const int j = blockIdx.y * blockDim.x + threadIdx.x;
   const long long c = blockIdx.x;
   if (j >= d) return;
   const long long i0 = c * kCenterChunk;
   const long long i1 = min(n, i0 + kCenterChunk);
   float s = 0.0f;
-  for (long long i = i0; i < i1; ++i) s = __fadd_rn(s, X[i * d + j]);
+  for (long long i = i0; i < i1; ++i) s = __fadd_rn(s, X[i * xs + j]);
   part[c * d + j] = s;
 }
 
@@ -77,14 +78,15 @@ __global__ void k_center_final(const float* __restrict__ part, long long nchunks
 }
 
 // One warp per row, four consecutive elements per lane and step.  APPLY: Xc =
-// X - mean (row stride ld, zero padded), flag non-finite values; otherwise Xc
-// is read.  With `i8`, the row's int8 copy for the screen of the FP32 form
+// X - mean (row stride ld, zero padded; X, of row stride xs, may be Xc itself:
+// an element is read and then written by one lane), flag non-finite values;
+// otherwise Xc is read.  With `i8`, the row's int8 copy for the screen of the FP32 form
 // (fpp_rows.cuh: head, then rint(x / scale)) and the largest row norm.  Bound
 // by HBM: one read of the row and one write of each copy (550 us at 1M x 200
 // with the int8 copy; an element per thread without it took 721 us).
 template <bool APPLY>
-__global__ void __launch_bounds__(256) k_center_rows(const float* __restrict__ X, long long n, int d, int ld,
-                                                     const float* __restrict__ mean, float* __restrict__ Xc,
+__global__ void __launch_bounds__(256) k_center_rows(const float* X, long long n, int d, int xs, int ld,
+                                                     const float* __restrict__ mean, float* Xc,
                                                      unsigned char* __restrict__ i8, int i8_bytes,
                                                      float* __restrict__ norm_max, int* __restrict__ bad) {
   constexpr int NC = 4;  // float4 chunks per lane held in registers (d <= 512)
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256) k_center_rows(const float* __restrict__ X
   bool nonfinite = false;
   auto centred = [&](long long i, int c) {  // chunk c of row i of X - mean, zero past d
     float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float* p = X + i * d + 4 * c;
+    const float* p = X + i * xs + 4 * c;
     const float* m = mean + 4 * c;
     if (vec) {
       x = __ldg(reinterpret_cast<const float4*>(p));
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(256) k_center_rows(const float* __restrict__ X
   if (i8 && lane == 0) atomicMax(reinterpret_cast<unsigned*>(norm_max), __float_as_uint(nmax));  // >= 0: bits order
 }
 
-cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
+cudaError_t alloc_index(const Params& P, DeviceIndex& di, size_t* left) {
   const size_t n = (size_t)P.n_points, d = (size_t)P.n_features;
   const size_t words = (size_t)2 * P.n_tables * 3 * (P.fhtDim < 32 ? 1 : P.fhtDim / 32);
   const size_t nb = (size_t)P.n_tables * 4 * P.n_proj * P.n_proj;
@@ -185,8 +187,8 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
   // or query needs after them: ids (growing), host data, low-precision rows
   const size_t later = (size_t)8 * P.n_tables * P.iProbes * n + 8 * n * d + ((size_t)1 << 30);
   cudaError_t e = cudaSuccess;
-  size_t have = 0, all = 0;
-  const bool known = cudaMemGetInfo(&have, &all) == cudaSuccess;
+  size_t have = 0;
+  const bool known = dev_mem_free(&have);
   for (bool extra = true;; extra = false) {
     Slab slab;
     slab.reserve(&di.Xc, n * di.ld);
@@ -208,6 +210,7 @@ cudaError_t alloc_index(const Params& P, DeviceIndex& di) {
     }
     if (extra && known && have < slab.bytes() + later) continue;
     e = slab.alloc(&di.slab);
+    if (left) *left = !known ? ~(size_t)0 : have > slab.bytes() ? have - slab.bytes() : 0;
     break;
   }
   return e;
@@ -261,7 +264,7 @@ cudaError_t make_hash_matrix(const Params& P, DeviceIndex& di, cudaStream_t s) {
 void make_screen_rows(const Params& P, DeviceIndex& di, cudaStream_t s) {
   if (!di.Xi8) return;
   cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s);
-  k_center_rows<false><<<1184, 256, 0, s>>>(nullptr, P.n_points, P.n_features, di.ld, nullptr, di.Xc, di.Xi8,
+  k_center_rows<false><<<1184, 256, 0, s>>>(nullptr, P.n_points, P.n_features, 0, di.ld, nullptr, di.Xc, di.Xi8,
                                             i8_row_bytes(P.n_features), di.i8_norm_max, nullptr);
 }
 
@@ -1296,6 +1299,8 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
   const unsigned arena_entries = (unsigned)std::min<unsigned long long>(
       opt.repair_arena > 0 ? std::min<unsigned>(kArenaEntries, opt.repair_arena) : kArenaEntries,
       (unsigned long long)L * n * IP);
+  bool in_place = x_on_device;  // no copy of X beside the index
+  size_t mem_left = 0;          // free beside the index's arrays
   const unsigned max_items =
       opt.repair_items > 0 ? std::min<unsigned>(kRepairItems, opt.repair_items) : kRepairItems;
 
@@ -1305,10 +1310,10 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     err.msg = "build: too many entries per table chunk";
     goto fail;
   }
-  FPP_CUDA(alloc_index(P, di));
-  {
+  FPP_CUDA(alloc_index(P, di, &mem_left));
+  for (;;) {
     Slab slab;
-    if (!x_on_device) slab.reserve(&Xstage, (size_t)n * d);
+    if (!in_place) slab.reserve(&Xstage, (size_t)n * d);
     slab.reserve(&part, (size_t)nchunks_c * d);
     slab.reserve(&d_bad, 1);
     slab.reserve(&counts, nb_chunk_max);
@@ -1334,23 +1339,41 @@ int build_index(const Params& P, const float* X, bool x_on_device, const HostBit
     slab.reserve(&blk_kept, nblk_max);
     slab.reserve(&totals, 4);
     slab.reserve(&d_maxkept, 1);
+    // Host data are copied beside the index (one copy at the link's rate) where
+    // that leaves room for the ids, and for the old ones while they grow;
+    // otherwise straight to their rows, which needs no memory of its own.
+    if (!in_place && mem_left < slab.bytes() + (size_t)8 * L * IP * n) {
+      in_place = true;
+      Xstage = nullptr;
+      continue;
+    }
     FPP_CUDA(slab.alloc(&scratch));
+    break;
   }
 
   // 1. centre
   {
     auto t0 = std::chrono::steady_clock::now();
     const float* Xd = X;
-    if (!x_on_device) {
+    int xs = d;
+    if (Xstage) {
       FPP_CUDA(stage.copy(Xstage, X, sizeof(float) * n * d, s));
       Xd = Xstage;
+    } else if (!x_on_device) {
+      if (ld == d)
+        FPP_CUDA(stage.copy(di.Xc, X, sizeof(float) * n * d, s));
+      else
+        FPP_CUDA(cudaMemcpy2DAsync(di.Xc, sizeof(float) * ld, X, sizeof(float) * d, sizeof(float) * d, n,
+                                   cudaMemcpyHostToDevice, s));
+      Xd = di.Xc;
+      xs = ld;
     }
     FPP_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
     dim3 g1((unsigned)nchunks_c, (unsigned)((d + 255) / 256));
-    k_center_partial<<<g1, 256, 0, s>>>(Xd, n, d, part);
+    k_center_partial<<<g1, 256, 0, s>>>(Xd, n, d, xs, part);
     k_center_final<<<(d + 255) / 256, 256, 0, s>>>(part, nchunks_c, n, d, di.center);
     if (di.Xi8) FPP_CUDA(cudaMemsetAsync(di.i8_norm_max, 0, sizeof(float), s));
-    k_center_rows<true><<<(unsigned)std::max(1, nsm * 8), 256, 0, s>>>(Xd, n, d, ld, di.center, di.Xc, di.Xi8,
+    k_center_rows<true><<<(unsigned)std::max(1, nsm * 8), 256, 0, s>>>(Xd, n, d, xs, ld, di.center, di.Xc, di.Xi8,
                                                                        i8_row_bytes(d), di.i8_norm_max, d_bad);
     FPP_CUDA(cudaGetLastError());
     FPP_CUDA(cudaMemcpyAsync(&h_bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -228,6 +228,7 @@ int set_last_error(int code, const std::string& msg) { return fail(code, msg); }
 int clear_last_error() { return ok(); }
 
 static std::atomic<long long> g_alloc_countdown{0};
+static std::atomic<long long> g_hold_back{0};
 
 cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
   long long c = g_alloc_countdown.load();
@@ -237,8 +238,25 @@ cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
+  if (g_hold_back.load() > 0) {
+    size_t have = 0;
+    if (dev_mem_free(&have) && have < bytes) {
+      *p = nullptr;
+      return cudaErrorMemoryAllocation;
+    }
+  }
   return cudaMalloc(p, bytes);
 }
+
+bool dev_mem_free(size_t* bytes) {
+  size_t have = 0, all = 0;
+  if (cudaMemGetInfo(&have, &all) != cudaSuccess) return false;
+  const size_t held = (size_t)g_hold_back.load();
+  *bytes = have > held ? have - held : 0;
+  return true;
+}
+
+void hold_back_memory(long long bytes) { g_hold_back.store(bytes > 0 ? bytes : 0); }
 
 void arm_alloc_failure(long long nth) { g_alloc_countdown.store(nth > 0 ? nth : 0); }
 }  // namespace fpp
@@ -365,6 +383,9 @@ int fpp_set_option(fpp_index* h, const char* key, long long value) {
   } else if (!strcmp(key, "inject_alloc_failure")) {
     if (value < 0) return fail(FPP_ERR_INVALID_ARGUMENT, "set_option: inject_alloc_failure must be >= 0");
     fpp::arm_alloc_failure(value);
+  } else if (!strcmp(key, "hold_back_memory")) {
+    if (value < 0) return fail(FPP_ERR_INVALID_ARGUMENT, "set_option: hold_back_memory must be >= 0");
+    fpp::hold_back_memory(value);
   } else if (!strcmp(key, "tables_per_chunk")) {
     if (value < 0) return fail(FPP_ERR_INVALID_ARGUMENT, "set_option: tables_per_chunk must be >= 0");
     h->opt.tables_per_chunk = (int)value;

@@ -39,6 +39,13 @@ inline cudaError_t dev_malloc(T** p, size_t bytes) {
 }
 void arm_alloc_failure(long long nth);
 
+// Free device memory as dev_malloc sees it.  hold_back_memory(bytes) makes
+// allocations that would leave less than `bytes` free fail like the driver's
+// own, and this report that much less: a device whose memory others hold, for
+// tests (0: none).  Process-wide.  False if the device does not say.
+bool dev_mem_free(size_t* bytes);
+void hold_back_memory(long long bytes);
+
 // Parameters mirror FalconnPP's members (src/FalconnPP.h:14-39).
 struct Params {
   int n_points = 0;
@@ -129,8 +136,9 @@ void free_index(DeviceIndex& di);
 // The index's arrays whose sizes follow from the parameters, in one allocation
 // (each allocation of the driver's takes a millisecond or so).  The int8
 // screening rows (for d <= 512, the batched form's range) and the hash matrix are part of
-// it; where memory is short, it is made without.
-cudaError_t alloc_index(const Params& P, DeviceIndex& di);
+// it; where memory is short, it is made without.  left (nullable): the memory
+// still free, about.
+cudaError_t alloc_index(const Params& P, DeviceIndex& di, size_t* left = nullptr);
 
 // One allocation cut into 256-byte aligned arrays: reserve() each pointer,
 // then alloc().  All pointers are null after a failure.

@@ -134,7 +134,9 @@ int fpp_get_stats(fpp_index* h, int kind, double* out, int n);
  * hashes in exact FP32 and probes the reference's buckets),
  * "inject_alloc_failure" (test switch, process-wide: n >= 1 makes the n-th
  * device allocation from now on fail once with FPP_ERR_OUT_OF_MEMORY, on the
- * host and without touching the GPU; 0 disarms). */
+ * host and without touching the GPU; 0 disarms), "hold_back_memory" (test
+ * switch, process-wide: device allocations that would leave fewer than this
+ * many bytes free fail, as on a GPU whose memory others hold; 0: none). */
 int fpp_set_option(fpp_index* h, const char* key, long long value);
 
 /* Prints the build report the reference writes to stdout after

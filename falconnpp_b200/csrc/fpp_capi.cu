@@ -80,16 +80,15 @@ int check_query_params(const fpp_index* h, int n_queries, int k) {
   return FPP_OK;
 }
 
-// A plain query that ran out of memory on the batched kernels: their scratch
-// (at most the 2 GiB of plain_through_batch, and the batch's lists) is given
-// back, and the three-kernel path, which sizes its own from the candidates
-// found, takes the call.  With 8 GiB free it was not for want of room.
+// A plain query that ran out of memory on the batched kernels: their scratch is
+// given back, and the three-kernel path, which sizes its own from the
+// candidates found, takes the call.  (A failure that a test armed is reported
+// as it is, so that the error path can be tested.)
 bool plain_falls_back(fpp_index* h, int rc) {
-  if (rc != FPP_ERR_OUT_OF_MEMORY) return false;
+  if (rc != FPP_ERR_OUT_OF_MEMORY || fpp::alloc_failure_was_armed()) return false;
   cudaGetLastError();
   h->bw.release();
-  size_t have = 0, all = 0;
-  return cudaMemGetInfo(&have, &all) == cudaSuccess && have < ((size_t)8 << 30);
+  return true;
 }
 
 std::string int2str(int x) {
@@ -229,11 +228,13 @@ int clear_last_error() { return ok(); }
 
 static std::atomic<long long> g_alloc_countdown{0};
 static std::atomic<long long> g_hold_back{0};
+static thread_local bool t_armed_failure = false;
 
 cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
   long long c = g_alloc_countdown.load();
   while (c > 0 && !g_alloc_countdown.compare_exchange_weak(c, c - 1)) {
   }
+  t_armed_failure = c == 1;
   if (c == 1) {  // this is the armed allocation: fail it on the host
     *p = nullptr;
     return cudaErrorMemoryAllocation;
@@ -257,6 +258,8 @@ bool dev_mem_free(size_t* bytes) {
 }
 
 void hold_back_memory(long long bytes) { g_hold_back.store(bytes > 0 ? bytes : 0); }
+
+bool alloc_failure_was_armed() { return t_armed_failure; }
 
 void arm_alloc_failure(long long nth) { g_alloc_countdown.store(nth > 0 ? nth : 0); }
 }  // namespace fpp

@@ -38,6 +38,7 @@ inline cudaError_t dev_malloc(T** p, size_t bytes) {
   return dev_malloc_bytes(reinterpret_cast<void**>(p), bytes);
 }
 void arm_alloc_failure(long long nth);
+bool alloc_failure_was_armed();  // whether this thread's last allocation was the armed one
 
 // Free device memory as dev_malloc sees it.  hold_back_memory(bytes) makes
 // allocations that would leave less than `bytes` free fail like the driver's

@@ -62,3 +62,35 @@ def test_host_build_needs_no_more_than_a_device_build(handle, d):
     assert fits(lambda: g.build(X), hi + (8 << 20))
     for a, b in zip(want, (g.dump_center(), *g.dump_tables()), strict=True):
         assert np.array_equal(a, b)
+
+
+def test_plain_query_whose_batched_scratch_does_not_fit(handle):
+    # one bucket of nearly all points makes the fused kernel's per-block lists
+    # large (they allow for qProbes of the largest), the candidates found are few
+    X = synth.mixture(200_000, 32, n_centres=64, seed=0)
+    X[:150_000] = X[0] * np.random.default_rng(0).uniform(0.5, 1.5, (150_000, 1)).astype(np.float32)
+    Q = synth.mixture(2000, 32, n_centres=64, seed=1)
+    Q = Q[Q @ X[0] < 0][:500]
+    g = handle(X, 10, 64, 20_000, 0.05, 1)
+    g.build(X)
+    g.set_qprobes(8)
+    want = g.query(Q, 10)
+    batched = g.stats(1)
+    _budget(g, 8 << 20)
+    assert np.array_equal(g.query(Q, 10), want)  # the workspace is there
+    g.clear()
+    _budget(g, None)
+    g.build(X)
+    g.set_qprobes(8)
+    import torch
+    q = torch.from_numpy(Q).cuda()
+    out = torch.full((500, 10), -7, dtype=torch.int32, device="cuda")
+    _budget(g, 200 << 20)
+    got = g.query(Q, 10)
+    stats = g.stats(1)
+    g.query_device(q.data_ptr(), 500, 10, out.data_ptr())
+    _budget(g, None)
+    # 8 bytes a candidate for qProbes of the largest bucket, 444 blocks: it cannot have been the fused kernel
+    assert 8 * 8 * g.info()["max_kept"] * 444 > 200 << 20
+    assert np.array_equal(got, want) and np.array_equal(out.cpu().numpy(), want)
+    assert np.array_equal(stats[:4], batched[:4])  # candidates, unique, empty, probes

@@ -198,10 +198,11 @@ class Index:
                                               ctypes.c_void_p(stream or 0)))
 
     def info(self) -> dict:
-        v = np.zeros(9, np.int64)
-        _check(lib().fpp_get_info(self.h, _ptr(v), 9))
+        v = np.zeros(11, np.int64)
+        _check(lib().fpp_get_info(self.h, _ptr(v), 11))
         return dict(fhtDim=int(v[0]), n_ids=int(v[1]), max_kept=int(v[2]), n_buckets=int(v[3]), built=bool(v[4]),
-                    device=int(v[5]), n_tables=int(v[6]), n_proj=int(v[7]), iProbes=int(v[8]))
+                    device=int(v[5]), n_tables=int(v[6]), n_proj=int(v[7]), iProbes=int(v[8]),
+                    screen_rows=bool(v[9]), hash_matrix=bool(v[10]))
 
     def stats(self, kind: int) -> np.ndarray:
         v = np.zeros(11, np.float64)

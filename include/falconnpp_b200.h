@@ -86,7 +86,11 @@ const char* fpp_last_error(void);
 
 /* Index facts: out[0] fhtDim, out[1] stored ids, out[2] largest stored bucket,
  * out[3] buckets (n_tables * 4 * n_proj^2), out[4] built (0/1), out[5] device,
- * out[6] n_tables, out[7] n_proj, out[8] iProbes (the first n are written). */
+ * out[6] n_tables, out[7] n_proj, out[8] iProbes, out[9] the index holds the
+ * int8 rows that screen FP32 candidates, out[10] and the rotations as matrices
+ * for the query hash (0/1; both are left out where memory is short or the sizes
+ * do not allow them: the results are the same, the queries slower).  The first
+ * n are written. */
 int fpp_get_info(fpp_index* h, long long* out, int n);
 
 /* Statistics of the last build (kind 0) or query (kind 1) as doubles.

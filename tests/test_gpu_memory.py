@@ -64,6 +64,34 @@ def test_host_build_needs_no_more_than_a_device_build(handle, d):
         assert np.array_equal(a, b)
 
 
+def test_index_without_its_optional_arrays(handle, tmp_path):
+    # little memory beside the index: no int8 rows and no hash matrix, the same
+    # results, whether it was built or loaded so
+    X = synth.mixture(30_000, 100, n_centres=16, seed=0)
+    Q = synth.mixture(700, 100, n_centres=16, seed=1)
+    roomy, tight, loaded = (handle(X, 20, 128, 100, 0.05, 2) for _ in range(3))
+    roomy.build(X)
+    roomy.save(str(tmp_path / "index"))
+    _budget(tight, 300 << 20)
+    tight.build(X)
+    loaded.load(str(tmp_path / "index"))
+    _budget(tight, None)
+    assert [roomy.info()[k] for k in ("screen_rows", "hash_matrix")] == [True, True]
+    for g in (tight, loaded):
+        assert [g.info()[k] for k in ("screen_rows", "hash_matrix")] == [False, False]
+        for a, b in zip(roomy.dump_tables(), g.dump_tables(), strict=True):
+            assert np.array_equal(a, b)
+        for nq in (5, 700):
+            for qp in (3, 20):
+                for form in ((0, 0, 4), (1, 0, 4), (1, 1, 2), (1, 2, 2)):
+                    got = []
+                    for h in (roomy, g):
+                        h.set_qprobes(qp)
+                        h.set_query_form(*form)
+                        got.append(h.query(Q[:nq], 10))
+                    assert np.array_equal(*got), (nq, qp, form)
+
+
 def test_plain_query_whose_batched_scratch_does_not_fit(handle):
     # one bucket of nearly all points makes the fused kernel's per-block lists
     # large (they allow for qProbes of the largest), the candidates found are few

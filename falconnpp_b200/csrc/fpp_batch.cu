@@ -503,10 +503,11 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
       e = vhash ? hash_lists_verified(P, di, rq.Q + q0 * d, (int)(q1 - q0), qq, rq.qprobes_max,
                                       bw.ext_lv + q0 * ext_stride, bw.ext_lb + q0 * ext_stride, ext_stride,
                                       rq.stage_timing ? &bw.counters->tc_exact : nullptr,
-                                      HashScratch{bw.hq, bw.htmax, &bw.counters->pipe, hash_nq}, s)
+                                      HashScratch{bw.hq, bw.htmax, &bw.counters->pipe, hash_nq}, s, &res.launches)
                 : hash_lists(P, di, rq.Q + q0 * d, (int)(q1 - q0), qq, rq.qprobes_max, bw.ext_lv + q0 * ext_stride,
                              bw.ext_lb + q0 * ext_stride, ext_stride, bw.hheap_v, bw.hheap_i, max_groups, s);
       if (e != cudaSuccess) return fail(e, "hash kernel");
+      if (!vhash) ++res.launches;
     }
     if (rq.stage_timing) cudaEventRecord(bw.tev[3], s);
   } else if (rq.Q_host) {
@@ -731,7 +732,7 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
         return fail(e, "launch");
     }
   }
-  res.launches = (reorder ? 3 : 1) + (split ? 1 : 0) + (pcut ? 1 : 0);
+  res.launches += (reorder ? 2 : 0) + (pcut ? 1 : 0) + 1;  // beside the hash's
   if (rq.stage_timing) {
     cudaEventRecord(bw.tev[2], s);
     if ((e = cudaEventSynchronize(bw.tev[2])) != cudaSuccess) return fail(e, "stage timing");

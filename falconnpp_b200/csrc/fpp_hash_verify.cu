@@ -542,7 +542,7 @@ long long hash_verified_wave_queries() {
 
 cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const float* Q, int nq, const int* q_qprobes,
                                 int qp_max, float* list_v, uint32_t* list_b, long long stride, unsigned* n_exact,
-                                const HashScratch& scr, cudaStream_t s) {
+                                const HashScratch& scr, cudaStream_t s, int* launches) {
   const int L = P.n_tables, D = P.n_proj;
   if ((!di.hmat && (P.fhtDim != kVFht || !di.tflips)) || L < 1 || L > kVMaxL || qp_max < 1 || 2 * qp_max > L || stride < L)
     return cudaErrorInvalidValue;
@@ -582,12 +582,14 @@ cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const fl
       a.nq = n;
       const unsigned grid = (unsigned)((n + kCheckWarps - 1) / kCheckWarps);
       const CheckArgs c{a, scr.tmax, D / 128, di.hmat_err, scr.status};
+      *launches += 3;
       if (P.fhtDim == 128) k_hash_check<128><<<grid, 32 * kCheckWarps, 0, s>>>(c);
       if (P.fhtDim == 256) k_hash_check<256><<<grid, 32 * kCheckWarps, 0, s>>>(c);
       if (P.fhtDim == 512) k_hash_check<512><<<grid, 32 * kCheckWarps, 0, s>>>(c);
     }
     return cudaGetLastError();
   }
+  ++*launches;
   k_query_hash_verified<<<(unsigned)nq, kVThreads, 0, s>>>(a);
   return cudaGetLastError();
 }

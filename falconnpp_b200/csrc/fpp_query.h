@@ -97,10 +97,11 @@ struct HashScratch {
 // <= 128), with di.hmat or for fhtDim 256: the rotations on the tensor cores, and an exact
 // FP32 re-hash of every table whose score can reach the probe cut (ties at
 // the cut: of every table), so the probe cut selects the same probes with the
-// same scores.  n_exact (device, nullable) += the tables re-hashed.
+// same scores.  n_exact (device, nullable) += the tables re-hashed; launches
+// += the kernels launched.
 cudaError_t hash_lists_verified(const Params& P, const DeviceIndex& di, const float* Q, int nq, const int* q_qprobes,
                                 int qp_max, float* list_v, uint32_t* list_b, long long stride, unsigned* n_exact,
-                                const HashScratch& scr, cudaStream_t s);
+                                const HashScratch& scr, cudaStream_t s, int* launches);
 
 // Queries k_query_hash_verified takes in one full wave of its blocks on the
 // current device (SMs x resident blocks x queries per block); 0 if unknown.

@@ -92,3 +92,26 @@ def test_calls_of_changing_shape_settle_on_one_allocation():
     finally:
         g.set_option("inject_alloc_failure", 0)
     g.close()
+
+
+@pytest.mark.parametrize("D,nq,host,launches", [
+    (64, 200, False, 3),     # exact hash, probe cut, clusters
+    (64, 600, False, 3),     # exact hash, probe cut, fused kernel
+    (64, 1000, False, 5),    # and the order's two kernels
+    (128, 1000, False, 7),   # the product hash: rows, product, check
+    (128, 5000, True, 16),   # four chunks of it
+    (64, 5000, True, 8),     # four chunks of the exact hash
+])
+def test_launches_are_counted(D, nq, host, launches):
+    import torch
+    Q = synth.mixture(nq, 64, n_centres=16, seed=1)
+    g = _index(D=D)
+    g.set_query_form(1, 2, 4)
+    if host:
+        g.query(Q, 10)
+    else:
+        dq = torch.from_numpy(Q).cuda()
+        ids = torch.zeros((nq, 10), dtype=torch.int32, device="cuda")
+        _batched(g, dq, nq, 10, 6, ids)
+    assert int(g.stats(1)[6]) == launches
+    g.close()

@@ -424,13 +424,17 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
   }
   if ((e = bw.grow_block(blk, s)) != cudaSuccess) return fail(e, "alloc");
   const long long ext_stride = (long long)L * std::max(mmax, 1);
-  // The verified hash: its GEMM and its check take about 40 us however few the
-  // queries; the exact one gives a group of 8 lanes to every (query, table), 12
-  // us per 64 groups an SM.  The exact one is faster up to four of those waves;
-  // that is 378 queries at 100 tables, and 256 leave the verified hash the
-  // batches where it is ahead with fewer tables too.
+  // The verified hash: its product and check have 25 to 40 us in launches and
+  // waits however few the queries; the exact one gives a group of lanes to
+  // every (query, table), 10 us per 64 groups an SM (fhtDim 256).  Exact /
+  // verified in us, d 200, n_proj 256: 100 tables, 257 queries 38 / 48, 300 47 /
+  // 50, 400 58 / 50, 1,200 137 / 73; 64 tables, 300 37 / 41, 600 59 / 48; 32
+  // tables, 300 26 / 34, 800 39 / 40, 2,000 89 / 53; 8 tables, 300 13 / 29, 4,000
+  // 48 / 53.  One line for all: with 100 tables and more the two are equal near
+  // it, with fewer the exact one would still be ahead by up to 17 us to about
+  // 28,000 (query, table) pairs.
   const bool vhash = split && rq.tc_hash && (di.hmat || (F == 256 && di.tflips)) && L <= 128 &&
-                     2 * rq.qprobes_max <= L && (rq.nq > 256 || (long long)rq.nq * L > 4LL * 64 * nsm);
+                     2 * rq.qprobes_max <= L && rq.nq > 256;
   // scratch of its GEMM, for up to 32,768 queries at a time (66 MB at 100 tables of 256)
   const long long hash_nq = vhash && di.hmat ? std::min<long long>(rq.nq, 32768) : 0;
   // per-batch buffers: lists of the hash, processing order, probe cuts

@@ -5,7 +5,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <system_error>
 #include <thread>
 
 namespace fpp {
@@ -67,8 +66,8 @@ cudaError_t HostStage::copy(void* dst, const void* src, size_t bytes, cudaStream
   for (int t = 1; t < kThreads; ++t) {
     try {
       th[t - 1] = std::thread(work, t);
-    } catch (const std::system_error&) {
-      break;  // the others take its pieces
+    } catch (...) {  // no thread, or no memory for one
+      break;         // the others take its pieces
     }
   }
   work(0);

@@ -394,16 +394,17 @@ int batch_query(const Params& P, DeviceIndex& di, BatchWorkspace& bw, const Batc
     return fail(e, "occupancy");
   if (rq.blocks_per_sm > 0) per_sm = std::min(per_sm, rq.blocks_per_sm);
   per_sm = std::max(per_sm, 1);
+  // graph mode keeps one grid for every batch size (idle blocks find no work)
+  const int grid = std::max(1, rq.use_graph ? nsm * per_sm : std::min(rq.nq, nsm * per_sm));
   // a batch that leaves SMs without a query: a cluster of blocks per query
+  // (each query on the scratch of one block of the grid)
   int cl = 1;
   KernelSel kc{nullptr, 0};
-  if (split && !big && kmode != kRowsF32 && !rq.blocks_per_sm) {
+  if (split && !big && kmode != kRowsF32 && !rq.blocks_per_sm && rq.nq <= grid) {
     cl = cluster_size(rq.nq, nsm);
     if (cl > 1) kc = pick_kernel_cluster(kmode, d);
     if (!kc.fn) cl = 1;
   }
-  // graph mode keeps one grid for every batch size (idle blocks find no work)
-  int grid = std::max(1, rq.use_graph ? nsm * per_sm : std::min(rq.nq, nsm * per_sm));
   const long long nwords = (P.n_points + 31) / 32;
   const long long cap = std::max<long long>(
       1, std::min<long long>(P.n_points, (long long)rq.qprobes_max * std::max<uint32_t>(di.max_kept, 1u)));

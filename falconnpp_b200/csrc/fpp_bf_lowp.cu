@@ -1166,7 +1166,6 @@ cudaError_t grow(T*& p, size_t& cap, size_t need) {
   return e;
 }
 
-// rows out[i] = in[idx[i]] of w 32-bit words, or (scatter) out[idx[i]] = in[i]
 __global__ void k_bf_move_rows(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                const unsigned* __restrict__ idx, int w, int scatter) {
   const size_t r = blockIdx.x, t = idx[blockIdx.x];
@@ -1257,6 +1256,10 @@ cudaError_t launch_scan(int mode, const void* qrows, int nq, const void* xrows, 
 }
 
 }  // namespace
+
+void launch_move_rows(const void* in, void* out, const unsigned* idx, unsigned n, int w, bool scatter, cudaStream_t s) {
+  k_bf_move_rows<<<n, 128, 0, s>>>(static_cast<const uint32_t*>(in), static_cast<uint32_t*>(out), idx, w, scatter);
+}
 
 void BfWorkspace::release() {
   cudaFree(qrows);
@@ -1444,15 +1447,11 @@ extern "C" int fpp_bruteforce_topk_lowp(fpp_index* h, const float* d_queries, in
     if ((e = grow(scr.fq, scr.cap_fq, (size_t)nf * d)) || (e = grow(scr.fo, scr.cap_fo, (size_t)nf * n_neighbors)) ||
         (e = grow(scr.fv, scr.cap_fv, (size_t)nf * n_neighbors)))
       return bf_fail(e);
-    k_bf_move_rows<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(d_queries), reinterpret_cast<uint32_t*>(scr.fq),
-                                      scr.fail + 1, d, 0);
+    launch_move_rows(d_queries, scr.fq, scr.fail + 1, nf, d, false, s);
     rc = run_heaps(h->P, h->di, scr, nsm, precision, scr.fq, (int)nf, n_neighbors, R, scr.fo, scr.fv, s);
     if (rc) return rc;
-    k_bf_move_rows<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(scr.fo), reinterpret_cast<uint32_t*>(d_out),
-                                      scr.fail + 1, n_neighbors, 1);
-    if (d_out_val)
-      k_bf_move_rows<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(scr.fv),
-                                        reinterpret_cast<uint32_t*>(d_out_val), scr.fail + 1, n_neighbors, 1);
+    launch_move_rows(scr.fo, d_out, scr.fail + 1, nf, n_neighbors, true, s);
+    if (d_out_val) launch_move_rows(scr.fv, d_out_val, scr.fail + 1, nf, n_neighbors, true, s);
     e = cudaMemcpyAsync(&st, scr.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return bf_fail(e);

@@ -14,6 +14,10 @@ namespace fpp {
 cudaError_t launch_hash_scan(const void* qrows, int nq, const void* matrix, int rows, int d, int ld, float* tmax,
                              unsigned* status, int nsm, cudaStream_t s);
 
+// Rows of w 32-bit words, n of them: out[i] = in[idx[i]], or with scatter
+// out[idx[i]] = in[i].  Asynchronous.
+void launch_move_rows(const void* in, void* out, const unsigned* idx, unsigned n, int w, bool scatter, cudaStream_t s);
+
 // Subtracted from a threshold: more than the absolute error that products and
 // sums below FP32's normal range can add (norms are at most 1e15).
 constexpr float kTruthSlack = 1e-34f;

@@ -250,14 +250,6 @@ __global__ void __launch_bounds__(kBfThreads) k_bf_rescore(const float* __restri
   }
 }
 
-__global__ void k_bf_rows32(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                            const unsigned* __restrict__ idx, int w, int scatter) {
-  const size_t r = blockIdx.x, t = idx[blockIdx.x];
-  const uint32_t* src = in + (scatter ? r : t) * (size_t)w;
-  uint32_t* dst = out + (scatter ? t : r) * (size_t)w;
-  for (int j = threadIdx.x; j < w; j += blockDim.x) dst[j] = src[j];
-}
-
 // The FP64 scores of every point (k_bf_partial, k_bf_merge); returns after the
 // results are written.
 cudaError_t topk_direct(const float* d_X, long long n_points, int n_features, const float* d_Q, int n_queries, int k,
@@ -333,14 +325,10 @@ cudaError_t topk_candidates(TruthScan& ts, const float* d_X, long long n, int d,
     if ((e = dev_malloc(&fq, sizeof(float) * (size_t)nf * d)) == cudaSuccess &&
         (e = dev_malloc(&fo, sizeof(int32_t) * (size_t)nf * k)) == cudaSuccess &&
         (e = dev_malloc(&fv, sizeof(double) * (size_t)nf * k)) == cudaSuccess) {
-      k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(d_Q), reinterpret_cast<uint32_t*>(fq), fail + 1,
-                                     d, 0);
+      launch_move_rows(d_Q, fq, fail + 1, nf, d, false, s);
       e = topk_direct(d_X, n, d, fq, (int)nf, k, fo, fv, nsm, s);
-      k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(fo), reinterpret_cast<uint32_t*>(d_out),
-                                     fail + 1, k, 1);
-      if (d_out_val)
-        k_bf_rows32<<<nf, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(fv), reinterpret_cast<uint32_t*>(d_out_val),
-                                       fail + 1, 2 * k, 1);
+      launch_move_rows(fo, d_out, fail + 1, nf, k, true, s);
+      if (d_out_val) launch_move_rows(fv, d_out_val, fail + 1, nf, 2 * k, true, s);
       const cudaError_t e3 = cudaStreamSynchronize(s);
       if (e == cudaSuccess) e = e3;
     }

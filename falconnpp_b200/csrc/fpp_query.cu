@@ -769,7 +769,7 @@ int query_index(const Params& P, const DeviceIndex& di, const float* Q, bool q_o
     qa.nq = nq;
     qa.d = d;
     qa.flips = di.flips;
-      qa.L = L;
+    qa.L = L;
     qa.D = D;
     qa.log2D = log2D;
     qa.NB = NB;

@@ -664,10 +664,11 @@ constexpr unsigned kRepairCap[2] = {880, 7000};
 __device__ __forceinline__ unsigned add_repair(const BucketArgs& a, uint32_t b, uint32_t B, uint32_t kp, uint32_t out) {
   const int c = B <= kRepairCap[0] ? 0 : B <= kRepairCap[1] ? 1 : 2;
   atomicAdd(a.n_repaired, 1ull);
+  // (failed ranges cannot wrap the counter: at most 148 blocks bring buckets of
+  // up to 2^23 entries at once, 444 of 2^13, 9,472 warps of 2^9)
   auto reserve = [](unsigned* used, unsigned want, unsigned cap) {
     return arena_reserve(
-        want, cap, [=] { return *(volatile unsigned*)used; },
-        [=](unsigned expect, unsigned value) { return atomicCAS(used, expect, value); });
+        want, cap, [=] { return *(volatile unsigned*)used; }, [=](unsigned v) { return atomicAdd(used, v); });
   };
   unsigned* items = a.deferred + 1 + c;
   if (*(volatile unsigned*)items < a.max_items) {  // else the class is full for good
@@ -1038,7 +1039,7 @@ __global__ void __launch_bounds__(kRepairThreads<CLS>) k_repair(BucketArgs a, bo
     else
       __syncwarp();
   };
-  const unsigned nrep = deferred ? a.deferred[1 + CLS] : a.counters[3 + CLS];
+  const unsigned nrep = deferred ? min(a.deferred[1 + CLS], a.max_items) : a.counters[3 + CLS];
   for (unsigned r = blockIdx.x; r < nrep; r += gridDim.x) {
     uint32_t B, kp;
     uint64_t* g;

@@ -21,7 +21,7 @@ struct fpp_index {
   fpp::BatchWorkspace bw;
   fpp::BfWorkspace bfw;
   fpp::HostStage stage;     // pageable data on its way to a build
-  int form = 0;             // 0 plain three-kernel path, 1 batched fused kernel
+  int form = 0;             // 0 plain (exact FP32, whichever kernels), 1 batched
   int precision = 0;        // batched form: 0 FP32 (exact), 1 BF16, 2 FP8-E4M3
   int shortlist_mult = 4;   // batched low precision: FP32 re-score of shortlist_mult * k
   bool use_graph = false;   // batched form: capture/replay the launch as a CUDA graph

@@ -123,8 +123,10 @@ int fpp_get_stats(fpp_index* h, int kind, double* out, int n);
  * cut of every query in its own kernel, before the fused gather / rerank /
  * top-k kernel; 0: one fused kernel that also rotates and hashes; the results
  * are the same), "tc_hash" (default
- * 1: with the split hash, fhtDim 256, n_tables <= 128 and 2 qProbes <=
- * n_tables, the hash kernel rotates on the tensor cores with FP16 operands,
+ * 1: with the split hash, n_tables <= 128, 2 qProbes <= n_tables, more than 256
+ * queries, and an index with the rotations as matrices (n_proj >= 128, fhtDim
+ * 128 to 512, n_features <= 256) or fhtDim 256, the hash rotates on the tensor
+ * cores with FP16 operands,
  * bounds the error of every table's score from the query's norm, and hashes
  * again in the reference's FP32 arithmetic every table whose score can reach
  * the probe cut (every table when exact scores tie at the cut); the probes
@@ -172,8 +174,9 @@ int fpp_query_dump(fpp_index* h, const float* queries, int n_queries, int n_neig
                    long long cand_cap);
 
 /* Selects the implementation behind fpp_query / fpp_query_device (and the
- * Python query()).  form 0 (default): the plain FP32 path of three kernels,
- * bit-exact with src/FalconnPP.cpp:310-707.  form 1: the batched path, one
+ * Python query()).  form 0 (default): the plain FP32 form, bit-exact with
+ * src/FalconnPP.cpp:310-707 (through the batched kernels inside their limits,
+ * where their scratch fits, else through three kernels of its own).  form 1: the batched path, one
  * persistent fused kernel per batch (rotate, hash, probe, gather, rerank,
  * top-k) with dynamic scheduling; precision 0 reranks in FP32 and equals the
  * plain path bit for bit; precision 1 (BF16) and 2 (FP8-E4M3 with a per-row

@@ -267,9 +267,9 @@ __device__ __forceinline__ int group_top_cp(const float (&y)[Geo<FHT>::E], int g
         br = orr;
       }
     }
-    // no comparable coordinate left (NaN): the group's later rounds find none
-    // either, but the warp's other groups need its lanes in their shuffles
-    const bool none = br == 0x7fffffff;
+    // fewer than cnt comparable coordinates (NaN) in any group: all of the warp's
+    // groups stop together, as their shuffles need every lane, and replay
+    if (__any_sync(kFullMask, br == 0x7fffffff)) break;
     int code = 0;
     if (br / E == gl) {
       const int e = br - gl * E;
@@ -281,13 +281,13 @@ __device__ __forceinline__ int group_top_cp(const float (&y)[Geo<FHT>::E], int g
       code = cp_code(x, br, log2D);
     }
     // the owner lane publishes the code
-    const int owner = (threadIdx.x & 31 & ~(G - 1)) + (none ? 0 : br / E);
+    const int owner = (threadIdx.x & 31 & ~(G - 1)) + br / E;
     code = __shfl_sync(kFullMask, code, owner);
-    if (gl == 0 && !none) {
+    if (gl == 0) {
       out_v[t] = bv;
       out_c[t] = code;
     }
-    found += none ? 0 : 1;
+    ++found;
   }
   return found;
 }
@@ -356,16 +356,16 @@ __device__ __forceinline__ int group_top_cp_small(const float (&y)[Geo<FHT>::E],
         wr = orr;
       }
     }
-    const bool none = wr == 0x7fffffff;  // stays so (see group_top_cp)
+    if (__any_sync(kFullMask, wr == 0x7fffffff)) break;  // (see group_top_cp)
     const bool mine = (wr == hr);
-    const int owner = (threadIdx.x & 31 & ~(G - 1)) + (none ? 0 : wr / E);
+    const int owner = (threadIdx.x & 31 & ~(G - 1)) + wr / E;
     const int code = __shfl_sync(kFullMask, hc, owner);
-    if (mine && !none) ++head;
-    if (gl == 0 && !none) {
+    if (mine) ++head;
+    if (gl == 0) {
       out_v[t] = wv;
       out_c[t] = code;
     }
-    found += none ? 0 : 1;
+    ++found;
   }
   return found;
 }
@@ -412,17 +412,17 @@ __device__ __forceinline__ int group_top2_cp(const float (&y)[Geo<FHT>::E], int 
         wr = orr;
       }
     }
-    const bool none = wr == 0x7fffffff;  // stays so (see group_top_cp)
+    if (__any_sync(kFullMask, wr == 0x7fffffff)) break;  // (see group_top_cp)
     const bool mine = (wr == myr);
     const float sy = took0 ? s1 : s0;
-    const int owner = (threadIdx.x & 31 & ~(G - 1)) + (none ? 0 : wr / E);
+    const int owner = (threadIdx.x & 31 & ~(G - 1)) + wr / E;
     const float wy = __shfl_sync(kFullMask, sy, owner);
-    if (mine && !none) took0 = true;
-    if (gl == 0 && !none) {
+    if (mine) took0 = true;
+    if (gl == 0) {
       out_v[t] = cp_value(wy);
       out_c[t] = cp_code(wy, wr, log2D);
     }
-    found += none ? 0 : 1;
+    ++found;
   }
   return found;
 }
@@ -614,13 +614,12 @@ __device__ __forceinline__ bool group_top_stored(float* v, int gl, int D, int lo
         br = orr;
       }
     }
-    // nothing comparable left (NaN): the replay decides, and the group stays for
-    // the other groups' shuffles
-    const bool none = br == 0x7fffffff;
-    strict = strict && !none && (t == 0 || pv > bv);
+    // not comparable (NaN): the replay decides, for all of the warp's groups
+    if (__any_sync(kFullMask, br == 0x7fffffff)) return false;
+    strict = strict && (t == 0 || pv > bv);
     pv = bv;
     pr = br;
-    if (gl == 0 && !none) {
+    if (gl == 0) {
       out_v[t] = bv;
       out_c[t] = cp_code(LaneVector<FHT>::at(v, br), br, log2D);
     }
